@@ -31,29 +31,29 @@ def listed():
     return [
         # a handful of small configurations on the device: what an interactive
         # search evaluates per step, bound by the launch
-        dict(name="energy, 48 x n=17", kind="energy", configs=48, n=17, count=False),
+        dict(name="energy: 48 x n=17", kind="energy", configs=48, n=17, count=False),
         # the benchmark's batch: 4,096 random configurations of 200 squares
-        dict(name="energy, 4096 x n=200", kind="energy", configs=4096, n=200, count=False),
+        dict(name="energy: 4096 x n=200", kind="energy", configs=4096, n=200, count=False),
         # the largest states the engine takes, candidate pairs counted
-        dict(name="energy, 1500 x n=999", kind="energy", configs=1500, n=999, count=True),
+        dict(name="energy: 1500 x n=999", kind="energy", configs=1500, n=999, count=True),
         # the same energy called on host arrays, a ragged batch
-        dict(name="energy from host, 777 x n=333", kind="energy_host", configs=777, n=333, count=True),
+        dict(name="energy from host: 777 x n=333", kind="energy_host", configs=777, n=333, count=True),
         # FP64 recompute of a search's candidate states, every size of the competition
-        dict(name="energy FP64, 400 of n 5-1000", kind="energy_fp64", count=400, n_lo=5, n_hi=1000),
+        dict(name="energy FP64 400 of n 5-1000", kind="energy_fp64", count=400, n_lo=5, n_hi=1000),
         # polish of a campaign's raw states, half of them overlapped
-        dict(name="polish, 64 of n 5-1000", kind="polish", count=64, n_lo=5, n_hi=1000, iters=200),
+        dict(name="polish: 64 of n 5-1000", kind="polish", count=64, n_lo=5, n_hi=1000, iters=200),
         # the gate on one candidate packing, as each merge step calls it
-        dict(name="certify, 1 of n 40-60", kind="certify", count=1, n_lo=40, n_hi=60, roundtrip=False),
+        dict(name="certify: 1 of n 40-60", kind="certify", count=1, n_lo=40, n_hi=60, roundtrip=False),
         # validation of a batch of submissions: exact grids, near-contact lattices, injected overlaps
-        dict(name="certify, 1500 of n 5-1000", kind="certify", count=1500, n_lo=5, n_hi=1000, roundtrip=False),
+        dict(name="certify: 1500 of n 5-1000", kind="certify", count=1500, n_lo=5, n_hi=1000, roundtrip=False),
         # the plain single-instance job: n = 10, 8 replicas, polish and certificate
-        dict(name="anneal, n=10 x 8 replicas", kind="anneal", n=10, replicas=8, sweeps=4000),
+        dict(name="anneal: n=10 x 8 replicas", kind="anneal", n=10, replicas=8, sweeps=4000),
         # one batched launch of many instances: n uniform in [20, 400], 32 replicas
-        dict(name="anneal batch, 256 x 32", kind="anneal_batch", count=256, n_lo=20, n_hi=400, replicas=32, sweeps=50),
+        dict(name="anneal batch: 256 x 32", kind="anneal_batch", count=256, n_lo=20, n_hi=400, replicas=32, sweeps=50),
         # the drop-in search programs' call: ladders of 8 chains below a shared best side
-        dict(name="search, n=50, 64 chains", kind="search", n=50, ladders=8, epochs=40, steps=64),
+        dict(name="search: n=50: 64 chains", kind="search", n=50, ladders=8, epochs=40, steps=64),
         # a burst of served jobs of mixed sizes
-        dict(name="serve, 32 jobs of n 5-300", kind="serve", count=32, n_lo=5, n_hi=300, sweeps=200),
+        dict(name="serve: 32 jobs of n 5-300", kind="serve", count=32, n_lo=5, n_hi=300, sweeps=200),
     ]
 
 
