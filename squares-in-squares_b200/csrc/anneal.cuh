@@ -38,6 +38,13 @@ struct JobDev {
     int32_t quench_stall;             // accepted slow steps (< 0.1% gained each) that end a quench
 };
 
+// One job of a batch call's state initialisation (init_states_kernel).
+struct InitRec {
+    int64_t src, dst;                 // double index of its uploaded start states, float4 index of its replicas
+    int32_t n, R;                     // squares, replicas
+    int32_t states, pad;              // start states uploaded: 1 (every replica's) or R (one a replica)
+};
+
 // Move-set options of a job (the same bits as SQS_JOB_ADAPT, _COLLECTIVE, _KICK).
 // kMoveSerial selects the one-at-a-time kernel instance and changes nothing else;
 // kCertAll (SQS_JOB_CERT_ALL) only drops the energy gate of the checkpoint's

@@ -563,7 +563,8 @@ static int anneal_run(sqs_ctx* ctx, const sqs_job* jobs, int njobs, int slice_sw
     std::vector<JobMut> jm((size_t)njobs);
     std::vector<Plan> plan((size_t)njobs);
     std::vector<sqs_job> eff((size_t)njobs);
-    int64_t pos_total = 0, best_total = 0;
+    std::vector<InitRec> init((size_t)njobs);
+    int64_t pos_total = 0, best_total = 0, start_total = 0;
     const int mode = njobs == 1 ? SQS_TUNE_LATENCY : 0;
     for (int j = 0; j < njobs; ++j) {
         std::memset(&out[j], 0, sizeof(sqs_job_result));
@@ -573,8 +574,11 @@ static int anneal_run(sqs_ctx* ctx, const sqs_job* jobs, int njobs, int slice_sw
         jd[(size_t)j].pos_off = pos_total;
         jd[(size_t)j].best_off = best_total;
         jd[(size_t)j].scr_off = pos_total + (int64_t)jobs[j].replicas * jobs[j].n;
+        const int states = jobs[j].xya_rep ? jobs[j].replicas : 1;
+        init[(size_t)j] = InitRec{start_total, pos_total, jobs[j].n, jobs[j].replicas, states, 0};
         pos_total += job_pos_elems(jobs[j]);
         best_total += 3 * (int64_t)jobs[j].n;
+        start_total += 3 * (int64_t)jobs[j].n * states;
     }
     // device state: one allocation, resident for the whole call
     size_t tot = 0;
@@ -582,6 +586,7 @@ static int anneal_run(sqs_ctx* ctx, const sqs_job* jobs, int njobs, int slice_sw
     const size_t o_jd = seg(sizeof(JobDev) * njobs), o_jm = seg(sizeof(JobMut) * njobs);
     const size_t o_pos = seg(sizeof(float4) * (size_t)pos_total), o_best = seg(sizeof(double) * (size_t)best_total);
     const size_t o_list = seg(sizeof(int32_t) * njobs);
+    const size_t o_init = seg(sizeof(InitRec) * njobs), o_start = seg(sizeof(double) * (size_t)start_total);
     // trace: one (job, replica) item and one record per replica
     int64_t ntrace = 0;
     size_t trace_smem = 0;
@@ -599,15 +604,21 @@ static int anneal_run(sqs_ctx* ctx, const sqs_job* jobs, int njobs, int slice_sw
     double* d_best = (double*)(D + o_best);
     int32_t* d_list = (int32_t*)(D + o_list);
     {
-        std::vector<float4> hpos((size_t)pos_total);
-        std::vector<double> hbest((size_t)best_total, 0.0);
-        for (int j = 0; j < njobs; ++j) init_replicas(jobs[j], hpos.data() + jd[(size_t)j].pos_off);
+        std::vector<double> hstart;
+        hstart.reserve((size_t)start_total);
+        for (int j = 0; j < njobs; ++j) {
+            const double* src = jobs[j].xya_rep ? jobs[j].xya_rep : jobs[j].xya;
+            hstart.insert(hstart.end(), src, src + 3 * (size_t)jobs[j].n * (size_t)init[(size_t)j].states);
+        }
         SQS_CUDA(cudaMemcpyAsync(d_jd, jd.data(), sizeof(JobDev) * njobs, cudaMemcpyHostToDevice, ctx->stream));
         SQS_CUDA(cudaMemcpyAsync(d_jm, jm.data(), sizeof(JobMut) * njobs, cudaMemcpyHostToDevice, ctx->stream));
-        SQS_CUDA(cudaMemcpyAsync(d_pos, hpos.data(), sizeof(float4) * hpos.size(), cudaMemcpyHostToDevice, ctx->stream));
-        SQS_CUDA(cudaMemcpyAsync(d_best, hbest.data(), sizeof(double) * hbest.size(), cudaMemcpyHostToDevice,
+        SQS_CUDA(cudaMemcpyAsync(D + o_init, init.data(), sizeof(InitRec) * njobs, cudaMemcpyHostToDevice, ctx->stream));
+        SQS_CUDA(cudaMemcpyAsync(D + o_start, hstart.data(), sizeof(double) * hstart.size(), cudaMemcpyHostToDevice,
                                  ctx->stream));
-        SQS_CUDA(cudaStreamSynchronize(ctx->stream));  // host vectors go out of scope
+        SQS_CUDA(cudaMemsetAsync(d_best, 0, sizeof(double) * (size_t)best_total, ctx->stream));
+        if (int r = launch_init(ctx->stream, njobs, (const InitRec*)(D + o_init), (const double*)(D + o_start), d_pos)) return r;
+        ctx->launches += 1;
+        // (the pageable copies have consumed hstart when they return)
     }
     // launch groups: jobs sharing (cluster size, replicas per CTA, kernel
     // instance); shared memory of the largest
