@@ -25,7 +25,7 @@ struct Shape {
 int prime_anneal();
 int launch_init(cudaStream_t stream, int njobs, const InitRec* rec, const double* start, float4* pos);
 int launch_trace(cudaStream_t stream, int items, const int2* list, const JobDev* jdev, const JobMut* jmut,
-                 const float4* pos, TraceRec* out, size_t smem);
+                 float4* pos, TraceRec* out, size_t smem);
 size_t energy_smem_bytes(int n);
 int launch_energy_states(cudaStream_t stream, int count, const int32_t* n_of, const int64_t* row0, const double* side,
                          const double* xya, double* energy_out, double* grad, size_t smem);

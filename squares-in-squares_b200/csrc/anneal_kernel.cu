@@ -89,12 +89,12 @@ __device__ __forceinline__ float wall_e(float x, float y, float c, float s, floa
 
 // Build the cell list of one replica (warp).  Returns false on overflow (a
 // cell asked for more than kCellK slots); the list is then incomplete but
-// every count is clamped to kCellK and every slot holds a valid index, so no
-// later scan can leave the replica's arrays.
+// every count is clamped to kCellK and the slots below it are all written
+// (ranks 0 .. kCellK - 1 were handed out), so no later scan can leave the
+// replica's arrays.  Slots at or past a cell's count are never read.
 __device__ bool build_cells(const Rep& R, int n, const Grid& g, int lane) {
     const int ncell = g.G * g.G;
-    for (int c = lane; c < ncell; c += 32) R.cnt[c] = 0;
-    for (int k = lane; k < ncell * kCellK; k += 32) R.slot[k] = 0;
+    for (int c = 4 * lane; c < ncell; c += 128) *reinterpret_cast<uint32_t*>(R.cnt + c) = 0u;
     __syncwarp();
     bool ok = true;
     for (int i = lane; i < n; i += 32) {
@@ -192,19 +192,41 @@ __device__ __forceinline__ double warp_min_d(double v) {
     return v;
 }
 
-// Full energy of one replica (walls + each neighbour pair once), fixed point.
+// Half of a square's 3 x 3 block: k = 0 its own cell, 1 the cell to the east,
+// 2..4 the row above.  Over all squares these visit each unordered pair of
+// neighbours once (in the own cell, from the lower index) when the lists are
+// current, that is every square is listed in the cell its centre lies in.
+__device__ __forceinline__ void half_block(int k, int& dx, int& dy) {
+    dx = k == 0 ? 0 : (k == 1 ? 1 : k - 3);
+    dy = k >= 2;
+}
+
+// Full energy of one replica (walls + each neighbour pair once), fixed
+// point, on current lists.  Work item w is square w / 5 against cell w % 5 of
+// its half block, a lane each: a warp takes 5 n / 32 short rounds.  One
+// square at a time with the warp on its whole block left most lanes without
+// a candidate and took n rounds of a nine-count prefix each; a collective
+// move spends most of its time here.  With the certified side split the same
+// way, the slots no longer cleared and the undo copies in shared memory, a
+// search of n = 50 with 64 chains (40 epochs x 64) went from 101.8 to 65.4 ms.
 __device__ long long full_energy(const Rep& R, int n, const Grid& g, float L, int lane) {
     long long e = 0;
-    for (int i = 0; i < n; ++i) {
+    for (int w = lane; w < 5 * n; w += 32) {
+        const int i = w / 5, c = w - 5 * i;
         const float4 P = R.sq[i];
-        if (lane == 0) e += qe(wall_e(P.x, P.y, P.z, P.w, L));
-        for_block(R, g, g.cx(P.x), g.cx(P.y), lane, [&](int j) {
-            if (j > i) {
-                const float4 Q = R.sq[j];
-                const float dx = Q.x - P.x, dy = Q.y - P.y;
-                if (dx * dx + dy * dy < kPairCut2) e += qe(sat_pair_energy(dx, dy, P.z, P.w, Q.z, Q.w));
-            }
-        });
+        if (c == 0) e += qe(wall_e(P.x, P.y, P.z, P.w, L));
+        int dx, dy;
+        half_block(c, dx, dy);
+        const int x = g.cx(P.x) + dx, y = g.cx(P.y) + dy;
+        if (x < 0 || x >= g.G || y >= g.G) continue;
+        const int cell = y * g.G + x, m = R.cnt[cell];
+        for (int k = 0; k < m; ++k) {
+            const int j = R.slot[cell * kCellK + k];
+            if (c == 0 && j <= i) continue;
+            const float4 Q = R.sq[j];
+            const float ex = Q.x - P.x, ey = Q.y - P.y;
+            if (ex * ex + ey * ey < kPairCut2) e += qe(sat_pair_energy(ex, ey, P.z, P.w, Q.z, Q.w));
+        }
     }
     return warp_sum_ll(e);
 }
@@ -214,41 +236,43 @@ __device__ long long full_energy(const Rep& R, int n, const Grid& g, float L, in
 // tau = 2.6e-8 gap along the best axis of every close pair, rejection above
 // 1.008, side of the bounding box of the dilated squares.  Products are kept
 // unfused so the result rounds like the host oracle's.
-__device__ double cert_side(const Rep& R, int n, const Grid& g, int lane, double& lam_out, double& x0_out,
+__device__ double cert_side(const Rep& R, int n, const Grid& g, int lane, double2* trig, double& lam_out, double& x0_out,
                             double& y0_out) {
     const double tau = 2.6e-8;
     double lam = 1.0;
     for (int i = lane; i < n; i += 32) {
+        double s, c;
+        sincos((double)R.ang[i], &s, &c);
+        trig[i] = make_double2(c, s);
+    }
+    __syncwarp();
+    // a lane per (square, cell of its half block): the required dilation of a
+    // pair is the same from either side, and the largest one needs no order
+    for (int w = lane; w < 5 * n; w += 32) {
+        const int i = w / 5, c = w - 5 * i;
         const float4 P = R.sq[i];
-        const double xi = P.x, yi = P.y;
-        double si, ci;
-        sincos((double)R.ang[i], &si, &ci);
-        const int cx = g.cx(P.x), cy = g.cx(P.y);
-        for (int dy = -1; dy <= 1; ++dy) {
-            for (int dxc = -1; dxc <= 1; ++dxc) {
-                const int x = cx + dxc, y = cy + dy;
-                if (x < 0 || x >= g.G || y < 0 || y >= g.G) continue;
-                const int cell = y * g.G + x;
-                const int m = R.cnt[cell];
-                for (int k = 0; k < m; ++k) {
-                    const int j = R.slot[cell * kCellK + k];
-                    if (j <= i) continue;
-                    const double dx = __dsub_rn(xi, (double)R.sq[j].x), dyv = __dsub_rn(yi, (double)R.sq[j].y);
-                    if (__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dyv, dyv)) >= 2.05) continue;
-                    double sj, cj;
-                    sincos((double)R.ang[j], &sj, &cj);
-                    const double c12 = fabs(__dadd_rn(__dmul_rn(ci, cj), __dmul_rn(si, sj)));
-                    const double s12 = fabs(__dadd_rn(__dmul_rn(-si, cj), __dmul_rn(ci, sj)));
-                    const double r = __dadd_rn(0.5, __dmul_rn(0.5, __dadd_rn(c12, s12)));
-                    const double v1 = fabs(__dadd_rn(__dmul_rn(dx, ci), __dmul_rn(dyv, si)));
-                    const double v2 = fabs(__dadd_rn(__dmul_rn(-dx, si), __dmul_rn(dyv, ci)));
-                    const double v3 = fabs(__dadd_rn(__dmul_rn(dx, cj), __dmul_rn(dyv, sj)));
-                    const double v4 = fabs(__dadd_rn(__dmul_rn(-dx, sj), __dmul_rn(dyv, cj)));
-                    const double vmax = fmax(fmax(v1, v2), fmax(v3, v4));
-                    const double req = vmax > 1e-12 ? __ddiv_rn(__dadd_rn(r, tau), vmax) : 1e9;
-                    lam = fmax(lam, req);
-                }
-            }
+        int hx, hy;
+        half_block(c, hx, hy);
+        const int x = g.cx(P.x) + hx, y = g.cx(P.y) + hy;
+        if (x < 0 || x >= g.G || y >= g.G) continue;
+        const int cell = y * g.G + x, m = R.cnt[cell];
+        const double xi = P.x, yi = P.y, ci = trig[i].x, si = trig[i].y;
+        for (int k = 0; k < m; ++k) {
+            const int j = R.slot[cell * kCellK + k];
+            if (c == 0 && j <= i) continue;
+            const double dx = __dsub_rn(xi, (double)R.sq[j].x), dyv = __dsub_rn(yi, (double)R.sq[j].y);
+            if (__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dyv, dyv)) >= 2.05) continue;
+            const double cj = trig[j].x, sj = trig[j].y;
+            const double c12 = fabs(__dadd_rn(__dmul_rn(ci, cj), __dmul_rn(si, sj)));
+            const double s12 = fabs(__dadd_rn(__dmul_rn(-si, cj), __dmul_rn(ci, sj)));
+            const double r = __dadd_rn(0.5, __dmul_rn(0.5, __dadd_rn(c12, s12)));
+            const double v1 = fabs(__dadd_rn(__dmul_rn(dx, ci), __dmul_rn(dyv, si)));
+            const double v2 = fabs(__dadd_rn(__dmul_rn(-dx, si), __dmul_rn(dyv, ci)));
+            const double v3 = fabs(__dadd_rn(__dmul_rn(dx, cj), __dmul_rn(dyv, sj)));
+            const double v4 = fabs(__dadd_rn(__dmul_rn(-dx, sj), __dmul_rn(dyv, cj)));
+            const double vmax = fmax(fmax(v1, v2), fmax(v3, v4));
+            const double req = vmax > 1e-12 ? __ddiv_rn(__dadd_rn(r, tau), vmax) : 1e9;
+            lam = fmax(lam, req);
         }
     }
     lam = warp_max_d(lam);
@@ -258,9 +282,7 @@ __device__ double cert_side(const Rep& R, int n, const Grid& g, int lane, double
     for (int i = lane; i < n; i += 32) {
         const float4 P = R.sq[i];
         const double x = __dmul_rn((double)P.x, lam), y = __dmul_rn((double)P.y, lam);
-        double s, c;
-        sincos((double)R.ang[i], &s, &c);
-        const double r = __dmul_rn(0.5, __dadd_rn(fabs(c), fabs(s)));
+        const double r = __dmul_rn(0.5, __dadd_rn(fabs(trig[i].x), fabs(trig[i].y)));
         bx0 = fmin(bx0, __dsub_rn(x, r));
         bx1 = fmax(bx1, __dadd_rn(x, r));
         by0 = fmin(by0, __dsub_rn(y, r));
@@ -367,8 +389,7 @@ struct BarGrp {
 template <class Grp>
 __device__ bool build_cells_grp(const Grp& gp, const Rep& R, int n, const Grid& g) {
     const int ncell = g.G * g.G, tid = gp.t(), nt = gp.nt();
-    for (int c = tid; c < ncell; c += nt) R.cnt[c] = 0;
-    for (int k = tid; k < ncell * kCellK; k += nt) R.slot[k] = 0;
+    for (int c = 4 * tid; c < ncell; c += 4 * nt) *reinterpret_cast<uint32_t*>(R.cnt + c) = 0u;
     gp.sync();
     bool ok = true;
     for (int i = tid; i < n; i += nt) {
@@ -692,8 +713,7 @@ __device__ __forceinline__ float wrap_quarter_f(float a) {
 // the drawn square by `th` for modes 3 and 4, and every moved square turned by
 // `th` (seeded.cu:547-613).  Centres stay in [0.5, L - 0.5].  The move is
 // judged on the full fixed-point energy; a rejected move (or one that
-// overflows a cell) is undone from `save`, the replica's own HBM slot, which
-// holds nothing else while a slice runs.  Returns whether it was accepted;
+// overflows a cell) is undone from `save`, the replica's scratch block.  Returns whether it was accepted;
 // *ovf counts overflows.
 __device__ __forceinline__ bool collective_move(const Rep& rep, const Grid& g, int n, float L, int lane, int mode, int c,
                                              float tx, float ty, float th, float u, float invT, long long& E,
@@ -1030,7 +1050,13 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
     int win = (MOVES && active) ? S.jm.win[r] : 0;
     float cool = cool_of(adaptive, S.jm.xround);
     float invT = active ? 1.0f / (S.temps[S.jm.perm[r]] * cool) : 0.f;
-    float4* save = pos + jd.pos_off + (int64_t)r * n;  // this replica's HBM slot: free while the slice runs
+    // this replica's scratch block (kQuenchScr n float4): in shared memory after
+    // the replicas when the launch left room for every replica's, else in HBM;
+    // between quenches it holds the undo copy of a collective move or kick and
+    // the FP64 trig of the certified side
+    const bool smem_scr = (int64_t)dyn_bytes >= (int64_t)Rl * (rb + (int64_t)sizeof(float4) * kQuenchScr * n);
+    float4* scr_own = smem_scr ? reinterpret_cast<float4*>(dyn + (int64_t)Rl * rb) + (int64_t)(active ? w : 0) * kQuenchScr * n
+                               : pos + jd.scr_off + (int64_t)r * kQuenchScr * n;
 
     // Proposals are numbered per replica across the whole job (a sweep is n
     // of them); checkpoints fall after every xprops proposals and at the end
@@ -1110,7 +1136,7 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     const float da = sda * sc;
                     bool acc;
                     if (MOVES && mode != 0) {
-                        acc = collective_move(rep, g, n, Lr, lane, mode, i, dx, dy, da, u_acc, invT, E, save, &ovf);
+                        acc = collective_move(rep, g, n, Lr, lane, mode, i, dx, dy, da, u_acc, invT, E, scr_own, &ovf);
                         ++props;
                         accs += acc;
                     } else {
@@ -1272,7 +1298,6 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
             // the replicas when the launch left room for all of them, else
             // the replica's own block of the job's scratch in HBM
             const int gw = (int)(blockDim.x >> 5) / Rl, q = w / gw;
-            const bool smem_scr = (int64_t)dyn_bytes >= (int64_t)Rl * (rb + (int64_t)sizeof(float4) * kQuenchScr * n);
             float4* qw = smem_scr ? reinterpret_cast<float4*>(dyn + (int64_t)Rl * rb) + (int64_t)q * kQuenchScr * n
                                   : pos + jd.scr_off + ((int64_t)rank * Rl + q) * kQuenchScr * n;
             if (gw == 1) {
@@ -1318,7 +1343,8 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
             // so the energy gate skips states that cannot pass); under
             // SQS_JOB_CERT_ALL every replica is measured, as the reference
             // search measures every chain after its polish (seeded.cu:716)
-            if (E < qe(1e-4f) || (jd.flags & kCertAll)) Lc = cert_side(rep, n, g, lane, lam, x0, y0);
+            if (E < qe(1e-4f) || (jd.flags & kCertAll)) 
+                Lc = cert_side(rep, n, g, lane, reinterpret_cast<double2*>(scr_own), lam, x0, y0);
             if (lane == 0) {
                 S.wE[w] = E;
                 S.wL[w] = Lc;
@@ -1478,7 +1504,7 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
         // overlapped replicas are kicked (the round just completed decides
         // whether the worst square is also moved)
         if (MOVES && active && (jd.flags & kMoveKick) && E > qe(1e-12f))
-            E = kick_replica(rep, g, n, Lr, lane, r, S.jm.xround, k0, k1, E, save);
+            E = kick_replica(rep, g, n, Lr, lane, r, S.jm.xround, k0, k1, E, scr_own);
     }
 
     // ---- write the slice back
@@ -1549,7 +1575,7 @@ int launch_init(cudaStream_t stream, int njobs, const InitRec* rec, const double
 // dilation-certified side, and reports the temperature and step scale its
 // next proposal would use.
 __global__ void __launch_bounds__(32) trace_kernel(const int2* __restrict__ items, const JobDev* __restrict__ jdev,
-                                                   const JobMut* __restrict__ jmut, const float4* __restrict__ pos,
+                                                   const JobMut* __restrict__ jmut, float4* __restrict__ pos,
                                                    TraceRec* __restrict__ out) {
     extern __shared__ __align__(16) unsigned char dyn[];
     const int2 it = items[blockIdx.x];
@@ -1571,7 +1597,8 @@ __global__ void __launch_bounds__(32) trace_kernel(const int2* __restrict__ item
     const bool ok = build_cells(rep, n, g, lane);
     const long long E = full_energy(rep, n, g, L, lane);
     double lam = 0, x0 = 0, y0 = 0;
-    const double Lc = cert_side(rep, n, g, lane, lam, x0, y0);
+    const double Lc = cert_side(rep, n, g, lane, reinterpret_cast<double2*>(pos + jd.scr_off + (int64_t)r * kQuenchScr * n), lam,
+                                x0, y0);
     if (lane == 0) {
         const bool adaptive = (jd.flags & kMoveAdapt) != 0;
         const float cool = cool_of(adaptive, jm.xround);
@@ -1591,7 +1618,7 @@ __global__ void __launch_bounds__(32) trace_kernel(const int2* __restrict__ item
 }
 
 int launch_trace(cudaStream_t stream, int items, const int2* list, const JobDev* jdev, const JobMut* jmut,
-                 const float4* pos, TraceRec* out, size_t smem) {
+                 float4* pos, TraceRec* out, size_t smem) {
     static bool attr_done[64] = {false};
     int dev = 0;
     SQS_CUDA(cudaGetDevice(&dev));

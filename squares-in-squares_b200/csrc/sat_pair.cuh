@@ -40,10 +40,12 @@ __device__ __forceinline__ bool sat_pair_grad(float dx, float dy, float cp, floa
     const float cd = __fadd_rn(__fmul_rn(cp, cq), __fmul_rn(sp, sq));
     const float sd = __fsub_rn(__fmul_rn(sp, cq), __fmul_rn(cp, sq));
     const float rad = 0.5f + 0.5f * (fabsf(cd) + fabsf(sd));
-    const float v0 = dx * cp + dy * sp;
-    const float v1 = dy * cp - dx * sp;
-    const float v2 = dx * cq + dy * sq;
-    const float v3 = dy * cq - dx * sq;
+    // Projections with every rounding spelled out, as in sat_pair_energy: the
+    // quench compiles this into several group forms whose results must agree.
+    const float v0 = __fmaf_rn(dx, cp, __fmul_rn(dy, sp));
+    const float v1 = __fmaf_rn(dy, cp, -__fmul_rn(dx, sp));
+    const float v2 = __fmaf_rn(dx, cq, __fmul_rn(dy, sq));
+    const float v3 = __fmaf_rn(dy, cq, -__fmul_rn(dx, sq));
     const float z0 = fabsf(v0) - rad, z1 = fabsf(v1) - rad;
     const float z2 = fabsf(v2) - rad, z3 = fabsf(v3) - rad;
     const float gap = fmaxf(fmaxf(z0, z1), fmaxf(z2, z3));
