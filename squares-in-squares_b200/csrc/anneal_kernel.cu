@@ -174,10 +174,13 @@ __device__ __forceinline__ long long pair_delta(float4 Q, float nx, float ny, fl
     return (ex * ex + ey * ey < kPairCut2 ? en : 0) - (fx * fx + fy * fy < kPairCut2 ? eo : 0);
 }
 
+// Exact 64-bit warp sum in three warp reductions: the value's 26 low bits,
+// the next 26 and the signed rest each sum within 32 bits.
 __device__ __forceinline__ long long warp_sum_ll(long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    const unsigned s0 = __reduce_add_sync(0xffffffffu, (unsigned)v & 0x3ffffffu);
+    const unsigned s1 = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 26) & 0x3ffffffu);
+    const int s2 = __reduce_add_sync(0xffffffffu, (int)(v >> 52));
+    return (long long)(((unsigned long long)(long long)s2 << 52) + ((unsigned long long)s1 << 26) + s0);
 }
 
 __device__ __forceinline__ double warp_max_d(double v) {
@@ -297,46 +300,12 @@ __device__ double cert_side(const Rep& R, int n, const Grid& g, int lane, double
     return fmax(__dsub_rn(bx1, bx0), __dsub_rn(by1, by0));
 }
 
-__device__ long long block_sum_ll(long long v, long long* red);
-
-// Three sums at once over the warps w < nw of a group whose warp partials
-// go to red[3 w .. 3 w + 2]; `sync` orders the slots' writes and reads.
-template <class Sync>
-__device__ __forceinline__ void group_sum3(long long& a, long long& b, long long& c, long long* red, int wg, int nw,
-                                           Sync&& sync) {
-    a = warp_sum_ll(a);
-    b = warp_sum_ll(b);
-    c = warp_sum_ll(c);
-    sync();
-    if ((threadIdx.x & 31) == 0) {
-        red[3 * wg] = a;
-        red[3 * wg + 1] = b;
-        red[3 * wg + 2] = c;
-    }
-    sync();
-    a = b = c = 0;
-    for (int k = 0; k < nw; ++k) {
-        a += red[3 * k];
-        b += red[3 * k + 1];
-        c += red[3 * k + 2];
-    }
-}
-
-// ---- Cooperative forms: a group of threads works on one replica, either
-// the whole CTA (CtaGrp) or one warp (WarpGrp).  Results do not depend on the
-// group: every sum below is an integer sum and slot order within a cell list
-// changes no energy, gradient or decision.
-struct CtaGrp {
-    long long* red;  // one slot per warp of the CTA
-    __device__ __forceinline__ int t() const { return threadIdx.x; }
-    __device__ __forceinline__ int nt() const { return blockDim.x; }
-    __device__ __forceinline__ void sync() const { __syncthreads(); }
-    __device__ __forceinline__ bool sync_or(bool p) const { return __syncthreads_or(p); }
-    __device__ __forceinline__ long long sum(long long v) const { return block_sum_ll(v, red); }
-    __device__ __forceinline__ void sum3(long long& a, long long& b, long long& c) const {
-        group_sum3(a, b, c, red, (int)threadIdx.x >> 5, (int)(blockDim.x + 31) >> 5, [] { __syncthreads(); });
-    }
-};
+// ---- Cooperative forms: a group of warps works on one replica, one warp
+// (WarpGrp) or several on a named barrier (BarGrp).  Results do not depend on
+// the group: every sum below is an integer sum and slot order within a cell
+// list changes no energy, gradient or decision.  A group sum publishes one
+// partial a warp and takes one barrier; each kind of sum has its own slots,
+// and two sums of one kind always have another barrier between them.
 struct WarpGrp {
     int lane;
     __device__ __forceinline__ int t() const { return lane; }
@@ -352,37 +321,69 @@ struct WarpGrp {
         b = warp_sum_ll(b);
         c = warp_sum_ll(c);
     }
+    // group maximum of m and group OR of f; orders the group's memory like sync()
+    __device__ __forceinline__ void max_or(unsigned& m, bool& f) const {
+        m = __reduce_max_sync(0xffffffffu, m);
+        f = __any_sync(0xffffffffu, f);
+        __syncwarp();
+    }
 };
+constexpr int kGrpSlots = 5;  // three sums, the energy sum, maximum and flag
 // `nw` consecutive warps of the CTA (nw >= 2) on named barrier `id` (1..15).
+// The barrier is the non-aligned form: after a lane-strided loop nothing
+// promises that a warp reaches it converged.
 struct BarGrp {
     int id, nw, t0;  // barrier, warps, first thread of the group
-    long long* red;  // three slots per warp of the group
+    long long* red;  // kGrpSlots slots per warp of the group
     __device__ __forceinline__ int t() const { return (int)threadIdx.x - t0; }
     __device__ __forceinline__ int nt() const { return 32 * nw; }
     __device__ __forceinline__ void sync() const {
-        asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(32 * nw) : "memory");
+        asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(32 * nw) : "memory");
     }
     __device__ __forceinline__ bool sync_or(bool p) const {
         unsigned r;
         asm volatile(
-            "{\n\t.reg .pred ip, op;\n\tsetp.ne.u32 ip, %1, 0;\n\tbar.red.or.pred op, %2, %3, ip;\n\t"
+            "{\n\t.reg .pred ip, op;\n\tsetp.ne.u32 ip, %1, 0;\n\tbarrier.red.or.pred op, %2, %3, ip;\n\t"
             "selp.u32 %0, 1, 0, op;\n\t}"
             : "=r"(r)
             : "r"((unsigned)p), "r"(id), "r"(32 * nw)
             : "memory");
         return r != 0;
     }
+    __device__ __forceinline__ long long slot_sum(int k) const {
+        const int lane = threadIdx.x & 31;
+        return warp_sum_ll(lane < nw ? red[kGrpSlots * lane + k] : 0);
+    }
     __device__ __forceinline__ long long sum(long long v) const {
         v = warp_sum_ll(v);
-        sync();  // every read of the slots by the previous sum is done
-        if ((threadIdx.x & 31) == 0) red[t() >> 5] = v;
+        if ((threadIdx.x & 31) == 0) red[kGrpSlots * (t() >> 5) + 3] = v;
         sync();
-        long long s = 0;
-        for (int k = 0; k < nw; ++k) s += red[k];
-        return s;
+        return slot_sum(3);
     }
     __device__ __forceinline__ void sum3(long long& a, long long& b, long long& c) const {
-        group_sum3(a, b, c, red, t() >> 5, nw, [this] { sync(); });
+        a = warp_sum_ll(a);
+        b = warp_sum_ll(b);
+        c = warp_sum_ll(c);
+        if ((threadIdx.x & 31) == 0) {
+            long long* r = red + kGrpSlots * (t() >> 5);
+            r[0] = a;
+            r[1] = b;
+            r[2] = c;
+        }
+        sync();
+        a = slot_sum(0);
+        b = slot_sum(1);
+        c = slot_sum(2);
+    }
+    __device__ __forceinline__ void max_or(unsigned& m, bool& f) const {
+        m = __reduce_max_sync(0xffffffffu, m);
+        f = __any_sync(0xffffffffu, f);
+        const int lane = threadIdx.x & 31;
+        if (lane == 0) red[kGrpSlots * (t() >> 5) + 4] = (long long)(((unsigned long long)f << 32) | m);
+        sync();
+        const unsigned long long v = lane < nw ? (unsigned long long)red[kGrpSlots * lane + 4] : 0ull;
+        m = __reduce_max_sync(0xffffffffu, (unsigned)v);
+        f = __any_sync(0xffffffffu, (v >> 32) != 0);
     }
 };
 
@@ -409,21 +410,10 @@ __device__ bool build_cells_grp(const Grp& gp, const Rep& R, int n, const Grid& 
     return !bad;
 }
 
-__device__ long long block_sum_ll(long long v, long long* red) {
-    v = warp_sum_ll(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    __syncthreads();
-    if (lane == 0) red[w] = v;
-    __syncthreads();
-    long long t = 0;
-    for (int k = 0; k < nw; ++k) t += red[k];
-    return t;
-}
-
-// Full fixed-point energy by the whole CTA.  Work item w is square w / 9
-// against the squares listed in cell w % 9 of its 3 x 3 block (each pair
-// counted from its lower index), so a small replica still spreads over
-// many threads.
+// Full fixed-point energy of a trial state on the lists of the state it
+// moved from.  Work item w is square w / 9 against the squares listed in cell
+// w % 9 of its 3 x 3 block, each pair counted from its lower index (the half
+// block of full_energy needs current lists).
 template <class Grp>
 __device__ long long full_energy_grp(const Grp& gp, const Rep& R, int n, const Grid& g, float L) {
     long long e = 0;
@@ -482,171 +472,187 @@ __device__ __forceinline__ long long clamp_q24(int v) { return max(-(1 << 24), m
 // The checkpoint quench of one replica (the coldest, or each one under
 // SQS_JOB_QUENCH_ALL) by a group of threads: the reference's conjugate-gradient
 // polish (seeded.cu:621-715) on the overlap energy.  Each iteration takes the
-// gradient (one thread per (square, neighbouring cell) work item), a
-// Polak-Ribiere direction d = -g + beta d (beta = max(0, (g - g_old).g /
-// g_old.g), 0 on the first iteration and every 25th), and a backtracking
-// line search of up to 5 trials from the carried step (x 0.45 per trial).
-// An accepted trial sets the step to min(0.15, 1.25 alpha); when no trial
-// improves, the state goes back, the direction is dropped and the step
-// halves (at least 1e-7) -- the polish goes on, it does not stop there.  It
-// ends at zero energy, at a zero gradient, after `iters` iterations, or, with
-// a stall limit (not kQuenchNoStall), after `stall_limit` accepted steps in a
-// row that each gained less than 0.1% or at a line search without a gain.
+// gradient, a Polak-Ribiere direction d = -g + beta d (beta = max(0, (g -
+// g_old).g / g_old.g), 0 on the first iteration and every 25th), and a
+// backtracking line search of up to 5 trials from the carried step (x 0.45
+// per trial).  An accepted trial sets the step to min(0.15, 1.25 alpha); when
+// no trial improves, the direction is dropped and the step halves (at least
+// 1e-7) -- the polish goes on from the same state, whose gradient is kept.
+// It ends at zero energy, at a zero gradient, after `iters` iterations, or,
+// with a stall limit (not kQuenchNoStall), after `stall_limit` accepted steps
+// in a row that each gained less than 0.1% or at a line search without a gain.
 // Gradients and their dot products are integer sums, so the result does not
-// depend on the group's width.  Scratch: kQuenchScr n float4 (gradient sums,
-// previous gradient, direction, saved state, pair list: a counter, the
-// largest direction component and up to 8 n - 2 pairs).
+// depend on the group's width.
+//
+// A step is a chain of short phases with a group barrier after each, so the
+// barriers are what it costs: an accepted first trial takes four (gradient;
+// dot products; direction, trial state, largest component and cell changes
+// at once; energy).  Square i belongs to thread i mod nt throughout, so what
+// only its owner reads (direction, saved state, old gradient) needs none, and
+// the cell lists are rebuilt only when a square of the accepted trial has
+// left its cell.  Scratch: kQuenchScr n float4 (gradient sums of this and of
+// the previous iteration, direction, saved state, pair list: two counters and
+// up to 8 n - 2 pairs).
 template <class Grp>
 __device__ long long quench_grp(const Grp& gp, const Rep& R, int n, const Grid& g, float L, int iters, int stall_limit,
                                 float4* scr, long long E) {
-    int4* acc = reinterpret_cast<int4*>(scr);       // gradient sums of this iteration
-    int4* gold = reinterpret_cast<int4*>(scr + n);  // the previous iteration's
+    int4* acc = reinterpret_cast<int4*>(scr);       // gradient sums at the current state
+    int4* gold = reinterpret_cast<int4*>(scr + n);  // at the state before (zero once consumed)
     float4* dir = scr + 2 * n;                      // search direction
     float4* saved = scr + 3 * n;                    // state before the line search
-    uint32_t* plist = reinterpret_cast<uint32_t*>(scr + 4 * n);  // [0] count, [1] max |d|, pairs
+    uint32_t* plist = reinterpret_cast<uint32_t*>(scr + 4 * n);  // [cur] count, [cur ^ 1] zero, pairs
     const int pcap = 8 * n - 2;
     float step = 0.04f;
     int stall = 0;  // consecutive accepted steps that gained less than 0.1%
     float drift = 1e30f;  // bound on any centre's per-axis move since the pair list was built (none yet)
+    int cur = 0;          // the pair list's counter
+    bool fresh = true;    // the state moved since its gradient was taken
+    bool away = false;    // the replica holds a rejected trial, not the saved state
+    long long s_gg = 0;
     for (int i = gp.t(); i < n; i += gp.nt()) {
+        acc[i] = make_int4(0, 0, 0, 0);
         gold[i] = make_int4(0, 0, 0, 0);
         dir[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        saved[i] = make_float4(R.sq[i].x, R.sq[i].y, R.ang[i], 0.f);
     }
+    if (gp.t() == 0) plist[0] = plist[1] = 0u;
+    gp.sync();
+    auto restore = [&]() {  // the owner's squares back to the saved state
+        for (int i = gp.t(); i < n; i += gp.nt()) {
+            const float4 o = saved[i];
+            float sn, cs;
+            state_trig(o.z, &sn, &cs);
+            R.sq[i] = make_float4(o.x, o.y, cs, sn);
+            R.ang[i] = o.z;
+        }
+        gp.sync();
+    };
     for (int it = 0; it < iters && E > 0; ++it) {
-        for (int i = gp.t(); i < n; i += gp.nt()) {
-            acc[i] = make_int4(0, 0, 0, 0);
-            saved[i] = make_float4(R.sq[i].x, R.sq[i].y, R.ang[i], 0.f);
-        }
-        // the pair list stays exact while no centre has moved more than
-        // kListStep per axis since it was built; past that it is rebuilt
-        const bool rebuild = !(drift <= kListStep);
-        if (gp.t() == 0) {
-            if (rebuild) plist[0] = 0u;
-            plist[1] = 0u;
-        }
-        gp.sync();
-        if (!rebuild) {
-            // gradient over the list: walls, then both sides of every pair
-            // within the cut-off (the cell scan's operations and sums)
-            for (int i = gp.t(); i < n; i += gp.nt()) {
-                const float4 P = R.sq[i];
-                float wx = 0.f, wy = 0.f, wa = 0.f;
-                wall_energy_grad(P.x, P.y, P.z, P.w, L, wx, wy, wa);
-                const int ax = qg(wx), ay = qg(wy), aa = qg(wa);
-                if (ax | ay | aa) {
-                    atomicAdd(&acc[i].x, ax);
-                    atomicAdd(&acc[i].y, ay);
-                    atomicAdd(&acc[i].z, aa);
+        float beta = 0.f;
+        if (fresh) {
+            // the pair list stays exact while no centre has moved more than
+            // kListStep per axis since it was built; past that it is rebuilt
+            const bool rebuild = !(drift <= kListStep);
+            if (!rebuild) {
+                // gradient over the list: walls, then both sides of every pair
+                // within the cut-off (the cell scan's operations and sums)
+                for (int i = gp.t(); i < n; i += gp.nt()) {
+                    const float4 P = R.sq[i];
+                    float wx = 0.f, wy = 0.f, wa = 0.f;
+                    wall_energy_grad(P.x, P.y, P.z, P.w, L, wx, wy, wa);
+                    const int ax = qg(wx), ay = qg(wy), aa = qg(wa);
+                    if (ax | ay | aa) {
+                        atomicAdd(&acc[i].x, ax);
+                        atomicAdd(&acc[i].y, ay);
+                        atomicAdd(&acc[i].z, aa);
+                    }
                 }
-            }
-            const int np = (int)plist[0];
-            for (int k = gp.t(); k < np; k += gp.nt()) {
-                const uint32_t pr = plist[2 + k];
-                const int i = (int)(pr & 0xffffu), j = (int)(pr >> 16);
-                const float4 P = R.sq[i], Q = R.sq[j];
-                const float ex = Q.x - P.x, ey = Q.y - P.y;
-                if (ex * ex + ey * ey >= kPairCut2) continue;
-                PairGrad pg;
-                if (sat_pair_grad(ex, ey, P.z, P.w, Q.z, Q.w, pg)) {
-                    atomicAdd(&acc[i].x, qg(pg.px));
-                    atomicAdd(&acc[i].y, qg(pg.py));
-                    atomicAdd(&acc[i].z, qg(pg.pa));
-                }
-                if (sat_pair_grad(P.x - Q.x, P.y - Q.y, Q.z, Q.w, P.z, P.w, pg)) {
-                    atomicAdd(&acc[j].x, qg(pg.px));
-                    atomicAdd(&acc[j].y, qg(pg.py));
-                    atomicAdd(&acc[j].z, qg(pg.pa));
-                }
-            }
-        }
-        // work item w: square w / 9 against cell w % 9 of its block; it also
-        // lists the block's pairs (i < j) closer than sqrt(kListCut2)
-        for (int w = gp.t(); rebuild && w < 9 * n; w += gp.nt()) {
-            const int i = w / 9, c = w - 9 * i;
-            const float4 P = R.sq[i];
-            int ax = 0, ay = 0, aa = 0;
-            if (c == 0) {
-                float wx = 0.f, wy = 0.f, wa = 0.f;
-                wall_energy_grad(P.x, P.y, P.z, P.w, L, wx, wy, wa);
-                ax = qg(wx);
-                ay = qg(wy);
-                aa = qg(wa);
-            }
-            const int x = g.cx(P.x) + c % 3 - 1, y = g.cx(P.y) + c / 3 - 1;
-            if (x >= 0 && x < g.G && y >= 0 && y < g.G) {
-                const int cell = y * g.G + x, m = R.cnt[cell];
-                for (int k = 0; k < m; ++k) {
-                    const int j = R.slot[cell * kCellK + k];
-                    if (j == i) continue;
-                    const float4 Q = R.sq[j];
+                const int np = (int)plist[cur];
+                for (int k = gp.t(); k < np; k += gp.nt()) {
+                    const uint32_t pr = plist[2 + k];
+                    const int i = (int)(pr & 0xffffu), j = (int)(pr >> 16);
+                    const float4 P = R.sq[i], Q = R.sq[j];
                     const float ex = Q.x - P.x, ey = Q.y - P.y;
-                    const float d2 = ex * ex + ey * ey;
-                    if (j > i && d2 < kListCut2) {
-                        const uint32_t slot = atomicAdd(&plist[0], 1u);
-                        if (slot < (uint32_t)pcap) plist[2 + slot] = (uint32_t)i | ((uint32_t)j << 16);
-                    }
-                    if (d2 >= kPairCut2) continue;
-                    PairGrad pg;
+                    if (ex * ex + ey * ey >= kPairCut2) continue;
+                    PairGrad pg;  // q's side equals the pair taken from q, bit for bit
                     if (sat_pair_grad(ex, ey, P.z, P.w, Q.z, Q.w, pg)) {
-                        ax += qg(pg.px);
-                        ay += qg(pg.py);
-                        aa += qg(pg.pa);
+                        atomicAdd(&acc[i].x, qg(pg.px));
+                        atomicAdd(&acc[i].y, qg(pg.py));
+                        atomicAdd(&acc[i].z, qg(pg.pa));
+                        atomicAdd(&acc[j].x, qg(pg.qx));
+                        atomicAdd(&acc[j].y, qg(pg.qy));
+                        atomicAdd(&acc[j].z, qg(pg.qa));
+                    }
+                }
+            } else {
+                // work item w: square w / 9 against cell w % 9 of its block; it also
+                // lists the block's pairs (i < j) closer than sqrt(kListCut2)
+                cur ^= 1;
+                for (int w = gp.t(); w < 9 * n; w += gp.nt()) {
+                    const int i = w / 9, c = w - 9 * i;
+                    const float4 P = R.sq[i];
+                    int ax = 0, ay = 0, aa = 0;
+                    if (c == 0) {
+                        float wx = 0.f, wy = 0.f, wa = 0.f;
+                        wall_energy_grad(P.x, P.y, P.z, P.w, L, wx, wy, wa);
+                        ax = qg(wx);
+                        ay = qg(wy);
+                        aa = qg(wa);
+                    }
+                    const int x = g.cx(P.x) + c % 3 - 1, y = g.cx(P.y) + c / 3 - 1;
+                    if (x >= 0 && x < g.G && y >= 0 && y < g.G) {
+                        const int cell = y * g.G + x, m = R.cnt[cell];
+                        for (int k = 0; k < m; ++k) {
+                            const int j = R.slot[cell * kCellK + k];
+                            if (j == i) continue;
+                            const float4 Q = R.sq[j];
+                            const float ex = Q.x - P.x, ey = Q.y - P.y;
+                            const float d2 = ex * ex + ey * ey;
+                            if (j > i && d2 < kListCut2) {
+                                const uint32_t slot = atomicAdd(&plist[cur], 1u);
+                                if (slot < (uint32_t)pcap) plist[2 + slot] = (uint32_t)i | ((uint32_t)j << 16);
+                            }
+                            if (d2 >= kPairCut2) continue;
+                            PairGrad pg;
+                            if (sat_pair_grad(ex, ey, P.z, P.w, Q.z, Q.w, pg)) {
+                                ax += qg(pg.px);
+                                ay += qg(pg.py);
+                                aa += qg(pg.pa);
+                            }
+                        }
+                    }
+                    if (ax | ay | aa) {
+                        atomicAdd(&acc[i].x, ax);
+                        atomicAdd(&acc[i].y, ay);
+                        atomicAdd(&acc[i].z, aa);
                     }
                 }
             }
-            if (ax | ay | aa) {
-                atomicAdd(&acc[i].x, ax);
-                atomicAdd(&acc[i].y, ay);
-                atomicAdd(&acc[i].z, aa);
+            gp.sync();
+            if (rebuild) drift = plist[cur] <= (uint32_t)pcap ? 0.f : 1e30f;  // an overflowed list is not used
+            // Polak-Ribiere: g_old.g_old, (g - g_old).g and g.g as exact integer
+            // sums of components clamped to 2^24 (a gradient of 16; only beta
+            // sees the clamp): 3 n <= 3000 terms below 2^49 each fit 64 bits
+            long long s_oo = 0, s_dg = 0;
+            s_gg = 0;
+            for (int i = gp.t(); i < n; i += gp.nt()) {
+                const int4 a = acc[i], o = gold[i];
+                const long long gx = clamp_q24(a.x), gy = clamp_q24(a.y), ga = clamp_q24(a.z);
+                const long long ox = clamp_q24(o.x), oy = clamp_q24(o.y), oa = clamp_q24(o.z);
+                s_oo += ox * ox + oy * oy + oa * oa;
+                s_dg += (gx - ox) * gx + (gy - oy) * gy + (ga - oa) * ga;
+                s_gg += gx * gx + gy * gy + ga * ga;
             }
+            gp.sum3(s_oo, s_dg, s_gg);
+            beta = (it == 0 || s_oo == 0 || it % 25 == 0) ? 0.f : fmaxf(0.f, (float)((double)s_dg / (double)s_oo));
         }
-        gp.sync();
-        if (rebuild) drift = plist[0] <= (uint32_t)pcap ? 0.f : 1e30f;  // an overflowed list is not used
-        // Polak-Ribiere: g_old.g_old, (g - g_old).g and g.g as exact integer
-        // sums of components clamped to 2^24 (a gradient of 16; only beta
-        // sees the clamp): 3 n <= 3000 terms below 2^49 each fit 64 bits
-        long long s_oo = 0, s_dg = 0, s_gg = 0;
-        for (int i = gp.t(); i < n; i += gp.nt()) {
-            const int4 a = acc[i], o = gold[i];
-            const long long gx = clamp_q24(a.x), gy = clamp_q24(a.y), ga = clamp_q24(a.z);
-            const long long ox = clamp_q24(o.x), oy = clamp_q24(o.y), oa = clamp_q24(o.z);
-            s_oo += ox * ox + oy * oy + oa * oa;
-            s_dg += (gx - ox) * gx + (gy - oy) * gy + (ga - oa) * ga;
-            s_gg += gx * gx + gy * gy + ga * ga;
-        }
-        gp.sum3(s_oo, s_dg, s_gg);
-        const float beta =
-            (it == 0 || s_oo == 0 || it % 25 == 0) ? 0.f : fmaxf(0.f, (float)((double)s_dg / (double)s_oo));
         if (s_gg == 0 && beta == 0.f) break;  // no direction left at the sums' resolution
-        uint32_t dmax_bits = 0u;  // largest |d.x|, |d.y| (bits of non-negative floats order as integers)
-        for (int i = gp.t(); i < n; i += gp.nt()) {
-            const int4 a = acc[i];
-            const float4 d0 = dir[i];
-            const float4 d1 = make_float4(__fmaf_rn(beta, d0.x, -(float)a.x * (1.0f / kQScale)),
-                                          __fmaf_rn(beta, d0.y, -(float)a.y * (1.0f / kQScale)),
-                                          __fmaf_rn(beta, d0.z, -(float)a.z * (1.0f / kQScale)), 0.f);
-            dir[i] = d1;
-            gold[i] = a;
-            dmax_bits = max(dmax_bits, __float_as_uint(fmaxf(fabsf(d1.x), fabsf(d1.y))));
-        }
-        dmax_bits = __reduce_max_sync(0xffffffffu, dmax_bits);
-        if ((threadIdx.x & 31) == 0) atomicMax(&plist[1], dmax_bits);
-        gp.sync();
-        const int npairs = (int)plist[0];
-        const float dmax = __uint_as_float(plist[1]);
+        const int npairs = (int)plist[cur];
+        float dmax = 0.f;
         // Trial steps move every coordinate by at most 0.1, so each partner
         // within the pair cut-off of a moved square still sits in one of the
         // 3 x 3 cells around it on the lists built for the saved state
-        // (1.4142 + 0.1 < 1.59 <= cell side): trial energies use those lists,
-        // and the lists are rebuilt only for an accepted step.  A trial that
-        // keeps every centre within kListStep per axis of where the pair list
-        // was built sums the list instead (the same energy, without the cell
-        // scan).
+        // (1.4142 + 0.1 < 1.59 <= cell side): trial energies use those lists.
+        // A trial that keeps every centre within kListStep per axis of where
+        // the pair list was built sums the list instead (the same energy,
+        // without the cell scan).
         float alpha = step;
         bool moved = false;
         for (int tries = 0; tries < 5 && !moved; ++tries) {
+            unsigned dbits = 0u;  // largest |d.x|, |d.y| (bits of non-negative floats order as integers)
+            bool left = false;    // a square left its cell
             for (int i = gp.t(); i < n; i += gp.nt()) {
-                const float4 d = dir[i], o = saved[i];
+                float4 d = dir[i];
+                if (tries == 0) {
+                    const int4 a = acc[i];
+                    d = make_float4(__fmaf_rn(beta, d.x, -(float)a.x * (1.0f / kQScale)),
+                                    __fmaf_rn(beta, d.y, -(float)a.y * (1.0f / kQScale)),
+                                    __fmaf_rn(beta, d.z, -(float)a.z * (1.0f / kQScale)), 0.f);
+                    dir[i] = d;
+                    gold[i] = make_int4(0, 0, 0, 0);  // consumed: the next gradient is summed here
+                    dbits = max(dbits, __float_as_uint(fmaxf(fabsf(d.x), fabsf(d.y))));
+                }
+                const float4 o = saved[i];
                 const float sx = fminf(0.1f, fmaxf(-0.1f, alpha * d.x));
                 const float sy = fminf(0.1f, fmaxf(-0.1f, alpha * d.y));
                 float a = o.z + fminf(0.1f, fmaxf(-0.1f, alpha * d.z));
@@ -654,49 +660,61 @@ __device__ long long quench_grp(const Grp& gp, const Rep& R, int n, const Grid& 
                 if (!(a >= 0.f && a < kHalfPiF)) a = 0.f;
                 float sn, cs;
                 state_trig(a, &sn, &cs);
-                R.sq[i] = make_float4(o.x + sx, o.y + sy, cs, sn);
+                const float nx = o.x + sx, ny = o.y + sy;
+                R.sq[i] = make_float4(nx, ny, cs, sn);
                 R.ang[i] = a;
+                left |= g.cx(nx) != g.cx(o.x) || g.cx(ny) != g.cx(o.y);
             }
-            gp.sync();
+            if (tries == 0 && gp.t() == 0) plist[cur ^ 1] = 0u;
+            gp.max_or(dbits, left);
+            if (tries == 0) dmax = __uint_as_float(dbits);
             const bool by_list = npairs <= pcap && drift + alpha * dmax <= kListStep;
             const long long En = by_list ? list_energy(gp, R, n, L, plist + 2, npairs) : full_energy_grp(gp, R, n, g, L);
-            if (En < E && build_cells_grp(gp, R, n, g)) {
+            if (En < E && (!left || build_cells_grp(gp, R, n, g))) {
                 stall = En > E - E / 1000 ? stall + 1 : 0;  // less than 0.1% gained
                 E = En;
                 step = fminf(0.15f, alpha * 1.25f);
                 drift += fminf(0.1f, alpha * dmax);  // every centre moved at most this far per axis
                 moved = true;
+                for (int i = gp.t(); i < n; i += gp.nt())
+                    saved[i] = make_float4(R.sq[i].x, R.sq[i].y, R.ang[i], 0.f);
             } else {
                 if (En < E) {  // the better state overflows a cell: lists back to the saved state
-                    for (int i = gp.t(); i < n; i += gp.nt()) {
-                        const float4 o = saved[i];
-                        float sn, cs;
-                        state_trig(o.z, &sn, &cs);
-                        R.sq[i] = make_float4(o.x, o.y, cs, sn);
-                        R.ang[i] = o.z;
-                    }
-                    gp.sync();
+                    restore();
                     build_cells_grp(gp, R, n, g);  // the saved state fitted
                 }
                 alpha *= 0.45f;
             }
         }
-        if (!moved) {  // back to the saved state (its lists are current), direction dropped
-            for (int i = gp.t(); i < n; i += gp.nt()) {
-                const float4 o = saved[i];
-                float sn, cs;
-                state_trig(o.z, &sn, &cs);
-                R.sq[i] = make_float4(o.x, o.y, cs, sn);
-                R.ang[i] = o.z;
-                dir[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+        fresh = moved;
+        away = !moved;
+        if (moved) {
+            int4* const s = acc;
+            acc = gold;
+            gold = s;
+        } else {  // direction dropped (beta is 0 next), the saved state's gradient kept
             step = fmaxf(1e-7f, step * 0.5f);
-            gp.sync();
             if (stall_limit < kQuenchNoStall) break;  // the library's default quench ends here
         }
         if (stall >= stall_limit) break;
     }
+    if (away) restore();  // the lists are those of the saved state
     return E;
+}
+
+// Quench of replica view R by warps 0 .. gw - 1 of a group that starts at
+// thread t0 (all of them call this): one warp a 16 squares, at most gw.  More
+// warps than that add barrier latency and no parallelism (n = 10: one warp
+// against eight, with the phases above, took 400 checkpoints from 87 to 76 ms;
+// n = 50, 64 chains: 55.8 ms, 56.0 with 8 squares a warp, 61.1 with 32).
+constexpr int kQuenchSquares = 16;
+__device__ __forceinline__ long long quench_group(int id, int gw, int t0, long long* red, const Rep& R, int n,
+                                                  const Grid& g, float L, int iters, int stall_limit, float4* scr,
+                                                  long long E) {
+    const int nw = min(gw, (n + kQuenchSquares - 1) / kQuenchSquares), t = (int)threadIdx.x - t0;
+    if (t >= 32 * nw) return E;
+    if (nw == 1) return quench_grp(WarpGrp{t}, R, n, g, L, iters, stall_limit, scr, E);
+    return quench_grp(BarGrp{id, nw, t0, red}, R, n, g, L, iters, stall_limit, scr, E);
 }
 
 __device__ __forceinline__ float wrap_quarter_f(float a) {
@@ -949,9 +967,10 @@ struct CtaShared {
     int reset0;                // SQS_JOB_TARGETS: the gain resets every rung of ladder 0, not only heads
     float newL;
     unsigned long long props[kMaxRl], accs[kMaxRl];
-    long long red[3 * kMaxRl];   // group sums: up to three values a warp
+    long long red[kGrpSlots * kMaxRl];  // group sums: kGrpSlots values a warp
     long long qE;              // energy of the replica quenched by this CTA
-    long long qEv[kMaxRl];     // each replica's energy through a group quench
+    long long qEv[kMaxRl];     // each replica's energy before a group quench
+    long long qEnew[kMaxRl];   // and after it
 };
 
 // MOVES: whether the move-set options (adaptation, collective moves, kicks)
@@ -1306,19 +1325,19 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                 if (active && lane == 0) S.qEv[w] = E;
                 __syncthreads();
                 if (q < Rl) {
-                    const BarGrp gp{1 + q, gw, q * gw * 32, S.red + 3 * q * gw};
                     const Rep cr = rep_view(dyn + q * rb, n, jd.Gmax);
-                    const long long e =
-                        quench_grp(gp, cr, n, g, S.wside[q], jd.quench_iters, jd.quench_stall, qw, S.qEv[q]);
-                    if (gp.t() == 0) S.qEv[q] = e;
+                    const long long e0 = S.qEv[q];
+                    __syncwarp();
+                    const long long e = quench_group(1 + q, gw, q * gw * 32, S.red + kGrpSlots * q * gw, cr, n, g,
+                                                     S.wside[q], jd.quench_iters, jd.quench_stall, qw, e0);
+                    if (tid == q * gw * 32) S.qEnew[q] = e;
                 }
                 __syncthreads();
-                if (active) E = S.qEv[w];
+                if (active) E = S.qEnew[w];
             }
             __syncthreads();
         } else {
-            // the replica on the coldest rung, by every thread of the CTA that
-            // holds it; its scratch in shared memory after the replicas when
+            // the replica on the coldest rung, by warps of the CTA that holds it; its scratch in shared memory after the replicas when
             // the launch left room, else this CTA's block of the job's scratch
             float4* qs = (int64_t)dyn_bytes >= (int64_t)Rl * rb + (int64_t)sizeof(float4) * kQuenchScr * n
                              ? reinterpret_cast<float4*>(dyn + (int64_t)Rl * rb)
@@ -1330,10 +1349,11 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                 if (w == cold % Rl && lane == 0) S.qE = E;
                 __syncthreads();
                 const Rep cr = rep_view(dyn + (cold % Rl) * rb, n, jd.Gmax);
-                const long long qe_out = quench_grp(CtaGrp{S.red}, cr, n, g, S.wside[cold % Rl], jd.quench_iters,
-                                                    jd.quench_stall, qs, S.qE);
-                if (w == cold % Rl) E = qe_out;
+                const long long e = quench_group(1, (int)(blockDim.x >> 5), 0, S.red, cr, n, g, S.wside[cold % Rl],
+                                                 jd.quench_iters, jd.quench_stall, qs, S.qE);
+                if (tid == 0) S.qEnew[0] = e;
                 __syncthreads();
+                if (w == cold % Rl) E = S.qEnew[0];
             }
         }
         if (active) {
