@@ -32,24 +32,32 @@ struct PairGrad {
     float qx, qy, qa;   // d e / d q
 };
 
-// Evaluate an overlapping pair.  Returns false (and leaves g untouched) when
-// the squares do not overlap.  cp, sp: cos/sin of p's angle; cq, sq of q's.
-__device__ __forceinline__ bool sat_pair_grad(float dx, float dy, float cp, float sp, float cq,
-                                              float sq, PairGrad& g) {
-    // Products kept unfused so that equal angles give sd == 0 exactly.
-    const float cd = __fadd_rn(__fmul_rn(cp, cq), __fmul_rn(sp, sq));
-    const float sd = __fsub_rn(__fmul_rn(sp, cq), __fmul_rn(cp, sq));
-    const float rad = 0.5f + 0.5f * (fabsf(cd) + fabsf(sd));
-    // Projections with every rounding spelled out, as in sat_pair_energy: the
-    // quench compiles this into several group forms whose results must agree.
-    const float v0 = __fmaf_rn(dx, cp, __fmul_rn(dy, sp));
-    const float v1 = __fmaf_rn(dy, cp, -__fmul_rn(dx, sp));
-    const float v2 = __fmaf_rn(dx, cq, __fmul_rn(dy, sq));
-    const float v3 = __fmaf_rn(dy, cq, -__fmul_rn(dx, sq));
-    const float z0 = fabsf(v0) - rad, z1 = fabsf(v1) - rad;
-    const float z2 = fabsf(v2) - rad, z3 = fabsf(v3) - rad;
-    const float gap = fmaxf(fmaxf(z0, z1), fmaxf(z2, z3));
-    if (!(gap < 0.f)) return false;
+// The four projections of a pair and its gap (the largest |v_k| - r).
+struct PairAxes {
+    float cd, sd, rad, v0, v1, v2, v3, gap;
+};
+
+// Products kept unfused so that equal angles give sd == 0 exactly, and every
+// rounding spelled out as in sat_pair_energy: gap^2 is that energy bit for
+// bit, and the kernels that compile this in several forms agree.
+__device__ __forceinline__ PairAxes sat_axes(float dx, float dy, float cp, float sp, float cq, float sq) {
+    PairAxes a;
+    a.cd = __fadd_rn(__fmul_rn(cp, cq), __fmul_rn(sp, sq));
+    a.sd = __fsub_rn(__fmul_rn(sp, cq), __fmul_rn(cp, sq));
+    a.rad = 0.5f + 0.5f * (fabsf(a.cd) + fabsf(a.sd));
+    a.v0 = __fmaf_rn(dx, cp, __fmul_rn(dy, sp));
+    a.v1 = __fmaf_rn(dy, cp, -__fmul_rn(dx, sp));
+    a.v2 = __fmaf_rn(dx, cq, __fmul_rn(dy, sq));
+    a.v3 = __fmaf_rn(dy, cq, -__fmul_rn(dx, sq));
+    a.gap = fmaxf(fmaxf(fabsf(a.v0), fabsf(a.v1)), fmaxf(fabsf(a.v2), fabsf(a.v3))) - a.rad;
+    return a;
+}
+
+// Energy and gradients of a pair with gap < 0.
+__device__ __forceinline__ void sat_grad(const PairAxes& a, float cp, float sp, float cq, float sq, PairGrad& g) {
+    const float cd = a.cd, sd = a.sd, v0 = a.v0, v1 = a.v1, v2 = a.v2, v3 = a.v3, gap = a.gap;
+    const float z0 = fabsf(v0) - a.rad, z1 = fabsf(v1) - a.rad;
+    const float z2 = fabsf(v2) - a.rad, z3 = fabsf(v3) - a.rad;
     const float deriv = 0.5f * (sgnf(sd) * cd - sgnf(cd) * sd);
     const float two_gap = 2.f * gap;
     g.e = gap * gap;
@@ -69,7 +77,7 @@ __device__ __forceinline__ bool sat_pair_grad(float dx, float dy, float cp, floa
         g.qx = -g.px;
         g.qy = -g.py;
         g.qa = two_gap * (tq + deriv);
-        return true;
+        return;
     }
     // first maximum in order 0,1,2,3 (gradient of p), as selects
     {
@@ -95,6 +103,15 @@ __device__ __forceinline__ bool sat_pair_grad(float dx, float dy, float cp, floa
         g.qy = two_gap * s * uy;
         g.qa = two_gap * (torque + deriv);
     }
+}
+
+// Evaluate an overlapping pair.  Returns false (and leaves g untouched) when
+// the squares do not overlap.  cp, sp: cos/sin of p's angle; cq, sq of q's.
+__device__ __forceinline__ bool sat_pair_grad(float dx, float dy, float cp, float sp, float cq,
+                                              float sq, PairGrad& g) {
+    const PairAxes a = sat_axes(dx, dy, cp, sp, cq, sq);
+    if (!(a.gap < 0.f)) return false;
+    sat_grad(a, cp, sp, cq, sq, g);
     return true;
 }
 
