@@ -115,36 +115,43 @@ __device__ bool build_cells(const Rep& R, int n, const Grid& g, int lane) {
     return ok;
 }
 
-// Visit the squares of the 3x3 cell block around (cx, cy): returns through
-// `fn(j)` for every candidate t = lane, lane + kStride, ... (kStride lanes
-// share the block: the whole warp, or one half of it).
+// Visit the squares of the 3x3 cell block around (cx, cy): calls fn(j) for
+// every candidate t = lane, lane + kStride, ... (kStride lanes share the
+// block: the whole warp, or a part of it).  The three counts of a block row
+// are neighbouring bytes: two aligned word loads and a funnel shift fetch
+// them (the word past the counts is the slots'), and one multiplication turns
+// them into running sums, a byte each.  Slot t of the block is then found by
+// two compares for its row and two for its cell.  Against nine guarded byte
+// loads, a nine-step sum and an eight-step search this halves the instructions
+// around a candidate.
 template <int kStride = 32, typename Fn>
 __device__ __forceinline__ void for_block(const Rep& R, const Grid& g, int cx, int cy, int lane, Fn&& fn) {
-    // Every lane reads the nine cell counts (broadcast shared loads) and
-    // forms their running sum; slot t of the block belongs to the first cell
-    // whose running count exceeds t.  Lanes take slots 32 apart.  The cell
-    // of slot t is rebuilt from (cx, cy) and its index in the block, so no
-    // per-lane array is indexed at run time.
-    int ends[9];
-    int run = 0;
+    const unsigned mask = cx == g.G - 1 ? 0x00ffffu : 0xffffffu;
+    const int xs = cx > 0 ? cx - 1 : 0;
+    unsigned p[3];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) {
-        const int x = cx + c % 3 - 1, y = cy + c / 3 - 1;
-        const bool in = (unsigned)x < (unsigned)g.G && (unsigned)y < (unsigned)g.G;
-        run += in ? (int)R.cnt[y * g.G + x] : 0;
-        ends[c] = run;
-    }
-    for (int t = lane; t < run; t += kStride) {
-        int c = 0, start = 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const bool past = t >= ends[k];
-            c = past ? k + 1 : c;
-            start = past ? ends[k] : start;
+    for (int r = 0; r < 3; ++r) {
+        const int y = cy + r - 1;
+        unsigned w = 0u;
+        if ((unsigned)y < (unsigned)g.G) {
+            const int a = y * g.G + xs;
+            const uint32_t* q = reinterpret_cast<const uint32_t*>(R.cnt + (a & ~3));
+            w = __funnelshift_r(q[0], q[1], 8 * (a & 3));
+            w = (cx > 0 ? w : w << 8) & mask;
         }
-        const int cr = (c * 43) >> 7;  // c / 3 for c < 9
-        const int cell = (cy + cr - 1) * g.G + cx + (c - 3 * cr) - 1;
-        fn((int)R.slot[cell * kCellK + (t - start)]);
+        p[r] = w * 0x010101u;  // bytes: c0, c0 + c1, c0 + c1 + c2
+    }
+    const int t0 = (p[0] >> 16) & 0xff, t1 = t0 + (int)((p[1] >> 16) & 0xff), run = t1 + (int)((p[2] >> 16) & 0xff);
+    const int cell0 = (cy - 1) * g.G + cx - 1;
+    for (int t = lane; t < run; t += kStride) {
+        const bool r1 = t >= t0, r2 = t >= t1;
+        const unsigned q = r2 ? p[2] : (r1 ? p[1] : p[0]);
+        const int u = t - (r2 ? t1 : (r1 ? t0 : 0));
+        const int row = cell0 + (r2 ? 2 * g.G : (r1 ? g.G : 0));
+        const int c0 = q & 0xff, c1 = (q >> 8) & 0xff;
+        const bool k1 = u >= c0, k2 = u >= c1;
+        const int cell = row + (int)k1 + (int)k2;
+        fn((int)R.slot[cell * kCellK + u - (k2 ? c1 : (k1 ? c0 : 0))]);
     }
 }
 
@@ -1189,6 +1196,13 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
         const int64_t next_cp = min(P_total, (p_at / xp + 1) * xp);
         const int64_t stop = min(next_cp, p_end);
         if (active) {
+            const bool small = !MOVES && n <= 32;
+            float4 own = make_float4(0.f, 0.f, 1.f, 0.f);
+            int own_cell = -1;
+            if (small && lane < n) {
+                own = rep.sq[lane];
+                own_cell = g.cx(own.y) * g.G + g.cx(own.x);
+            }
             for (int64_t base = p_at; base < stop; base += 32) {
                 // Lane l draws proposal base + l: two Philox blocks keyed by
                 // (proposal index, replica, 0 / 1), Box-Muller for the centre
@@ -1238,67 +1252,100 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                         rep.cnt[ncell] = (uint8_t)(rep.cnt[ncell] + 1);
                     }
                 };
+                // A lane's own proposal against the current state: the trial
+                // position and trig, the wall energy's change, and the old and
+                // new cells.  It depends on the proposal's square alone, so
+                // without move-set options (whose step scale follows the
+                // acceptance before) all 32 are formed at once, a lane each,
+                // and a proposal only broadcasts its own; `stale` marks a lane
+                // whose square has moved since, which forms its trial again
+                // when its turn comes.  A group of four proposals used to form
+                // its trials with eight lanes each repeating the work.
+                float tx = 0.f, ty = 0.f, tc = 1.f, ts = 0.f, ta = 0.f;
+                long long tw = 0;
+                int tcells = 0;
+                bool stale = false;
+                auto form_trial = [&](float dx, float dy, float da) {
+                    const int i = di & 0xffff;
+                    const float4 P = rep.sq[i];
+                    // keep centres in [0.5, Lr - 0.5] without ever moving a square
+                    // further than the clamped step (it may start outside)
+                    tx = fminf(fmaxf(P.x, Lr - 0.5f), fmaxf(fminf(P.x, 0.5f), P.x + dx));
+                    ty = fminf(fmaxf(P.y, Lr - 0.5f), fmaxf(fminf(P.y, 0.5f), P.y + dy));
+                    ta = rep.ang[i] + da;
+                    ta = ta - kHalfPiF * floorf(ta * (1.0f / kHalfPiF));
+                    if (!(ta >= 0.f && ta < kHalfPiF)) ta = 0.f;
+                    state_trig(ta, &ts, &tc);
+                    tw = qe(wall_e(tx, ty, tc, ts, Lr)) - qe(wall_e(P.x, P.y, P.z, P.w, Lr));
+                    tcells = pack_cells(g.cx(P.x), g.cx(P.y), g.cx(tx), g.cx(ty));
+                };
+                auto form_plain = [&]() {
+                    form_trial(fminf(kMaxStep, fmaxf(-kMaxStep, ddx)), fminf(kMaxStep, fmaxf(-kMaxStep, ddy)), dda);
+                };
+                if (!MOVES) form_plain();
                 // proposal q of this batch, evaluated by the whole warp; returns
                 // the square it moved (-1: none) and its old and new cells
                 auto single = [&](int q) -> Moved {
                     Moved mv{-1, 0};
                     const int dpk = __shfl_sync(0xffffffffu, di, q);
                     const int i = dpk & 0xffff, mode = dpk >> 16;
-                    const float sdx = __shfl_sync(0xffffffffu, ddx, q), sdy = __shfl_sync(0xffffffffu, ddy, q);
-                    const float sda = __shfl_sync(0xffffffffu, dda, q), u_acc = __shfl_sync(0xffffffffu, du, q);
-                    float sc = 1.f;  // step scale (adaptive moves)
+                    const float u_acc = __shfl_sync(0xffffffffu, du, q);
                     const uint64_t pidx = (uint64_t)(base + q);
-                    if (adaptive) {
-                        sc = step_scale(jd, adapt, S.jm.perm[r], cool);
-                        if ((pidx & 15u) == 0) sc *= 3.5f;
-                    }
-                    const float dx = fminf(kMaxStep, fmaxf(-kMaxStep, sdx * sc));
-                    const float dy = fminf(kMaxStep, fmaxf(-kMaxStep, sdy * sc));
-                    const float da = sda * sc;
                     bool acc;
+                    float dx = 0.f, dy = 0.f, da = 0.f;
+                    if (MOVES) {
+                        float sc = 1.f;  // step scale (adaptive moves)
+                        if (adaptive) {
+                            sc = step_scale(jd, adapt, S.jm.perm[r], cool);
+                            if ((pidx & 15u) == 0) sc *= 3.5f;
+                        }
+                        dx = fminf(kMaxStep, fmaxf(-kMaxStep, __shfl_sync(0xffffffffu, ddx, q) * sc));
+                        dy = fminf(kMaxStep, fmaxf(-kMaxStep, __shfl_sync(0xffffffffu, ddy, q) * sc));
+                        da = __shfl_sync(0xffffffffu, dda, q) * sc;
+                    }
                     if (MOVES && mode != 0) {
                         acc = collective_move(rep, g, n, Lr, lane, mode, i, dx, dy, da, u_acc, invT, E, scr_own, npl,
                                               &ovf);
                         ++props;
                         accs += acc;
                     } else {
-                    const float4 P = rep.sq[i];
-                    // keep centres in [0.5, Lr - 0.5] without ever moving a square
-                    // further than the clamped step (it may start outside)
-                    const float nx = fminf(fmaxf(P.x, Lr - 0.5f), fmaxf(fminf(P.x, 0.5f), P.x + dx));
-                    const float ny = fminf(fmaxf(P.y, Lr - 0.5f), fmaxf(fminf(P.y, 0.5f), P.y + dy));
-                    float na = rep.ang[i] + da;
-                    na = na - kHalfPiF * floorf(na * (1.0f / kHalfPiF));
-                    if (!(na >= 0.f && na < kHalfPiF)) na = 0.f;
-                    float ns, nc;
-                    state_trig(na, &ns, &nc);
-                    const int ocx = g.cx(P.x), ocy = g.cx(P.y);
-                    long long dq = 0;
-                    if (lane == 0) dq = qe(wall_e(nx, ny, nc, ns, Lr)) - qe(wall_e(P.x, P.y, P.z, P.w, Lr));
-                    for_block(rep, g, ocx, ocy, lane, [&](int j) {
-                        const long long d = pair_delta(rep.sq[j], nx, ny, nc, ns, P);
-                        dq += j != i ? d : 0;
-                    });
-                    dq = warp_sum_dq(dq);
-                    const float de = (float)dq * (1.0f / kEScale);
-                    acc = dq <= 0 || u_acc < __expf(-de * invT);
-                    const int ncx = g.cx(nx), ncy = g.cx(ny);
-                    const int oc = ocy * g.G + ocx, ncell = ncy * g.G + ncx;
-                    if (acc && oc != ncell && rep.cnt[ncell] >= kCellK) {
-                        acc = false;
-                        ++ovf;
-                    }
-                    ++props;
-                    if (acc) {
-                        ++accs;
-                        E += dq;
-                        if (lane == 0) apply_move(i, nx, ny, nc, ns, na, oc, ncell);
-                        if (MOVES && npl >= 0) {  // out of the pair list's reach?
-                            const float2 o = reinterpret_cast<const float2*>(scr_own + 3 * n)[i];
-                            if (!(fabsf(nx - o.x) <= kListStep && fabsf(ny - o.y) <= kListStep)) npl = -1;
+                        if (MOVES) {
+                            if (lane == q) form_trial(dx, dy, da);
+                        } else if (__shfl_sync(0xffffffffu, (int)stale, q)) {
+                            if (stale) form_plain();
+                            stale = false;
                         }
-                        mv = Moved{i, pack_cells(ocx, ocy, ncx, ncy)};
-                    }
+                        const float nx = __shfl_sync(0xffffffffu, tx, q), ny = __shfl_sync(0xffffffffu, ty, q);
+                        const float nc = __shfl_sync(0xffffffffu, tc, q), ns = __shfl_sync(0xffffffffu, ts, q);
+                        const int cells = __shfl_sync(0xffffffffu, tcells, q);
+                        const int ocx = cells & 0xff, ocy = (cells >> 8) & 0xff, ncx = (cells >> 16) & 0xff,
+                                  ncy = (int)((unsigned)cells >> 24);
+                        const float4 P = rep.sq[i];
+                        long long dq = lane == q ? tw : 0;
+                        for_block(rep, g, ocx, ocy, lane, [&](int j) {
+                            const long long d = pair_delta(rep.sq[j], nx, ny, nc, ns, P);
+                            dq += j != i ? d : 0;
+                        });
+                        dq = warp_sum_dq(dq);
+                        const float de = (float)dq * (1.0f / kEScale);
+                        acc = dq <= 0 || u_acc < __expf(-de * invT);
+                        const int oc = ocy * g.G + ocx, ncell = ncy * g.G + ncx;
+                        if (acc && oc != ncell && rep.cnt[ncell] >= kCellK) {
+                            acc = false;
+                            ++ovf;
+                        }
+                        ++props;
+                        if (acc) {
+                            ++accs;
+                            E += dq;
+                            if (lane == q) apply_move(i, tx, ty, tc, ts, ta, oc, ncell);
+                            stale |= (di & 0xffff) == i;
+                            if (MOVES && npl >= 0) {  // out of the pair list's reach?
+                                const float2 o = reinterpret_cast<const float2*>(scr_own + 3 * n)[i];
+                                if (!(fabsf(nx - o.x) <= kListStep && fabsf(ny - o.y) <= kListStep)) npl = -1;
+                            }
+                            mv = Moved{i, cells};
+                        }
                     }
                     if (adaptive) {  // every 16 proposals: steer toward 25% acceptance
                         win += acc;
@@ -1311,37 +1358,37 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     return mv;
                 };
                 // Proposals q .. q + M - 1 evaluated at once, one per group of
-                // 32 / M lanes, all against the current state, then decided in
-                // order.  A proposal's result stands unless an earlier move of
-                // the group that was accepted touched what it read: the same
-                // square, or an old or new cell of that move inside its 3x3
-                // block (cells are wider than a step, so a move changes a
-                // square's cell by at most one; every other read -- counts and
-                // slots of the block, squares in it, the count of its target
-                // cell -- lies in that block).  Then the whole warp evaluates it
-                // again on the current state.  Energies are exact and
-                // order-free, so the trajectory is the one-at-a-time trajectory,
-                // bit for bit.
+                // 32 / M lanes, all against the current state.  A proposal's
+                // result stands unless an earlier move of the group that was
+                // accepted touched what it read: the same square, or an old or
+                // new cell of that move inside its 3x3 block (cells are wider
+                // than a step, so a move changes a square's cell by at most one;
+                // every other read -- counts and slots of the block, squares in
+                // it, the count of its target cell -- lies in that block).
+                // When no accepted move touches a later proposal, all decisions
+                // stand, the accepted moves lie in distinct cells, and each
+                // proposal's own lane applies its move at the same time.
+                // Otherwise they are decided in order, and a proposal that was
+                // touched is evaluated again by the whole warp on the current
+                // state.  Energies are exact and order-free, so the trajectory
+                // is the one-at-a-time trajectory, bit for bit.
                 auto group = [&](int q, auto mtag) {
                     constexpr int M = decltype(mtag)::value, W = 32 / M;
                     const int grp = lane / W, gl = lane % W;
                     const int qs = q + grp;
-                    const int i = __shfl_sync(0xffffffffu, di, qs) & 0xffff;
-                    const float sdx = __shfl_sync(0xffffffffu, ddx, qs), sdy = __shfl_sync(0xffffffffu, ddy, qs);
-                    const float sda = __shfl_sync(0xffffffffu, dda, qs), u_acc = __shfl_sync(0xffffffffu, du, qs);
-                    const float dx = fminf(kMaxStep, fmaxf(-kMaxStep, sdx));
-                    const float dy = fminf(kMaxStep, fmaxf(-kMaxStep, sdy));
+                    if (__any_sync(0xffffffffu, stale && lane >= q && lane < q + M)) {
+                        if (stale) form_plain();
+                        stale = false;
+                    }
+                    const int i = __shfl_sync(0xffffffffu, di, qs);
+                    const float nx = __shfl_sync(0xffffffffu, tx, qs), ny = __shfl_sync(0xffffffffu, ty, qs);
+                    const float nc = __shfl_sync(0xffffffffu, tc, qs), ns = __shfl_sync(0xffffffffu, ts, qs);
+                    const int cells = __shfl_sync(0xffffffffu, tcells, qs);
+                    const float u_acc = __shfl_sync(0xffffffffu, du, qs);
+                    const int ocx = cells & 0xff, ocy = (cells >> 8) & 0xff, ncx = (cells >> 16) & 0xff,
+                              ncy = (int)((unsigned)cells >> 24);
                     const float4 P = rep.sq[i];
-                    const float nx = fminf(fmaxf(P.x, Lr - 0.5f), fmaxf(fminf(P.x, 0.5f), P.x + dx));
-                    const float ny = fminf(fmaxf(P.y, Lr - 0.5f), fmaxf(fminf(P.y, 0.5f), P.y + dy));
-                    float na = rep.ang[i] + sda;
-                    na = na - kHalfPiF * floorf(na * (1.0f / kHalfPiF));
-                    if (!(na >= 0.f && na < kHalfPiF)) na = 0.f;
-                    float ns, nc;
-                    state_trig(na, &ns, &nc);
-                    const int ocx = g.cx(P.x), ocy = g.cx(P.y);
                     long long dq = 0;
-                    if (gl == 0) dq = qe(wall_e(nx, ny, nc, ns, Lr)) - qe(wall_e(P.x, P.y, P.z, P.w, Lr));
                     for_block<W>(rep, g, ocx, ocy, gl, [&](int j) {
                         const long long d = pair_delta(rep.sq[j], nx, ny, nc, ns, P);
                         dq += j != i ? d : 0;
@@ -1355,9 +1402,11 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                         hi += __shfl_xor_sync(0xffffffffu, hi, off);
                         lo += __shfl_xor_sync(0xffffffffu, lo, off);
                     }
-                    const long long mine = (long long)hi * 1048576ll + (long long)lo;
+                    const unsigned wlo = __shfl_sync(0xffffffffu, (unsigned)(unsigned long long)tw, qs);
+                    const int whi = __shfl_sync(0xffffffffu, (int)(tw >> 32), qs);
+                    const long long mine = (long long)hi * 1048576ll + (long long)lo +
+                                           (long long)(((unsigned long long)(unsigned)whi << 32) | wlo);
                     const float de = (float)mine * (1.0f / kEScale);
-                    const int ncx = g.cx(nx), ncy = g.cx(ny);
                     const int oc = ocy * g.G + ocx, ncell = ncy * g.G + ncx;
                     int acc = mine <= 0 || u_acc < __expf(-de * invT);
                     int ov = 0;
@@ -1365,7 +1414,31 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                         acc = 0;
                         ov = 1;
                     }
-                    const int cells = pack_cells(ocx, ocy, ncx, ncy);
+                    // does an accepted move of an earlier proposal touch this one?
+                    const int mv_i = acc ? i : -1;
+                    bool hit = false;
+#pragma unroll
+                    for (int d = 1; d < M; ++d) {
+                        const int oi = __shfl_up_sync(0xffffffffu, mv_i, d * W);
+                        const int ocl = __shfl_up_sync(0xffffffffu, cells, d * W);
+                        hit |= grp >= d && touches(oi, ocl, i, cells);
+                    }
+                    if (!__any_sync(0xffffffffu, hit)) {
+                        const unsigned am = __ballot_sync(0xffffffffu, acc && gl == 0);
+                        ovf += __popc(__ballot_sync(0xffffffffu, ov && gl == 0));
+                        props += M;
+                        if (am) {
+                            accs += __popc(am);
+                            E += warp_sum_ll(acc && gl == 0 ? mine : 0);
+                            if (lane >= q && lane < q + M && (am >> ((lane - q) * W) & 1u))
+                                apply_move(di, tx, ty, tc, ts, ta, ((tcells >> 8) & 0xff) * g.G + (tcells & 0xff),
+                                           (int)((unsigned)tcells >> 24) * g.G + ((tcells >> 16) & 0xff));
+#pragma unroll
+                            for (int k = 0; k < M; ++k) stale |= (am >> (k * W) & 1u) && di == __shfl_sync(0xffffffffu, i, k * W);
+                        }
+                        __syncwarp();
+                        return;
+                    }
                     int mi[M], mc[M];  // the group's moves so far: square (-1: none), cells
 #pragma unroll
                     for (int k = 0; k < M; ++k) {
@@ -1385,20 +1458,69 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                             ++props;
                             accs += ak;
                             ovf += ovk;
-                            if (ak) E += (long long)(((unsigned long long)(unsigned)dhi << 32) | dlo);
-                            if (ak && lane == src) apply_move(i, nx, ny, nc, ns, na, oc, ncell);
+                            if (ak) {
+                                E += (long long)(((unsigned long long)(unsigned)dhi << 32) | dlo);
+                                if (lane == q + k)
+                                    apply_move(di, tx, ty, tc, ts, ta, ((tcells >> 8) & 0xff) * g.G + (tcells & 0xff),
+                                               (int)((unsigned)tcells >> 24) * g.G + ((tcells >> 16) & 0xff));
+                                stale |= di == ik;
+                            }
                             __syncwarp();
                             mi[k] = ak ? ik : -1;
                             mc[k] = ck;
                         }
                     }
                 };
+                // A replica of up to 32 squares without move-set options holds
+                // square `lane` in registers and tests a proposal against every
+                // other square, a lane each, cell lists aside: pairs outside the
+                // cut-off add zero, so the change is the same, and the chain of
+                // dependent loads (counts, slot, square) is gone.  A cell's
+                // count, for the capacity rule, is a ballot.
+                auto tiny = [&](int q) {
+                    const int i = __shfl_sync(0xffffffffu, di, q);
+                    if (__shfl_sync(0xffffffffu, (int)stale, q)) {
+                        if (stale) form_plain();
+                        stale = false;
+                    }
+                    const float nx = __shfl_sync(0xffffffffu, tx, q), ny = __shfl_sync(0xffffffffu, ty, q);
+                    const float nc = __shfl_sync(0xffffffffu, tc, q), ns = __shfl_sync(0xffffffffu, ts, q);
+                    const float u_acc = __shfl_sync(0xffffffffu, du, q);
+                    const float4 P = rep.sq[i];
+                    const long long d = pair_delta(own, nx, ny, nc, ns, P);
+                    const long long dq = warp_sum_dq((lane != i && lane < n ? d : 0) + (lane == q ? tw : 0));
+                    ++props;
+                    bool acc = dq <= 0 || u_acc < __expf(-((float)dq * (1.0f / kEScale)) * invT);
+                    if (!acc) return;
+                    if (n > kCellK) {
+                        const int cells = __shfl_sync(0xffffffffu, tcells, q);
+                        const int ncell = (int)((unsigned)cells >> 24) * g.G + ((cells >> 16) & 0xff);
+                        const int there = __popc(__ballot_sync(0xffffffffu, own_cell == ncell));
+                        if (ncell != ((cells >> 8) & 0xff) * g.G + (cells & 0xff) && there >= kCellK) {
+                            ++ovf;
+                            return;
+                        }
+                        if (lane == i) own_cell = ncell;
+                    }
+                    ++accs;
+                    E += dq;
+                    if (lane == i) own = make_float4(nx, ny, nc, ns);
+                    if (lane == q) {
+                        rep.sq[i] = make_float4(nx, ny, nc, ns);
+                        rep.ang[i] = ta;
+                    }
+                    stale |= di == i;
+                    __syncwarp();
+                };
                 // groups need room: on small grids most proposals would be
                 // evaluated twice; the move-set instance keeps one at a time
                 // (its step scale follows the acceptance of the previous move)
                 const bool fours = !MOVES && g.G >= 8, twos = !MOVES && g.G >= 4;
                 for (int q = 0; q < kn;) {
-                    if (fours && q + 3 < kn) {
+                    if (small) {
+                        tiny(q);
+                        ++q;
+                    } else if (fours && q + 3 < kn) {
                         group(q, IntTag<4>{});
                         q += 4;
                     } else if (twos && q + 1 < kn) {
@@ -1410,6 +1532,7 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     }
                 }
             }
+            if (small) build_cells(rep, n, g, lane);  // every cell within its capacity
         }
         p_at = stop;
         // ---- checkpoint: best-state search, shrink, replica exchange.  Only
