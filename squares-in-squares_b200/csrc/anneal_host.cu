@@ -636,6 +636,12 @@ static int anneal_run(sqs_ctx* ctx, const sqs_job* jobs, int njobs, int slice_sw
             rb = std::max(rb, plan[(size_t)j].rb);
             nmax = std::max(nmax, jobs[j].n);
         }
+        // clusters start in list order as others end: the jobs with the longest
+        // budget per replica first, so that no long one starts last (256 jobs of
+        // n 20..400 and 32 replicas: 50.9 to 47.1 ms)
+        std::stable_sort(kv.second.begin(), kv.second.end(), [&](int32_t a, int32_t b) {
+            return jd[(size_t)a].props_total > jd[(size_t)b].props_total;
+        });
         spans.push_back({lists.size(), kv.second.size()});
         lists.insert(lists.end(), kv.second.begin(), kv.second.end());
         smems.push_back(anneal_smem(std::get<0>(kv.first), std::get<1>(kv.first), rb, nmax, std::get<2>(kv.first) != 0,
