@@ -8,10 +8,18 @@
 // a factor (1 - delta) into a side L (1 - delta), descend the same energy
 // with a backtracking line search until it vanishes, and keep the result if
 // its dilation-certified side (device_certified_side, seeded.cu:175-226) is
-// smaller; delta shrinks after every failure.  Pairs are evaluated all
-// against all (n <= 1000, one CTA): every thread owns squares and loops over
-// all partners, so gradients need no atomics and reductions have a fixed
-// order (the result is deterministic).
+// smaller; delta shrinks after every failure.  Every square's pairs are taken
+// in ascending order of the partner, over a neighbour list found through a
+// cell grid, so gradients need no atomics and all sums have a fixed order:
+// the result is deterministic and equals the all-pairs loop's bit for bit.
+//
+// Bound by the FP64 pipe for large n (one CTA on one SM) and by the chain of
+// dependent FP64 operations for small n.  A line-search trial brings the
+// gradient of its state along, so an accepted step evaluates its state once
+// instead of twice; lists and certified sides go through cells instead of all
+// pairs; a trial takes two block barriers instead of six, and for small n
+// several lanes share a square's partners.  64 packings of n 5..1000, half of
+// them overlapped, 200 steps: 7.8 -> 3.2 ms a call (one B200).
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -23,20 +31,34 @@
 namespace sqs {
 namespace ann {
 
-constexpr int kPT = 256;  // threads per polish CTA
+constexpr int kPT = 512;  // threads per polish CTA
+constexpr int kPS = 256;  // an energy's partial sums (see energy())
 
 // Neighbour lists of the polish: every partner within sqrt(2.000001) + 0.25
 // of a square when the list was built (at most kNbK, ascending), valid while
-// no square has moved more than 0.125 since -- then every pair inside the
+// no square has moved more than kNbMove since -- then every pair inside the
 // pair cut-off is listed.  Energies over the list sum the same nonzero terms
 // in the same order as the all-pairs loop, so they are bit-identical to it.
 constexpr int kNbK = 24;
 constexpr double kNbR2 = 2.7697;       // (sqrt(2.000001) + 0.25)^2 = 2.76961, rounded up
-constexpr double kNbMove2 = 0.015625;  // 0.125^2
+constexpr double kNbMove = 0.1249;     // below 0.125 by more than the bounds' rounding
+// Cells of the grid that finds neighbours: wider than the list's radius
+// (1.66424) and the certified side's (sqrt 2.05), at most kCG a side.
+constexpr double kCellW = 1.6645, kCellMinW = 1.6643;
+constexpr int kCG = 32;
 
-// q0, q, g, sv (double3), cs (double2), the list's reference centres
-// (double2), partner indices (uint16) and counts (uint8)
-size_t polish_smem_bytes(int n) { return (size_t)n * (4 * 24 + 16 + 16 + 2 * kNbK + 1) + 64; }
+constexpr int kTerms = 4;  // energy terms kept a square (see energy())
+// An array in the CTA's dynamic shared memory by its byte offset: buffers that
+// are passed around and swapped stay visibly shared, so every access is a
+// shared-memory instruction (as pointers they became generic loads, a third
+// of the kernel's stalls).
+extern __shared__ __align__(16) unsigned char polish_dyn[];
+template <class T>
+struct Sh {
+    int off;
+    __device__ __forceinline__ T& operator[](int i) const { return reinterpret_cast<T*>(polish_dyn + off)[i]; }
+    __device__ __forceinline__ Sh operator+(int i) const { return Sh{off + i * (int)sizeof(T)}; }
+};
 
 __device__ __forceinline__ double sgn_s(double x) { return fabs(x) > 1e-6 ? (x >= 0.0 ? 1.0 : -1.0) : 0.0; }
 
@@ -86,17 +108,7 @@ __device__ __forceinline__ double wall_smooth(double x, double y, double c, doub
     return e;
 }
 
-__device__ double block_sum(double v, double* red) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    for (int w = 0; w < kPT / 32; ++w) t += red[w];
-    return t;
-}
-
-__device__ double block_max(double v, double* red) {
+__device__ double block_max(double v, Sh<double> red) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
@@ -107,87 +119,269 @@ __device__ double block_max(double v, double* red) {
 }
 
 struct NbrList {
-    double2* ref;   // centres at the build
-    uint16_t* idx;  // partners of square i: idx[i * kNbK + k], k < cnt[i]
-    uint8_t* cnt;
+    Sh<uint16_t> idx;  // partners of square i: idx[i * kNbK + k], k < cnt[i]
+    Sh<uint8_t> cnt;
 };
 
-// Energy (and gradient into g when g != nullptr) of the state q at side L,
-// over the neighbour list when nb != nullptr, else over all pairs.
-__device__ double energy(int n, const double3* q, const double2* cs, double L, double3* g, double* red,
-                         const NbrList* nb = nullptr) {
-    double e = 0.0;
-    for (int i = threadIdx.x; i < n; i += kPT) {
-        const double3 p = q[i];
-        const double2 pc = cs[i];
-        double gx = 0, gy = 0, ga = 0;
-        e += wall_smooth(p.x, p.y, pc.x, pc.y, L, gx, gy, ga);
-        const int m = nb ? nb->cnt[i] : n;
-        for (int k = 0; k < m; ++k) {
-            const int j = nb ? (int)nb->idx[i * kNbK + k] : k;
-            if (j == i) continue;
-            const double3 o = q[j];
-            const double2 oc = cs[j];
-            double hx = 0, hy = 0, ha = 0;
-            const double pe = pair_smooth(p.x, p.y, pc.x, pc.y, o.x, o.y, oc.x, oc.y, hx, hy, ha);
-            if (j > i) e += pe;
-            gx += hx;
-            gy += hy;
-            ga += ha;
+// Squares by cell: order[start[c] .. start[c + 1]) lie in cell c = cy * G + cx
+// of a G x G grid over [x0, x0 + side] x [y0, y0 + side].  A square outside
+// counts into the nearest edge cell, which keeps any two squares closer than
+// a cell's width in the same or adjacent cells.
+struct Cells {
+    Sh<uint16_t> order;
+    Sh<int> start;  // kCG * kCG + 1
+    double x0, y0, inv;
+    int G;
+    __device__ __forceinline__ int at(double x) const { return min(G - 1, max(0, __double2int_rd(x * inv))); }
+    __device__ __forceinline__ int cx(const double3& p) const { return at(p.x - x0); }
+    __device__ __forceinline__ int cy(const double3& p) const { return at(p.y - y0); }
+};
+
+// Sort the squares of q into cells.  Starts and ends with a barrier.
+__device__ void build_cells(int n, Cells& c, Sh<double3> q, double x0, double y0, double side) {
+    c.x0 = x0;
+    c.y0 = y0;
+    c.G = min(kCG, max(1, __double2int_rd(side / kCellW)));
+    c.inv = (double)c.G / side;
+    if (!(c.inv > 0.0 && c.inv * kCellMinW <= 1.0)) c.inv = 0.0, c.G = 1;  // a side below one cell, or not finite
+    const int ncell = c.G * c.G, t = threadIdx.x;
+    __syncthreads();
+    for (int k = t; k <= ncell; k += kPT) c.start[k] = 0;
+    __syncthreads();
+    int rank[kMaxN / kPT + 1], cell[kMaxN / kPT + 1];
+#pragma unroll
+    for (int m = 0; m < kMaxN / kPT + 1; ++m) {
+        const int i = t + m * kPT;
+        if (i < n) {
+            cell[m] = c.cy(q[i]) * c.G + c.cx(q[i]);
+            rank[m] = atomicAdd(&c.start[cell[m]], 1);
         }
-        if (g) g[i] = make_double3(gx, gy, ga);
     }
-    return block_sum(e, red);
+    __syncthreads();
+    if (t < 32) {  // exclusive scan, a run of cells a lane
+        const int per = (ncell + 31) / 32, lo = t * per, hi = min(lo + per, ncell);
+        int sum = 0;
+        for (int k = lo; k < hi; ++k) sum += c.start[k];
+        int incl = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (t >= o) incl += v;
+        }
+        int run = incl - sum;
+        for (int k = lo; k < hi; ++k) {
+            const int v = c.start[k];
+            c.start[k] = run;
+            run += v;
+        }
+        if (t == 31) c.start[ncell] = incl;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < kMaxN / kPT + 1; ++m) {
+        const int i = t + m * kPT;
+        if (i < n) c.order[c.start[cell[m]] + rank[m]] = (uint16_t)i;
+    }
+    __syncthreads();
 }
 
-// Build the list for state q; false when a square has more than kNbK
-// partners (the callers then use all pairs).
-__device__ bool build_nbr(int n, const NbrList& nb, const double3* q, double* red) {
-    double over = 0.0;
+// Build the list for state q from its cells; false when a square has more
+// than kNbK partners (the callers then use all pairs).
+__device__ bool build_nbr(int n, const NbrList& nb, const Cells& c, Sh<double3> q) {
+    bool over = false;
     for (int i = threadIdx.x; i < n; i += kPT) {
         const double3 p = q[i];
-        int c = 0;
-        for (int j = 0; j < n; ++j) {
-            if (j == i) continue;
-            const double dx = q[j].x - p.x, dy = q[j].y - p.y;
-            if (dx * dx + dy * dy < kNbR2) {
-                if (c < kNbK) nb.idx[i * kNbK + c] = (uint16_t)j;
-                ++c;
+        const Sh<uint16_t> L = nb.idx + i * kNbK;
+        const int cx = c.cx(p), cy = c.cy(p);
+        const int xa = max(cx - 1, 0), xb = min(cx + 1, c.G - 1);
+        int m = 0;
+        for (int y = max(cy - 1, 0); y <= min(cy + 1, c.G - 1); ++y) {
+            for (int k = c.start[y * c.G + xa]; k < c.start[y * c.G + xb + 1]; ++k) {
+                const int j = c.order[k];
+                if (j == i) continue;
+                const double dx = q[j].x - p.x, dy = q[j].y - p.y;
+                if (dx * dx + dy * dy < kNbR2) {
+                    if (m < kNbK) {  // insert in ascending order
+                        int w = m;
+                        for (; w > 0 && L[w - 1] > j; --w) L[w] = L[w - 1];
+                        L[w] = (uint16_t)j;
+                    }
+                    ++m;
+                }
             }
         }
-        nb.cnt[i] = (uint8_t)min(c, kNbK);
-        nb.ref[i] = make_double2(p.x, p.y);
-        if (c > kNbK) over = 1.0;
+        nb.cnt[i] = (uint8_t)min(m, kNbK);
+        over |= m > kNbK;
     }
-    return block_max(over, red) == 0.0;
+    return !__syncthreads_or(over);
 }
 
-// Largest squared centre displacement of q since the list was built.
-__device__ double moved2(int n, const NbrList& nb, const double3* q, double* red) {
-    double m = 0.0;
-    for (int i = threadIdx.x; i < n; i += kPT) {
-        const double dx = q[i].x - nb.ref[i].x, dy = q[i].y - nb.ref[i].y;
-        m = fmax(m, dx * dx + dy * dy);
+// Energy of the state q at side L, its gradient into g, and the largest
+// squared centre gradient into gmax2: over the neighbour list when nb != nullptr, else
+// over all pairs.  The energy is kPS partial sums, added by butterflies and
+// then warp by warp: partial s takes squares s, s + kPS, ..., of each the wall
+// first, then the partners above it in ascending order -- one order whatever
+// the number of threads.  For n <= kPS over a list, 2, 4 or 8 lanes evaluate a
+// square's partners at once and add the nonzero terms in that order.  For
+// larger n a thread takes whole squares and leaves their nonzero energy terms
+// (at most kTerms; a square with more is summed again) to the threads that
+// add up the partials.  The barrier that publishes the state before a call
+// also ends the reads of the call before.
+struct Red {
+    Sh<double> e;       // [kPS / 32]
+    Sh<double> m;       // [kPT / 32]
+    Sh<double> es;      // [kPS]: squares' sums of the lane-parallel form
+    Sh<double> terms;   // [n][kTerms]
+    Sh<uint8_t> nterm;  // [n]: terms there, kTerms + 1: more than fit
+};
+
+// Energy terms of square i added to e in their order (no gradient).
+__device__ __noinline__ double add_square(double e, int i, int n, Sh<double3> q, Sh<double2> cs, double L,
+                                          const NbrList& nb, bool listed) {
+    const double3 p = q[i];
+    const double2 pc = cs[i];
+    double gx = 0, gy = 0, ga = 0;
+    e += wall_smooth(p.x, p.y, pc.x, pc.y, L, gx, gy, ga);
+    const int m = listed ? nb.cnt[i] : n;
+    for (int k = 0; k < m; ++k) {
+        const int j = listed ? (int)nb.idx[i * kNbK + k] : k;
+        if (j <= i) continue;
+        const double3 o = q[j];
+        const double2 oc = cs[j];
+        e += pair_smooth(p.x, p.y, pc.x, pc.y, o.x, o.y, oc.x, oc.y, gx, gy, ga);
     }
-    return block_max(m, red);
+    return e;
+}
+
+__device__ double energy(int n, Sh<double3> q, Sh<double2> cs, double L, Sh<double3> g, double& gmax2, const Red& red,
+                         const NbrList& nb, bool listed) {
+    double e = 0.0, gm = 0.0;
+    const int t = threadIdx.x;
+    const int w = !listed || 2 * n > min(kPT, 2 * kPS) ? 1 : (4 * n > kPT ? 2 : (8 * n > kPT ? 4 : 8));
+    if (w == 1) {
+        for (int i = t; i < n; i += kPT) {
+            const double3 p = q[i];
+            const double2 pc = cs[i];
+            double gx = 0, gy = 0, ga = 0;
+            const Sh<double> T = red.terms + i * kTerms;
+            int nt = 0;
+            auto term = [&](double v) {
+                if (v != 0.0) {
+                    if (nt < kTerms) T[nt] = v;
+                    nt = min(nt + 1, kTerms + 1);
+                }
+            };
+            term(wall_smooth(p.x, p.y, pc.x, pc.y, L, gx, gy, ga));
+            const int m = listed ? nb.cnt[i] : n;
+            for (int k = 0; k < m; ++k) {
+                const int j = listed ? (int)nb.idx[i * kNbK + k] : k;
+                if (j == i) continue;
+                const double3 o = q[j];
+                const double2 oc = cs[j];
+                double hx = 0, hy = 0, ha = 0;
+                const double pe = pair_smooth(p.x, p.y, pc.x, pc.y, o.x, o.y, oc.x, oc.y, hx, hy, ha);
+                if (j > i) term(pe);
+                gx += hx;
+                gy += hy;
+                ga += ha;
+            }
+            red.nterm[i] = (uint8_t)nt;
+            g[i] = make_double3(gx, gy, ga);
+            gm = fmax(gm, gx * gx + gy * gy);
+        }
+        __syncthreads();
+        for (int i = t; t < kPS && i < n; i += kPS) {
+            const int nt = red.nterm[i];
+            if (nt > kTerms) {
+                e = add_square(e, i, n, q, cs, L, nb, listed);
+                continue;
+            }
+            for (int k = 0; k < nt; ++k) e += red.terms[i * kTerms + k];
+        }
+    } else {
+        const int i = t / w, l = t % w, lane = t & 31, base = lane - l;
+        double gx = 0, gy = 0, ga = 0, ei = 0;
+        double3 p = make_double3(0, 0, 0);
+        double2 pc = make_double2(1, 0);
+        int m = 0;
+        if (i < n) {
+            p = q[i];
+            pc = cs[i];
+            ei += wall_smooth(p.x, p.y, pc.x, pc.y, L, gx, gy, ga);
+            m = nb.cnt[i];
+        }
+        const int most = __reduce_max_sync(0xffffffffu, m);
+        for (int k0 = 0; k0 < most; k0 += w) {
+            double hx = 0, hy = 0, ha = 0, pe = 0;
+            int j = -1;
+            if (k0 + l < m) {
+                j = nb.idx[i * kNbK + k0 + l];
+                const double3 o = q[j];
+                const double2 oc = cs[j];
+                pe = pair_smooth(p.x, p.y, pc.x, pc.y, o.x, o.y, oc.x, oc.y, hx, hy, ha);
+            }
+            // the lanes with a nonzero term, in order
+            unsigned hit = __ballot_sync(0xffffffffu, pe > 0.0) >> base & ((1u << w) - 1u);
+            const int rounds = __reduce_max_sync(0xffffffffu, __popc(hit));
+            for (int r = 0; r < rounds; ++r) {
+                const int src = base + (hit ? __ffs(hit) - 1 : 0);
+                const double ax = __shfl_sync(0xffffffffu, hx, src), ay = __shfl_sync(0xffffffffu, hy, src);
+                const double aa = __shfl_sync(0xffffffffu, ha, src), ae = __shfl_sync(0xffffffffu, pe, src);
+                const int aj = __shfl_sync(0xffffffffu, j, src);
+                if (hit) {
+                    gx += ax;
+                    gy += ay;
+                    ga += aa;
+                    if (aj > i) ei += ae;
+                    hit &= hit - 1;
+                }
+            }
+        }
+        if (i < n && l == 0) {
+            g[i] = make_double3(gx, gy, ga);
+            red.es[i] = ei;
+            gm = gx * gx + gy * gy;
+        }
+        __syncthreads();
+        e = t < n ? red.es[t] : 0.0;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        e += __shfl_xor_sync(0xffffffffu, e, o);
+        gm = fmax(gm, __shfl_xor_sync(0xffffffffu, gm, o));
+    }
+    if ((t & 31) == 0) {
+        if (t < kPS) red.e[t >> 5] = e;
+        red.m[t >> 5] = gm;
+    }
+    __syncthreads();
+    double s = 0.0, mx = 0.0;
+    for (int k = 0; k < kPS / 32; ++k) s += red.e[k];
+    for (int k = 0; k < kPT / 32; ++k) mx = fmax(mx, red.m[k]);
+    gmax2 = mx;
+    return s;
 }
 
 // Certified side of q (dilation lambda, bounding box of the dilated state).
-__device__ double cert_side_all(int n, const double3* q, const double2* cs, double* red, double& lam_out,
-                                double& x0, double& y0) {
+__device__ double cert_side_all(int n, Sh<double3> q, Sh<double2> cs, const Cells& c, Sh<double> red,
+                                double& lam_out, double& x0, double& y0) {
     double lam = 1.0;
     for (int i = threadIdx.x; i < n; i += kPT) {
         const double3 p = q[i];
         const double ci = cs[i].x, si = cs[i].y;
-        for (int j = i + 1; j < n; ++j) {
-            const double dx = p.x - q[j].x, dy = p.y - q[j].y;
-            if (dx * dx + dy * dy >= 2.05) continue;
-            const double cj = cs[j].x, sj = cs[j].y;
-            const double c12 = fabs(ci * cj + si * sj), s12 = fabs(-si * cj + ci * sj);
-            const double r = 0.5 + 0.5 * (c12 + s12);
-            const double v = fmax(fmax(fabs(dx * ci + dy * si), fabs(-dx * si + dy * ci)),
-                                  fmax(fabs(dx * cj + dy * sj), fabs(-dx * sj + dy * cj)));
-            lam = fmax(lam, v > 1e-12 ? (r + 2.6e-8) / v : 1e9);
+        const int cx = c.cx(p), cy = c.cy(p);
+        const int xa = max(cx - 1, 0), xb = min(cx + 1, c.G - 1);
+        for (int yy = max(cy - 1, 0); yy <= min(cy + 1, c.G - 1); ++yy) {
+            for (int k = c.start[yy * c.G + xa]; k < c.start[yy * c.G + xb + 1]; ++k) {
+                const int j = c.order[k];
+                if (j <= i) continue;
+                const double dx = p.x - q[j].x, dy = p.y - q[j].y;
+                if (dx * dx + dy * dy >= 2.05) continue;
+                const double cj = cs[j].x, sj = cs[j].y;
+                const double c12 = fabs(ci * cj + si * sj), s12 = fabs(-si * cj + ci * sj);
+                const double r = 0.5 + 0.5 * (c12 + s12);
+                const double v = fmax(fmax(fabs(dx * ci + dy * si), fabs(-dx * si + dy * ci)),
+                                      fmax(fabs(dx * cj + dy * sj), fabs(-dx * sj + dy * cj)));
+                lam = fmax(lam, v > 1e-12 ? (r + 2.6e-8) / v : 1e9);
+            }
         }
     }
     lam = block_max(lam, red);
@@ -210,11 +404,11 @@ __device__ double cert_side_all(int n, const double3* q, const double2* cs, doub
 }
 
 __device__ __forceinline__ double wrap_q(double a) {
-    a = fmod(a, 1.57079632679489661923);
+    if (!(fabs(a) < 1.57079632679489661923)) a = fmod(a, 1.57079632679489661923);  // fmod(a, b) is a below b
     return a < 0.0 ? a + 1.57079632679489661923 : a;
 }
 
-__device__ void trig_of(int n, const double3* q, double2* cs) {
+__device__ void trig_of(int n, Sh<double3> q, Sh<double2> cs) {
     for (int i = threadIdx.x; i < n; i += kPT) {
         double s, c;
         sincos(q[i].z, &s, &c);
@@ -225,33 +419,63 @@ __device__ void trig_of(int n, const double3* q, double2* cs) {
 
 // Shared-memory views of one polish CTA.
 struct PolishBufs {
-    double3* q0;  // accepted state of the descent
-    double3* q;   // trial state
-    double3* g;   // gradient at q0
-    double3* sv;  // best so far (translated, dilated)
-    double2* cs;  // cos/sin of the state being evaluated
+    Sh<double3> q0;  // accepted state of the descent
+    Sh<double3> q;   // trial state
+    Sh<double3> g;   // gradient at q0
+    Sh<double3> tg;  // gradient at q
+    Sh<double3> sv;  // best so far (translated, dilated)
+    Sh<double2> cs;  // cos/sin of the state being evaluated
+    Sh<double> max;  // [kPT / 32] partials of block_max
     NbrList nb;   // neighbour list of the descent
+    Cells cells;
+    Red red;
 };
 
-__device__ __forceinline__ PolishBufs polish_bufs(unsigned char* dyn, int n) {
+// The evaluation's share of the layout (from `off` on), then the polish's.
+constexpr int kRedDoubles = kPS / 32 + 2 * (kPT / 32) + kPS;
+__device__ __forceinline__ int eval_bufs(int off, int n, Red& red, NbrList& nb, Cells& cells) {
+    red.e = Sh<double>{off};
+    red.m = red.e + kPS / 32;
+    red.es = red.m + 2 * (kPT / 32);  // (block_max's partials lie between)
+    red.terms = red.es + kPS;
+    cells.start = Sh<int>{red.terms.off + 8 * kTerms * n};
+    nb.idx = Sh<uint16_t>{cells.start.off + 4 * (kCG * kCG + 1)};
+    cells.order = nb.idx + n * kNbK;
+    nb.cnt = Sh<uint8_t>{cells.order.off + 2 * n};
+    red.nterm = nb.cnt + n;
+    return red.nterm.off + n;
+}
+constexpr size_t eval_bytes(size_t n) {
+    return 8 * kRedDoubles + n * (8 * kTerms + 2 * kNbK + 2 + 2) + (kCG * kCG + 1) * 4;
+}
+
+__device__ __forceinline__ PolishBufs polish_bufs(int n) {
     PolishBufs b;
-    b.q0 = reinterpret_cast<double3*>(dyn);
+    b.cs = Sh<double2>{0};
+    b.q0 = Sh<double3>{16 * n};
     b.q = b.q0 + n;
     b.g = b.q + n;
-    b.sv = b.g + n;
-    b.cs = reinterpret_cast<double2*>(b.sv + n);
-    b.nb.ref = b.cs + n;
-    b.nb.idx = reinterpret_cast<uint16_t*>(b.nb.ref + n);
-    b.nb.cnt = reinterpret_cast<uint8_t*>(b.nb.idx + (size_t)n * kNbK);
+    b.tg = b.g + n;
+    b.sv = b.tg + n;
+    eval_bufs(b.sv.off + 24 * n, n, b.red, b.nb, b.cells);
+    b.max = b.red.m + kPT / 32;
     return b;
 }
 
-// Descend the energy of state q0 at side Lt until it vanishes (at most
-// *budget gradient steps, each with up to 8 backtracking trials).
-__device__ void descend(int n, const PolishBufs& B, double Lt, int* budget, double* red) {
+// q0, q, g, tg, sv (double3), cs (double2), and the evaluation's
+size_t polish_smem_bytes(int n) { return (size_t)n * (5 * 24 + 16) + eval_bytes(n) + 16; }
+
+// Descend the energy of state q0 (inside [0, Lt] up to its overhang) at side
+// Lt until it vanishes (at most *budget gradient steps, each with up to 8
+// backtracking trials).  Ends with the cells and trig of q0.
+__device__ void descend(int n, PolishBufs& B, double Lt, int* budget) {
     trig_of(n, B.q0, B.cs);
-    bool listed = build_nbr(n, B.nb, B.q0, red);
-    double E = energy(n, B.q0, B.cs, Lt, B.g, red, listed ? &B.nb : nullptr);
+    build_cells(n, B.cells, B.q0, 0.0, 0.0, Lt);
+    bool listed = build_nbr(n, B.nb, B.cells, B.q0);
+    double gm2;
+    double E = energy(n, B.q0, B.cs, Lt, B.g, gm2, B.red, B.nb, listed);
+    double gmax = sqrt(gm2);
+    double moved_by = 0.0;  // bound on any centre's distance from where the list was built
     double alpha = 0.05;
     while (*budget > 0 && E > 1e-26) {
         --*budget;
@@ -259,42 +483,57 @@ __device__ void descend(int n, const PolishBufs& B, double Lt, int* budget, doub
         for (int ls = 0; ls < 8 && !moved; ++ls) {
             for (int i = threadIdx.x; i < n; i += kPT) {
                 const double3 p = B.q0[i], d = B.g[i];
-                B.q[i] = make_double3(p.x - alpha * d.x, p.y - alpha * d.y, wrap_q(p.z - alpha * d.z));
+                const double3 v = make_double3(p.x - alpha * d.x, p.y - alpha * d.y, wrap_q(p.z - alpha * d.z));
+                double s, c;
+                sincos(v.z, &s, &c);
+                B.q[i] = v;
+                B.cs[i] = make_double2(c, s);
             }
             __syncthreads();
-            trig_of(n, B.q, B.cs);
-            const double d2 = listed ? moved2(n, B.nb, B.q, red) : 1e30;
-            const double En = energy(n, B.q, B.cs, Lt, nullptr, red, d2 <= kNbMove2 ? &B.nb : nullptr);
+            const double step = alpha * gmax;
+            bool rebuilt = false;
+            if (!(moved_by + step <= kNbMove)) {  // past the list's reach: a list of the trial itself
+                build_cells(n, B.cells, B.q, 0.0, 0.0, Lt);
+                listed = build_nbr(n, B.nb, B.cells, B.q);
+                rebuilt = true;
+            }
+            const double En = energy(n, B.q, B.cs, Lt, B.tg, gm2, B.red, B.nb, listed);
             if (En < E) {
                 E = En;
                 moved = true;
                 alpha = fmin(alpha * 1.5, 0.5);
-                for (int i = threadIdx.x; i < n; i += kPT) B.q0[i] = B.q[i];
-                __syncthreads();
-                // keep room for the next trials: rebuild once half the slack is used
-                if (d2 > 0.25 * kNbMove2) listed = build_nbr(n, B.nb, B.q0, red);
+                moved_by = rebuilt ? 0.0 : moved_by + step;
+                gmax = sqrt(gm2);
+                Sh<double3> s = B.q0;
+                B.q0 = B.q;
+                B.q = s;
+                s = B.g;
+                B.g = B.tg;
+                B.tg = s;
             } else {
                 alpha *= 0.3;
+                if (rebuilt) moved_by = step;
             }
         }
         if (!moved) break;
-        E = energy(n, B.q0, B.cs, Lt, B.g, red, listed ? &B.nb : nullptr);  // cs holds the trig of q == q0
     }
+    __syncthreads();
     trig_of(n, B.q0, B.cs);
+    build_cells(n, B.cells, B.q0, 0.0, 0.0, Lt);
 }
 
 // Compress-and-descend attempts on the certified state sv of side *Lb
 // (delta shrinking by 0.3 after every attempt that does not certify a
 // smaller side); sv and *Lb are updated in place.
-__device__ void polish_loop(int n, const PolishBufs& B, double* Lb, int* budget, double* red) {
+__device__ void polish_loop(int n, PolishBufs& B, double* Lb, int* budget, Sh<double> red) {
     double delta = 1e-4;
     for (int attempt = 0; attempt < 12 && *budget > 0 && delta > 1e-9; ++attempt) {
         const double f = 1.0 - delta, Lt = *Lb * f;
         for (int i = threadIdx.x; i < n; i += kPT) B.q0[i] = make_double3(B.sv[i].x * f, B.sv[i].y * f, B.sv[i].z);
         __syncthreads();
-        descend(n, B, Lt, budget, red);
+        descend(n, B, Lt, budget);
         double lam = 0, x0 = 0, y0 = 0;
-        const double Lc = cert_side_all(n, B.q0, B.cs, red, lam, x0, y0);
+        const double Lc = cert_side_all(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
         if (Lc < *Lb) {
             *Lb = Lc;
             for (int i = threadIdx.x; i < n; i += kPT)
@@ -309,14 +548,13 @@ __device__ void polish_loop(int n, const PolishBufs& B, double* Lb, int* budget,
 __global__ void __launch_bounds__(kPT) polish_kernel(const int32_t* __restrict__ job_list,
                                                      const JobDev* __restrict__ jdev, JobMut* __restrict__ jmut,
                                                      double* __restrict__ best) {
-    extern __shared__ __align__(16) unsigned char dyn[];
-    __shared__ double red[kPT / 32];
     const int job = job_list[blockIdx.x];
     const JobDev jd = jdev[job];
     const int n = jd.n;
     double Lb = jmut[job].best_L;
     if (jd.polish_iters <= 0 || Lb >= 1e29 || jmut[job].status < 0) return;
-    const PolishBufs B = polish_bufs(dyn, n);
+    PolishBufs B = polish_bufs(n);
+    const Sh<double> red = B.max;
     double* b = best + jd.best_off;
     for (int i = threadIdx.x; i < n; i += kPT) B.sv[i] = make_double3(b[3 * i], b[3 * i + 1], b[3 * i + 2]);
     __syncthreads();
@@ -340,34 +578,35 @@ __global__ void __launch_bounds__(kPT) polish_kernel(const int32_t* __restrict__
 __global__ void __launch_bounds__(kPT) polish_states_kernel(const int32_t* __restrict__ n_of,
                                                             const int64_t* __restrict__ row0, int iters,
                                                             double* __restrict__ xya, double* __restrict__ res) {
-    extern __shared__ __align__(16) unsigned char dyn[];
-    __shared__ double red[kPT / 32];
     const int k = blockIdx.x;
     const int n = n_of[k];
     double* st = xya + 3 * row0[k];
-    const PolishBufs B = polish_bufs(dyn, n);
+    PolishBufs B = polish_bufs(n);
+    const Sh<double> red = B.max;
     for (int i = threadIdx.x; i < n; i += kPT) B.q0[i] = make_double3(st[3 * i], st[3 * i + 1], wrap_q(st[3 * i + 2]));
     __syncthreads();
     trig_of(n, B.q0, B.cs);
     int budget = iters;
     double lam = 0, x0 = 0, y0 = 0;
-    double Lb = cert_side_all(n, B.q0, B.cs, red, lam, x0, y0);
+    // bounding box of the input
+    double a0 = 1e300, a1 = -1e300, b0 = 1e300, b1 = -1e300;
+    for (int i = threadIdx.x; i < n; i += kPT) {
+        const double r = 0.5 * (fabs(B.cs[i].x) + fabs(B.cs[i].y));
+        a0 = fmin(a0, B.q0[i].x - r);
+        a1 = fmax(a1, B.q0[i].x + r);
+        b0 = fmin(b0, B.q0[i].y - r);
+        b1 = fmax(b1, B.q0[i].y + r);
+    }
+    a0 = -block_max(-a0, red);
+    a1 = block_max(a1, red);
+    b0 = -block_max(-b0, red);
+    b1 = block_max(b1, red);
+    const double side = fmax(a1 - a0, b1 - b0);
+    build_cells(n, B.cells, B.q0, a0, b0, side);
+    double Lb = cert_side_all(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
     const double L_in = Lb, lam_in = lam;
     if (Lb >= 1e29) {
-        // bounding box of the input, translated to the origin, as the side
-        double a0 = 1e300, a1 = -1e300, b0 = 1e300, b1 = -1e300;
-        for (int i = threadIdx.x; i < n; i += kPT) {
-            const double r = 0.5 * (fabs(B.cs[i].x) + fabs(B.cs[i].y));
-            a0 = fmin(a0, B.q0[i].x - r);
-            a1 = fmax(a1, B.q0[i].x + r);
-            b0 = fmin(b0, B.q0[i].y - r);
-            b1 = fmax(b1, B.q0[i].y + r);
-        }
-        a0 = -block_max(-a0, red);
-        a1 = block_max(a1, red);
-        b0 = -block_max(-b0, red);
-        b1 = block_max(b1, red);
-        const double side = fmax(a1 - a0, b1 - b0);
+        // translated to the origin, with the bounding box as the side
         for (int i = threadIdx.x; i < n; i += kPT) {
             B.sv[i] = make_double3(B.q0[i].x - a0, B.q0[i].y - b0, B.q0[i].z);  // the input, at the origin
             B.q0[i] = B.sv[i];
@@ -379,16 +618,16 @@ __global__ void __launch_bounds__(kPT) polish_states_kernel(const int32_t* __res
         // most 1.5x) and descend in a box scaled alike
         int half = budget / 2;
         budget -= half;
-        descend(n, B, side, &half, red);
+        descend(n, B, side, &half);
         budget += half;
-        Lb = cert_side_all(n, B.q0, B.cs, red, lam, x0, y0);
+        Lb = cert_side_all(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
         if (Lb >= 1e29) {
             const double f = fmin(fmax(lam_in, 1.0), 1.5);
             for (int i = threadIdx.x; i < n; i += kPT)
                 B.q0[i] = make_double3(B.sv[i].x * f, B.sv[i].y * f, B.sv[i].z);
             __syncthreads();
-            descend(n, B, side * f, &budget, red);
-            Lb = cert_side_all(n, B.q0, B.cs, red, lam, x0, y0);
+            descend(n, B, side * f, &budget);
+            Lb = cert_side_all(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
         }
     }
     if (Lb < 1e29) {
@@ -410,8 +649,8 @@ __global__ void __launch_bounds__(kPT) polish_states_kernel(const int32_t* __res
 }
 
 // FP64 energy and gradient of arbitrary states, one CTA per state: the
-// polish's own energy function over all pairs (pair_smooth / wall_smooth
-// above), with cos and sin taken of the angles as given.  State k has n_of[k]
+// polish's own energy function over a neighbour list (all pairs, bit for
+// bit), with cos and sin taken of the angles as given.  State k has n_of[k]
 // rows at xya + 3 * row0[k] and side side[k]; energy[k], and the gradient rows
 // at the same offsets of grad when grad is not null.
 __global__ void __launch_bounds__(kPT) energy_states_kernel(const int32_t* __restrict__ n_of,
@@ -420,18 +659,22 @@ __global__ void __launch_bounds__(kPT) energy_states_kernel(const int32_t* __res
                                                             const double* __restrict__ xya,
                                                             double* __restrict__ energy_out,
                                                             double* __restrict__ grad) {
-    extern __shared__ __align__(16) unsigned char dyn[];
-    __shared__ double red[kPT / 32];
     const int k = blockIdx.x;
     const int n = n_of[k];
-    double3* q = reinterpret_cast<double3*>(dyn);
-    double3* g = q + n;
-    double2* cs = reinterpret_cast<double2*>(g + n);
+    const Sh<double2> cs{0};
+    const Sh<double3> q{16 * n}, g = q + n;
+    Red red;
+    NbrList nb;
+    Cells cells;
+    eval_bufs(g.off + 24 * n, n, red, nb, cells);
     const double* st = xya + 3 * row0[k];
     for (int i = threadIdx.x; i < n; i += kPT) q[i] = make_double3(st[3 * i], st[3 * i + 1], st[3 * i + 2]);
     __syncthreads();
     trig_of(n, q, cs);
-    const double e = energy(n, q, cs, side[k], grad ? g : nullptr, red, nullptr);
+    build_cells(n, cells, q, 0.0, 0.0, side[k]);
+    const bool listed = build_nbr(n, nb, cells, q);
+    double gm2;
+    const double e = energy(n, q, cs, side[k], g, gm2, red, nb, listed);
     if (threadIdx.x == 0) energy_out[k] = e;
     if (grad) {
         double* go = grad + 3 * row0[k];
@@ -443,7 +686,7 @@ __global__ void __launch_bounds__(kPT) energy_states_kernel(const int32_t* __res
     }
 }
 
-size_t energy_smem_bytes(int n) { return (size_t)n * (2 * sizeof(double3) + sizeof(double2)) + 64; }
+size_t energy_smem_bytes(int n) { return (size_t)n * (2 * sizeof(double3) + sizeof(double2)) + eval_bytes(n) + 16; }
 
 int launch_energy_states(cudaStream_t stream, int count, const int32_t* n_of, const int64_t* row0, const double* side,
                          const double* xya, double* energy_out, double* grad, size_t smem) {
@@ -451,7 +694,7 @@ int launch_energy_states(cudaStream_t stream, int count, const int32_t* n_of, co
     int dev = 0;
     SQS_CUDA(cudaGetDevice(&dev));
     if (!attr_done[dev & 63]) {
-        SQS_CUDA(cudaFuncSetAttribute(energy_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        SQS_CUDA(cudaFuncSetAttribute(energy_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
         attr_done[dev & 63] = true;
     }
     if (count <= 0) return SQS_OK;
@@ -466,7 +709,7 @@ int launch_polish_states(cudaStream_t stream, int count, const int32_t* n_of, co
     int dev = 0;
     SQS_CUDA(cudaGetDevice(&dev));
     if (!attr_done[dev & 63]) {
-        SQS_CUDA(cudaFuncSetAttribute(polish_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        SQS_CUDA(cudaFuncSetAttribute(polish_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
         attr_done[dev & 63] = true;
     }
     if (count <= 0) return SQS_OK;
@@ -481,7 +724,7 @@ int launch_polish(cudaStream_t stream, int njobs, const int32_t* job_list, const
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_done[dev & 63]) {
-        SQS_CUDA(cudaFuncSetAttribute(polish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        SQS_CUDA(cudaFuncSetAttribute(polish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
         attr_done[dev & 63] = true;
     }
     if (njobs <= 0) return SQS_OK;
