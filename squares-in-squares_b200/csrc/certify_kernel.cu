@@ -7,13 +7,12 @@
 //           (certifier.cpp:914-929), packings bucketed by n;
 //   kernel  cert_packing_kernel, one CTA per packing:
 //             literal syntax + exact double-range and bound checks
-//             (certifier.cpp:764-791), Fix<9> side measurement with Taylor
-//             sin/cos (:793-854), float corners + padded AABBs, bitonic sort
-//             of the AABBs, sort-and-sweep with the float SAT prefilter
-//             (:856-883); undecided pairs go to a global list;
-//   kernel  cert_fp64_kernel: directed-rounding FP64 interval SAT of the
-//           undecided pairs, deciding those whose sign it certifies (and
-//           exact axis-aligned dyadic pairs) the way the stages below would;
+//             (certifier.cpp:764-791), float corners + padded AABBs, Fix<9>
+//             side measurement with Taylor sin/cos of the squares that can
+//             hold an extreme (:793-854), bitonic sort of the AABBs,
+//             sort-and-sweep (:856-883) with a directed-rounding FP64
+//             evaluation of each pair that settles the float check and the
+//             pairs whose sign it certifies; the rest go to a global list;
 //   kernels the 7-, 15- and 58-limb interval SAT of the pairs still open at
 //           63, 135 and 522 decimal digits (:885-899), each stage taking the
 //           pairs the previous one left open;
@@ -66,7 +65,6 @@ struct Pair {
 
 struct Consts {
     Fix<9> half_pi9, two_pi9, half9;
-    Fix<3> half3;
     Iv<7> half_pi7, half7;
     Iv<15> half_pi15, half15;
     Iv<58> half_pi58, half58;
@@ -248,6 +246,123 @@ __device__ __noinline__ int float_sat(const FSq& p, const FSq& q) {
     return worst > 1e-8 ? -1 : 0;
 }
 
+// ------------------------------------------------------------ pair decision
+// One directed-rounding FP64 evaluation of the exact overlap of two squares
+// along the four axes.  Both squares have support 1/2 (own axes) and
+// (|cos d| + |sin d|) / 2 (the other's, d the angle between them), so every
+// axis's overlap is r - |v|, r = 1/2 + (|cos d| + |sin d|) / 2, v the centre
+// difference along the axis: 12 products of enclosures instead of the 64 of
+// two times four corners on four axes.  (Where one projection contains the
+// other the reference's overlap is smaller than r - |v|, but both are at
+// least 1 there.)  Enclosures are midpoint and radius, radii rounded up.
+//
+// It decides the reference's float check wherever that check's own rounding
+// cannot matter (kTol around its +-1e-8 thresholds; the check itself runs on
+// the rest), and of the pairs that leave open those the interval stages are
+// certain to decide the same way:
+//   * separated when some axis's overlap lies strictly below zero,
+//     overlapping when every axis's lies strictly above: the exact overlap of
+//     the exact decimal inputs then has that sign and is at least 2^-60 in
+//     magnitude, which the 7-limb stage (widths below 1e-60) resolves alike;
+//   * two axis-aligned squares (angle literals exactly zero, the reference's
+//     flat path) whose literals on an axis, and square 0's, are dyadic within
+//     25 decimal places are compared exactly on it: touching edges count as
+//     separated, as they do there.
+// The rest goes to the 7-limb stage.
+//
+// Bounds.  A coordinate is kept as its integer part and its fraction, the
+// latter within 2^-51 (one correctly rounded division, two additions), so a
+// centre difference is within 2^-48 of exact.  The angle's double is within
+// (|a| + 1) 2^-50, sin and cos (documented 2 ulp) within w of their exact
+// values, w = (|a| + 1) 2^-49 + 2^-50.
+struct MR {
+    double m, r;  // |value - m| <= r
+};
+__device__ __forceinline__ double round_err(double m) { return __fma_ru(fabs(m), 0x1p-53, 0x1p-1000); }
+__device__ __forceinline__ MR mr_mul(MR a, MR b) {
+    const double m = __dmul_rn(a.m, b.m);
+    const double r = __fma_ru(fabs(a.m), b.r, __fma_ru(fabs(b.m), a.r, __fma_ru(a.r, b.r, round_err(m))));
+    return MR{m, r};
+}
+__device__ __forceinline__ MR mr_add(MR a, MR b) {
+    const double m = __dadd_rn(a.m, b.m);
+    return MR{m, __dadd_ru(__dadd_ru(a.r, b.r), round_err(m))};
+}
+__device__ __forceinline__ MR mr_neg(MR a) { return MR{-a.m, a.r}; }
+
+enum : uint32_t { kSqFlat = 1u, kSqExactX = 2u, kSqExactY = 4u, kSqDyadicX = 8u, kSqDyadicY = 16u };
+
+// A square as the pair decision reads it (shared memory, by square id).
+struct PairSq {
+    double* xf;     // fractions of the coordinates, with their sign
+    double* yf;
+    float* w;       // error bound of the cached cos / sin
+    int16_t* xi;    // integer parts, with their sign
+    int16_t* yi;
+    uint8_t* fl;    // kSq* bits
+};
+
+// Whether two dyadic literals are at least 1 apart, exactly (27 decimals hold them).
+__device__ __noinline__ bool apart_exact(const char* text, const Lit& p, const Lit& q) {
+    Fix<3> d = fx::sub(fx::parse<3>(text, p, 0), fx::parse<3>(text, q, 0));
+    d.neg = 0;
+    return fx::cmp(d, fx::of_int<3>(1)) >= 0;
+}
+
+// 1 separated, -1 overlap by the float check, -2 overlap by the intervals,
+// 2 left to the multi-limb stages.  u < v are the squares' ids in the packing
+// whose literals start at L0.
+__device__ __forceinline__ int decide_pair(const FSq* sq, const PairSq& ps, int u, int v, const char* text, const Lit* L0) {
+    const FSq p = sq[u], q = sq[v];
+    const double wp = ps.w[u], wq = ps.w[v];
+    const MR dx{__dadd_rn((double)(ps.xi[v] - ps.xi[u]), __dsub_rn(ps.xf[v], ps.xf[u])), 0x1p-48};
+    const MR dy{__dadd_rn((double)(ps.yi[v] - ps.yi[u]), __dsub_rn(ps.yf[v], ps.yf[u])), 0x1p-48};
+    const MR cp{p.c, wp}, sp{p.s, wp}, cq{q.c, wq}, sq_{q.s, wq};
+    const MR cd = mr_add(mr_mul(cp, cq), mr_mul(sp, sq_)), sd = mr_add(mr_mul(sp, cq), mr_neg(mr_mul(cp, sq_)));
+    const MR sum = mr_add(MR{fabs(cd.m), cd.r}, MR{fabs(sd.m), sd.r});
+    const MR rad = mr_add(MR{0.5, 0.0}, MR{0.5 * sum.m, 0.5 * sum.r});
+    const MR vv[4] = {mr_add(mr_mul(dx, cp), mr_mul(dy, sp)), mr_add(mr_mul(dy, cp), mr_neg(mr_mul(dx, sp))),
+                      mr_add(mr_mul(dx, cq), mr_mul(dy, sq_)), mr_add(mr_mul(dy, cq), mr_neg(mr_mul(dx, sq_)))};
+    double hi = 1e300, lo = 1e300;  // bounds of the smallest overlap
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const MR ov = mr_add(rad, MR{-fabs(vv[k].m), vv[k].r});
+        hi = fmin(hi, __dadd_ru(ov.m, ov.r));
+        lo = fmin(lo, __dsub_rd(ov.m, ov.r));
+    }
+    // the float check's rounding: its corners and projections are within
+    // 2^-45 of the coordinates' size of exact
+    const double tol = 0x1p-44 * (fabs(p.x) + fabs(p.y) + fabs(q.x) + fabs(q.y) + 4.0);
+    if (hi < -1e-8 - tol) return 1;
+    if (lo > 1e-8 + tol) return -1;
+    if (!(lo > -1e-8 + tol && hi < 1e-8 - tol)) {
+        const int f = float_sat(p, q);
+        if (f != 0) return f;
+    }
+    const uint32_t fl = ps.fl[u] & ps.fl[v];
+    if (fl & kSqFlat) {
+        // per axis: apart, overlapping, or open (the exact distances of exact
+        // coordinates, the bounds above, or 3-limb arithmetic)
+        const uint32_t fo = fl & ps.fl[0];
+        bool open = false;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double d = fabs(k ? dy.m : dx.m);
+            if (fo & (k ? kSqExactY : kSqExactX)) {
+                if (d >= 1.0) return 1;
+            } else if (d - 0x1p-47 > 1.0) {
+                return 1;
+            } else if (!(d + 0x1p-47 < 1.0)) {
+                if (!(fo & (k ? kSqDyadicY : kSqDyadicX))) open = true;
+                else if (apart_exact(text, L0[3 * u + k], L0[3 * v + k])) return 1;
+            }
+        }
+        return open ? 2 : -2;
+    }
+    if (hi < 0.0) return 1;
+    return lo > 0.0 ? -2 : 2;
+}
+
 template <int F>
 __device__ void fix_shfl_min_max(Fix<F>& v, bool& have, bool want_min) {
     for (int o = 16; o > 0; o >>= 1) {
@@ -276,7 +391,17 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
     double* by0 = bx1 + NMAX;
     double* by1 = by0 + NMAX;
     double* key = by1 + NMAX;
-    int16_t* idx = reinterpret_cast<int16_t*>(key + NP);
+    PairSq ps;
+    ps.xf = key + NP;
+    ps.yf = ps.xf + NMAX;
+    ps.w = reinterpret_cast<float*>(ps.yf + NMAX);
+    ps.xi = reinterpret_cast<int16_t*>(ps.w + NMAX);
+    ps.yi = ps.xi + NMAX;
+    int16_t* idx = ps.yi + NMAX;                              // candidates of the side, then the sort
+    ps.fl = reinterpret_cast<uint8_t*>(idx + NP);
+    __shared__ Fix<9> series[T];                              // sin and cos series of a pair of threads
+    __shared__ double box[W][4];
+    __shared__ int s_cand;
     __shared__ Fix<9> ext[W][4];
     __shared__ int ext_have[W];
     __shared__ Fix<9> org[2];
@@ -294,6 +419,7 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
         s_err = kNoKey;
         s_fkey = kNoPair;
         s_undecided = 0;
+        s_cand = 0;
     }
     __syncthreads();
 
@@ -335,28 +461,25 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
     }
     __syncthreads();
 
-    // 2. Fix<9> corners (side) and float geometry, per square (the additions
-    // and comparisons inlined; products, parsing and sin/cos out of line)
-    Fix<9> mnx, mxx, mny, mxy;
-    fx::set_zero(mnx);
-    fx::set_zero(mxx);
-    fx::set_zero(mny);
-    fx::set_zero(mxy);
-    bool have = false;
+    // 2. float geometry of every square, and what the pair decision reads
     const Consts& C = c_consts;
+    double gx0 = 1e300, gx1 = -1e300, gy0 = 1e300, gy1 = -1e300;
     for (int i = tid; i < n; i += T) {
         const Lit lx = lits[3 * (s0 + i)], ly = lits[3 * (s0 + i) + 1], la = lits[3 * (s0 + i) + 2];
-        const Fix<9> X = fx::sub<9, true>(fx::parse<9>(text, lx, 0), org[0]);
-        const Fix<9> Y = fx::sub<9, true>(fx::parse<9>(text, ly, 0), org[1]);
+        const Fix<9> x = fx::parse<9>(text, lx, 0), y = fx::parse<9>(text, ly, 0);
         const Fix<9> A = fx::parse<9>(text, la, 0);
-        const long long turns = (long long)floor(fx::approx(A) / 6.283185307179586476925);
-        Fix<9> red = fx::sub<9, true>(A, fx::mul(fx::of_int<9>(turns), C.two_pi9, 0));
-        if (red.neg && !fx::is_zero(red)) red = fx::add<9, true>(red, C.two_pi9);
-        if (fx::cmp<9, true>(red, C.two_pi9) >= 0) red = fx::sub<9, true>(red, C.two_pi9);
+        const double a = fx::approx(A);
+        const long long turns = (long long)floor(a / 6.283185307179586476925);
+        double ang = a;
+        if (turns != 0 || A.neg || a > 6.28) {  // (else the reduction below would leave A as it is)
+            Fix<9> red = fx::sub<9, true>(A, fx::mul(fx::of_int<9>(turns), C.two_pi9, 0));
+            if (red.neg && !fx::is_zero(red)) red = fx::add<9, true>(red, C.two_pi9);
+            if (fx::cmp<9, true>(red, C.two_pi9) >= 0) red = fx::sub<9, true>(red, C.two_pi9);
+            ang = fx::approx(red);
+        }
         FSq q;
-        q.x = fx::approx(X);
-        q.y = fx::approx(Y);
-        const double ang = fx::approx(red);
+        q.x = fx::approx(fx::sub<9, true>(x, org[0]));
+        q.y = fx::approx(fx::sub<9, true>(y, org[1]));
         q.c = cos(ang);
         q.s = sin(ang);
         sq[i] = q;
@@ -368,35 +491,103 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
             y0 = fmin(y0, cy[k]); y1 = fmax(y1, cy[k]);
         }
         bx0[i] = x0 - 1e-7; by0[i] = y0 - 1e-7; bx1[i] = x1 + 1e-7; by1[i] = y1 + 1e-7;
-
-        Fix<9> sn, cs;
-        if (la.zero_str || fx::is_zero(A)) {
-            cs = fx::of_int<9>(1);
-            fx::set_zero(sn);
-        } else {
-            fx::sincos_point(A, C.half_pi9, sn, cs);
-        }
-        const Fix<9> hc = fx::mul(C.half9, cs, 0), hs = fx::mul(C.half9, sn, 0);
-        const Fix<9> ux = fx::sub<9, true>(hc, hs), uy = fx::add<9, true>(hs, hc);
-        Fix<9> zero;
-        fx::set_zero(zero);
-        const Fix<9> vx = fx::sub<9, true>(zero, fx::add<9, true>(hc, hs)), vy = fx::sub<9, true>(hc, hs);
-        const Fix<9> px[4] = {fx::add<9, true>(X, ux), fx::add<9, true>(X, vx), fx::sub<9, true>(X, ux), fx::sub<9, true>(X, vx)};
-        const Fix<9> py[4] = {fx::add<9, true>(Y, uy), fx::add<9, true>(Y, vy), fx::sub<9, true>(Y, uy), fx::sub<9, true>(Y, vy)};
-        for (int k = 0; k < 4; ++k) {
-            if (!have) {
-                mnx = mxx = px[k];
-                mny = mxy = py[k];
-                have = true;
-                continue;
-            }
-            if (fx::cmp<9, true>(px[k], mnx) < 0) mnx = px[k];
-            if (fx::cmp<9, true>(px[k], mxx) > 0) mxx = px[k];
-            if (fx::cmp<9, true>(py[k], mny) < 0) mny = py[k];
-            if (fx::cmp<9, true>(py[k], mxy) > 0) mxy = py[k];
-        }
+        gx0 = fmin(gx0, x0); gx1 = fmax(gx1, x1);
+        gy0 = fmin(gy0, y0); gy1 = fmax(gy1, y1);
+        uint32_t fl = 0;
+        auto split = [&](const Fix<9>& v, const Lit& L, double& f, int16_t& whole, uint32_t dy, uint32_t ex) {
+            f = __ddiv_rn((double)v.d[1], 1e9) + ((double)v.d[2] * 1e-18 + (double)v.d[3] * 1e-27);
+            f = v.neg ? -f : f;
+            whole = (int16_t)(v.neg ? -(int)v.d[0] : (int)v.d[0]);  // |v| <= 1e4 (checked above)
+            uint32_t rest = 0;
+            for (int k = 2; k <= 9; ++k) rest |= v.d[k];
+            if (L.dyadic) fl |= rest ? dy : dy | ex;
+        };
+        split(x, lx, ps.xf[i], ps.xi[i], kSqDyadicX, kSqExactX);
+        split(y, ly, ps.yf[i], ps.yi[i], kSqDyadicY, kSqExactY);
+        bool flat = true;  // every digit of the angle is zero
+        for (int k = 0; k < la.ndig && flat; ++k) flat = fx::lit_digit(text, la, k) == 0;
+        ps.fl[i] = (uint8_t)(fl | (flat ? kSqFlat : 0u));
+        ps.w[i] = flat ? 0.f : __double2float_ru(__fma_ru(__dadd_ru(fabs(ang), 1.0), 0x1p-49, 0x1p-50));
     }
-    {
+    for (int o = 16; o > 0; o >>= 1) {
+        gx0 = fmin(gx0, __shfl_xor_sync(0xffffffffu, gx0, o));
+        gx1 = fmax(gx1, __shfl_xor_sync(0xffffffffu, gx1, o));
+        gy0 = fmin(gy0, __shfl_xor_sync(0xffffffffu, gy0, o));
+        gy1 = fmax(gy1, __shfl_xor_sync(0xffffffffu, gy1, o));
+    }
+    if (lane == 0) {
+        box[warp][0] = gx0;
+        box[warp][1] = gx1;
+        box[warp][2] = gy0;
+        box[warp][3] = gy1;
+    }
+    __syncthreads();
+    for (int w = 0; w < W; ++w) {
+        gx0 = fmin(gx0, box[w][0]);
+        gx1 = fmax(gx1, box[w][1]);
+        gy0 = fmin(gy0, box[w][2]);
+        gy1 = fmax(gy1, box[w][3]);
+    }
+    // The side: spans of the Fix<9> corners.  A double corner is within 1e-9
+    // of its Fix<9> value, so only squares whose float box reaches within
+    // 1e-8 of the packing's can hold an extreme: the 81-digit sin and cos are
+    // taken of those alone (a tilted layout has a handful; all of them before,
+    // which was most of this kernel), by two threads a square, one a series.
+    for (int i = tid; i < n; i += T) {
+        if (bx0[i] + 1e-7 <= gx0 + 1e-8 || bx1[i] - 1e-7 >= gx1 - 1e-8 || by0[i] + 1e-7 <= gy0 + 1e-8 ||
+            by1[i] - 1e-7 >= gy1 - 1e-8)
+            idx[atomicAdd(&s_cand, 1)] = (int16_t)i;
+    }
+    __syncthreads();
+    Fix<9> mnx, mxx, mny, mxy;
+    fx::set_zero(mnx);
+    fx::set_zero(mxx);
+    fx::set_zero(mny);
+    fx::set_zero(mxy);
+    bool have = false;
+    const int ncand = s_cand;
+    for (int base = 0; base < ncand; base += T / 2) {
+        const int k = base + tid / 2;
+        const bool in = k < ncand;
+        const int i = in ? idx[k] : 0;
+        const Lit la = lits[3 * (s0 + i) + 2];
+        const Fix<9> A = fx::parse<9>(text, la, 0);
+        const bool turned = in && !(la.zero_str || fx::is_zero(A));
+        int quad = 0;
+        if (turned) fx::sincos_series(A, C.half_pi9, tid & 1, series[tid], quad);
+        __syncwarp();
+        if (in && !(tid & 1)) {
+            Fix<9> sn, cs;
+            if (turned) fx::sincos_quadrant(series[tid + 1], series[tid], quad, sn, cs);
+            else {
+                cs = fx::of_int<9>(1);
+                fx::set_zero(sn);
+            }
+            const Fix<9> X = fx::sub<9, true>(fx::parse<9>(text, lits[3 * (s0 + i)], 0), org[0]);
+            const Fix<9> Y = fx::sub<9, true>(fx::parse<9>(text, lits[3 * (s0 + i) + 1], 0), org[1]);
+            const Fix<9> hc = fx::mul(C.half9, cs, 0), hs = fx::mul(C.half9, sn, 0);
+            const Fix<9> ux = fx::sub<9, true>(hc, hs), uy = fx::add<9, true>(hs, hc);
+            Fix<9> zero;
+            fx::set_zero(zero);
+            const Fix<9> vx = fx::sub<9, true>(zero, fx::add<9, true>(hc, hs)), vy = fx::sub<9, true>(hc, hs);
+            const Fix<9> px[4] = {fx::add<9, true>(X, ux), fx::add<9, true>(X, vx), fx::sub<9, true>(X, ux), fx::sub<9, true>(X, vx)};
+            const Fix<9> py[4] = {fx::add<9, true>(Y, uy), fx::add<9, true>(Y, vy), fx::sub<9, true>(Y, uy), fx::sub<9, true>(Y, vy)};
+            for (int c = 0; c < 4; ++c) {
+                if (!have) {
+                    mnx = mxx = px[c];
+                    mny = mxy = py[c];
+                    have = true;
+                    continue;
+                }
+                if (fx::cmp<9, true>(px[c], mnx) < 0) mnx = px[c];
+                if (fx::cmp<9, true>(px[c], mxx) > 0) mxx = px[c];
+                if (fx::cmp<9, true>(py[c], mny) < 0) mny = py[c];
+                if (fx::cmp<9, true>(py[c], mxy) > 0) mxy = py[c];
+            }
+        }
+        __syncwarp();
+    }
+    if (__any_sync(0xffffffffu, have)) {
         bool h0 = have, h1 = have, h2 = have, h3 = have;
         fix_shfl_min_max(mnx, h0, true);
         fix_shfl_min_max(mxx, h1, false);
@@ -407,9 +598,12 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
             ext[warp][1] = mxx;
             ext[warp][2] = mny;
             ext[warp][3] = mxy;
-            ext_have[warp] = h0;
+            ext_have[warp] = 1;
         }
+    } else if (lane == 0) {
+        ext_have[warp] = 0;
     }
+    __syncthreads();  // the candidates are read
     // 3. sort the AABBs by their padded min x, ties by square id
     for (int i = tid; i < NP; i += T) {
         key[i] = i < n ? bx0[i] : 1e300;
@@ -455,7 +649,7 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
         }
     }
 
-    // 4. sort and sweep with the float prefilter
+    // 4. sort and sweep with the pair decision
     for (int ii = tid; ii < n; ii += T) {
         const int i = idx[ii];
         const double ix1 = bx1[i], iy0 = by0[i], iy1 = by1[i], ix0 = bx0[i];
@@ -464,10 +658,12 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
             if (bx0[j] > ix1) break;
             if (ix1 < bx0[j] || bx1[j] < ix0 || iy1 < by0[j] || by1[j] < iy0) continue;
             const int u = min(i, j), v = max(i, j);
-            const int r = float_sat(sq[u], sq[v]);
-            if (r < 0) {
+            const int r = decide_pair(sq, ps, u, v, text, lits + 3 * s0);
+            if (r == -1) {
                 atomicMin(&s_fkey, ((unsigned long long)ii << 32) | (unsigned long long)jj);
-            } else if (r == 0) {
+            } else if (r == -2) {
+                atomicOr(&out[pk].flags, kCertOverlap);
+            } else if (r == 2) {
                 atomicAdd(&s_undecided, 1u);
                 const uint32_t slot = atomicAdd(pair_count, 1u);
                 if (slot < pair_cap) pairs[slot] = Pair{pk, (int16_t)u, (int16_t)v};
@@ -618,175 +814,6 @@ __global__ void __launch_bounds__(128) cert_stage_kernel(
     }
 }
 
-// ------------------------------------------------------------ FP64 prefilter
-// Directed-rounding FP64 interval SAT of the pairs the float check left open,
-// ahead of the multi-limb stages.  It decides a pair only where those stages
-// are certain to decide it the same way, so verdicts stay the reference's:
-//   * separated (1) when some axis's overlap interval lies strictly below
-//     zero, overlapping (-1) when every axis's lies strictly above: the
-//     intervals enclose the exact overlap of the exact decimal inputs, so its
-//     sign is certain, and an exact value of |v| >= 2^-1074 is resolved the
-//     same way by the 7-, 15- or 58-limb stage (widths below 1e-60);
-//   * two axis-aligned squares (angle literal exactly zero, the reference's
-//     flat path) whose coordinate literals and square 0's are all dyadic
-//     within 25 decimal places are compared exactly in 3-limb fixed point,
-//     the values the 7-limb stage computes exactly: touching edges decide
-//     as separated, as they do there;
-//   * everything else goes on to the 7-limb stage.
-// Bounds: a literal's value from its 27-decimal truncation (error < 1e-27)
-// converted to double (error below (|v| + 1) 2^-47), widened by both; sin
-// and cos from CUDA's double sincos, whose documented error is 2 ulp
-// (below 2^-51 in [-1, 1]), widened by that and by the angle's half-width.
-struct DIv {
-    double lo, hi;
-};
-__device__ __forceinline__ DIv d_add(DIv a, DIv b) { return DIv{__dadd_rd(a.lo, b.lo), __dadd_ru(a.hi, b.hi)}; }
-__device__ __forceinline__ DIv d_sub(DIv a, DIv b) { return DIv{__dsub_rd(a.lo, b.hi), __dsub_ru(a.hi, b.lo)}; }
-__device__ __forceinline__ DIv d_mul(DIv a, DIv b) {
-    const double l0 = __dmul_rd(a.lo, b.lo), l1 = __dmul_rd(a.lo, b.hi), l2 = __dmul_rd(a.hi, b.lo),
-                 l3 = __dmul_rd(a.hi, b.hi);
-    const double h0 = __dmul_ru(a.lo, b.lo), h1 = __dmul_ru(a.lo, b.hi), h2 = __dmul_ru(a.hi, b.lo),
-                 h3 = __dmul_ru(a.hi, b.hi);
-    return DIv{fmin(fmin(l0, l1), fmin(l2, l3)), fmax(fmax(h0, h1), fmax(h2, h3))};
-}
-__device__ __forceinline__ DIv d_half(DIv a) { return DIv{0.5 * a.lo, 0.5 * a.hi}; }  // exact
-__device__ __forceinline__ DIv d_neg(DIv a) { return DIv{-a.hi, -a.lo}; }
-
-// Enclosure of a literal's exact value.
-__device__ __forceinline__ DIv lit_iv(const char* text, const Lit& L) {
-    const double a = fx::approx(fx::parse<3>(text, L, 0));
-    const double eps = __dadd_ru(__dmul_ru(__dadd_ru(fabs(a), 1.0), 0x1p-47), 1e-27);
-    return DIv{__dsub_rd(a, eps), __dadd_ru(a, eps)};
-}
-
-__device__ __forceinline__ bool lit_is_zero(const char* text, const Lit& L) {
-    for (int k = 0; k < L.ndig; ++k)
-        if (fx::lit_digit(text, L, k) != 0) return false;
-    return true;
-}
-
-struct DSq {
-    bool flat;
-    DIv c, s, X, Y;
-    DIv px[4], py[4];
-};
-
-__device__ __noinline__ void make_dsq(const char* text, const Lit* L3, DIv ox, DIv oy, DSq& e) {
-    e.X = d_sub(lit_iv(text, L3[0]), ox);
-    e.Y = d_sub(lit_iv(text, L3[1]), oy);
-    e.flat = lit_is_zero(text, L3[2]);
-    if (e.flat) {
-        e.c = DIv{1.0, 1.0};
-        e.s = DIv{0.0, 0.0};
-    } else {
-        const DIv a = lit_iv(text, L3[2]);
-        const double mid = 0.5 * (a.lo + a.hi);
-        double sn, cs;
-        sincos(mid, &sn, &cs);
-        const double w = __dadd_ru(0x1p-50, __dsub_ru(a.hi, a.lo));
-        e.c = DIv{__dsub_rd(cs, w), __dadd_ru(cs, w)};
-        e.s = DIv{__dsub_rd(sn, w), __dadd_ru(sn, w)};
-    }
-    const DIv hc = d_half(e.c), hs = d_half(e.s);
-    const DIv ux = d_sub(hc, hs), uy = d_add(hs, hc);
-    const DIv vx = d_sub(d_neg(hc), hs), vy = d_add(d_neg(hs), hc);
-    e.px[0] = d_add(e.X, ux); e.py[0] = d_add(e.Y, uy);
-    e.px[1] = d_add(e.X, vx); e.py[1] = d_add(e.Y, vy);
-    e.px[2] = d_sub(e.X, ux); e.py[2] = d_sub(e.Y, uy);
-    e.px[3] = d_sub(e.X, vx); e.py[3] = d_sub(e.Y, vy);
-}
-
-// Exact box test of two axis-aligned squares with dyadic literals (the
-// reference's flat path on exact values): 1 separated or touching, -1 overlapping.
-__device__ __noinline__ int exact_flat_sat(const char* text, const Lit* P, const Lit* Q, const Lit* O) {
-    using F3 = Fix<3>;
-    const F3 ox = fx::parse<3>(text, O[0], 0), oy = fx::parse<3>(text, O[1], 0);
-    const F3 h = c_consts.half3;
-    const F3 px = fx::sub(fx::parse<3>(text, P[0], 0), ox), py = fx::sub(fx::parse<3>(text, P[1], 0), oy);
-    const F3 qx = fx::sub(fx::parse<3>(text, Q[0], 0), ox), qy = fx::sub(fx::parse<3>(text, Q[1], 0), oy);
-    auto mn = [](const F3& a, const F3& b) { return fx::cmp(a, b) < 0 ? a : b; };
-    auto mx = [](const F3& a, const F3& b) { return fx::cmp(a, b) > 0 ? a : b; };
-    F3 z;
-    fx::set_zero(z);
-    const F3 ovx = fx::sub(mn(fx::add(px, h), fx::add(qx, h)), mx(fx::sub(px, h), fx::sub(qx, h)));
-    if (fx::cmp(ovx, z) <= 0) return 1;
-    const F3 ovy = fx::sub(mn(fx::add(py, h), fx::add(qy, h)), mx(fx::sub(py, h), fx::sub(qy, h)));
-    if (fx::cmp(ovy, z) <= 0) return 1;
-    return -1;
-}
-
-// 1 separated, -1 overlapping, 0 left to the multi-limb stages.
-__device__ __noinline__ int fp64_sat(const DSq& p, const DSq& q) {
-    if (p.flat && q.flat) {
-        const DIv ox = DIv{__dsub_rd(fmin(__dadd_rd(p.X.lo, 0.5), __dadd_rd(q.X.lo, 0.5)),
-                                     fmax(__dsub_ru(p.X.hi, 0.5), __dsub_ru(q.X.hi, 0.5))),
-                           __dsub_ru(fmin(__dadd_ru(p.X.hi, 0.5), __dadd_ru(q.X.hi, 0.5)),
-                                     fmax(__dsub_rd(p.X.lo, 0.5), __dsub_rd(q.X.lo, 0.5)))};
-        const DIv oy = DIv{__dsub_rd(fmin(__dadd_rd(p.Y.lo, 0.5), __dadd_rd(q.Y.lo, 0.5)),
-                                     fmax(__dsub_ru(p.Y.hi, 0.5), __dsub_ru(q.Y.hi, 0.5))),
-                           __dsub_ru(fmin(__dadd_ru(p.Y.hi, 0.5), __dadd_ru(q.Y.hi, 0.5)),
-                                     fmax(__dsub_rd(p.Y.lo, 0.5), __dsub_rd(q.Y.lo, 0.5)))};
-        if (ox.hi < 0.0 || oy.hi < 0.0) return 1;
-        if (ox.lo > 0.0 && oy.lo > 0.0) return -1;
-        return 0;
-    }
-    bool all_pos = true;
-    for (int a = 0; a < 4; ++a) {
-        const DSq& o = a < 2 ? p : q;
-        const DIv ax = (a & 1) ? d_neg(o.s) : o.c, ay = (a & 1) ? o.c : o.s;
-        DIv mn1{1e300, 1e300}, mx1{-1e300, -1e300}, mn2{1e300, 1e300}, mx2{-1e300, -1e300};
-        for (int k = 0; k < 4; ++k) {
-            const DIv u = d_add(d_mul(ax, p.px[k]), d_mul(ay, p.py[k]));
-            const DIv v = d_add(d_mul(ax, q.px[k]), d_mul(ay, q.py[k]));
-            mn1 = DIv{fmin(mn1.lo, u.lo), fmin(mn1.hi, u.hi)};
-            mx1 = DIv{fmax(mx1.lo, u.lo), fmax(mx1.hi, u.hi)};
-            mn2 = DIv{fmin(mn2.lo, v.lo), fmin(mn2.hi, v.hi)};
-            mx2 = DIv{fmax(mx2.lo, v.lo), fmax(mx2.hi, v.hi)};
-        }
-        const DIv ov = d_sub(DIv{fmin(mx1.lo, mx2.lo), fmin(mx1.hi, mx2.hi)},
-                             DIv{fmax(mn1.lo, mn2.lo), fmax(mn1.hi, mn2.hi)});
-        if (ov.hi < 0.0) return 1;
-        all_pos &= ov.lo > 0.0;
-    }
-    return all_pos ? -1 : 0;
-}
-
-__global__ void __launch_bounds__(128) cert_fp64_kernel(const Pair* __restrict__ in, const uint32_t* __restrict__ in_count,
-                                                        uint32_t in_cap, Pair* __restrict__ next,
-                                                        uint32_t* __restrict__ next_count, uint32_t next_cap,
-                                                        const int64_t* __restrict__ pk_sq0,
-                                                        const Lit* __restrict__ lits, const char* __restrict__ text,
-                                                        PkOut* __restrict__ out) {
-    const uint32_t total = min(*in_count, in_cap);
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        const Pair pr = in[t];
-        PkOut& po = out[pr.pk];
-        if (po.fkey != kNoPair || (po.flags & kCertOverlap)) continue;
-        const int64_t s0 = pk_sq0[pr.pk];
-        const Lit* O = lits + 3 * s0;
-        const Lit* P = lits + 3 * (s0 + pr.u);
-        const Lit* Q = lits + 3 * (s0 + pr.v);
-        int r;
-        if (lit_is_zero(text, P[2]) && lit_is_zero(text, Q[2]) && O[0].dyadic && O[1].dyadic && P[0].dyadic &&
-            P[1].dyadic && Q[0].dyadic && Q[1].dyadic) {
-            r = exact_flat_sat(text, P, Q, O);
-        } else {
-            const DIv ox = lit_iv(text, O[0]), oy = lit_iv(text, O[1]);
-            DSq A, B;
-            make_dsq(text, P, ox, oy, A);
-            make_dsq(text, Q, ox, oy, B);
-            r = fp64_sat(A, B);
-        }
-        if (r < 0) {
-            atomicOr(&po.flags, kCertOverlap);
-        } else if (r == 0) {
-            const uint32_t slot = atomicAdd(next_count, 1u);
-            if (slot < next_cap) next[slot] = pr;
-            else atomicOr(&po.flags, kPairOverflow);
-        }
-    }
-}
-
 // ------------------------------------------------------------ cached stages
 // The same interval test with every square's interval corners computed once
 // per stage, as the reference caches them per square (ensure_sq_iv,
@@ -915,7 +942,6 @@ static int upload_consts(int device) {
     c.half_pi9 = fx::parse<9>(kHalfPi, hp, 0);
     c.two_pi9 = fx::parse<9>(kTwoPi, tp, 0);
     c.half9 = fx::parse<9>("0.5", h, 0);
-    c.half3 = fx::parse<3>("0.5", h, 0);
     c.half_pi7 = fx::parse_iv<7>(kHalfPi, hp);
     c.half7 = fx::parse_iv<7>("0.5", h);
     c.half_pi15 = fx::parse_iv<15>(kHalfPi, hp);
@@ -989,13 +1015,16 @@ static void put(char* dst, size_t cap, const std::string& s) {
     dst[k] = 0;
 }
 
+// FSq, AABB, sort key, PairSq and sort index of NMAX squares.
+constexpr size_t packing_smem(int nmax) { return (size_t)nmax * (sizeof(FSq) + 7 * sizeof(double) + 4 + 3 * 2 + 1); }
+
 template <int T, int NMAX>
 static int launch_packing(sqs_ctx* ctx, int count, const int32_t* bucket, const int32_t* pk_n,
                           const int64_t* pk_sq0, const char* text, const int64_t* raw_off,
                           const int32_t* raw_len, Lit* lits, PkOut* out, Pair* pairs, uint32_t* pair_count,
                           uint32_t cap) {
     if (count == 0) return SQS_OK;
-    const size_t smem = (size_t)NMAX * (sizeof(FSq) + 5 * sizeof(double) + sizeof(int16_t));
+    const size_t smem = packing_smem(NMAX);
     static std::atomic<bool> attr[64];  // set-up once per device (idempotent if repeated)
     if (!attr[ctx->device & 63]) {
         SQS_CUDA(cudaFuncSetAttribute(cert_packing_kernel<T, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1015,17 +1044,6 @@ static int launch_stage(sqs_ctx* ctx, const Pair* in, const uint32_t* in_count, 
                         const char* text, PkOut* out, int blocks) {
     cert_stage_kernel<F><<<blocks, 128, 0, ctx->stream>>>(in, in_count, in_cap, next, next_count, next_cap,
                                                          pk_sq0, lits, text, out);
-    SQS_CUDA(cudaGetLastError());
-    ctx->launches += 1;
-    return SQS_OK;
-}
-
-// The FP64 prefilter over a pair list (grid-stride; the count stays on the device).
-static int launch_fp64(sqs_ctx* ctx, const Pair* in, const uint32_t* in_count, uint32_t in_cap, Pair* next,
-                       uint32_t* next_count, uint32_t next_cap, const int64_t* pk_sq0, const Lit* lits,
-                       const char* text, PkOut* out, int blocks) {
-    cert_fp64_kernel<<<blocks, 128, 0, ctx->stream>>>(in, in_count, in_cap, next, next_count, next_cap, pk_sq0, lits,
-                                                       text, out);
     SQS_CUDA(cudaGetLastError());
     ctx->launches += 1;
     return SQS_OK;
@@ -1273,21 +1291,27 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
                                           d_text, d_off, d_len, d_lits, d_out, pa, cnt, cap)) return r;
     int32_t* slot_of = (int32_t*)(D + g_slot.off);
     SqRef* list = (SqRef*)(D + g_list.off);
-    // FP64 prefilter pa -> pb, then the 7-, 15- and 58-limb stages pb -> pa -> pb
-    if (int r = launch_fp64(ctx, pa, cnt, cap, pb, cnt + 5, cap, d_s0, d_lits, d_text, d_out, ctx->sm_count * 8))
-        return r;
-    if (int r = cached_stage<7>(ctx, pb, cnt + 5, cap, pa, cnt + 1, d_s0, d_lits, d_text, d_out, slot_of, list, cnt + 3,
-                                S))
-        return r;
-    if (int r = cached_stage<15>(ctx, pa, cnt + 1, cap, pb, cnt + 2, d_s0, d_lits, d_text, d_out, slot_of, list,
-                                 cnt + 3, S))
-        return r;
-    if (int r = cached_stage<58>(ctx, pb, cnt + 2, cap, nullptr, nullptr, d_s0, d_lits, d_text, d_out, slot_of, list,
-                                 cnt + 3, S))
-        return r;
+    // the records and the number of open pairs; most batches have none left
     std::vector<PkOut> h((size_t)count);
-    SQS_CUDA(cudaMemcpyAsync(h.data(), d_out, (size_t)count * sizeof(PkOut), cudaMemcpyDeviceToHost, ctx->stream));
-    SQS_CUDA(cudaStreamSynchronize(ctx->stream));
+    uint32_t open = 0;
+    auto read_back = [&](uint32_t* c) -> int {
+        SQS_CUDA(cudaMemcpyAsync(h.data(), d_out, (size_t)count * sizeof(PkOut), cudaMemcpyDeviceToHost, ctx->stream));
+        if (c) SQS_CUDA(cudaMemcpyAsync(&open, c, 4, cudaMemcpyDeviceToHost, ctx->stream));
+        SQS_CUDA(cudaStreamSynchronize(ctx->stream));
+        return SQS_OK;
+    };
+    if (int r = read_back(cnt)) return r;
+    if (open) {  // the 7-, 15- and 58-limb stages pa -> pb -> pa
+        if (int r = cached_stage<7>(ctx, pa, cnt, cap, pb, cnt + 1, d_s0, d_lits, d_text, d_out, slot_of, list, cnt + 3, S))
+            return r;
+        if (int r = cached_stage<15>(ctx, pb, cnt + 1, cap, pa, cnt + 2, d_s0, d_lits, d_text, d_out, slot_of, list,
+                                     cnt + 3, S))
+            return r;
+        if (int r = cached_stage<58>(ctx, pa, cnt + 2, cap, nullptr, nullptr, d_s0, d_lits, d_text, d_out, slot_of,
+                                     list, cnt + 3, S))
+            return r;
+        if (int r = read_back(nullptr)) return r;
+    }
     for (int p = 0; p < count; ++p) {
         if (!live[(size_t)p]) continue;
         sqs_verdict& v = out[p];
@@ -1395,7 +1419,7 @@ static PkOut s_out[kStaticMaxPackings];
 // place, so later calls allocate nothing.
 template <int T, int NMAX>
 static int packing_attr() {
-    const size_t smem = (size_t)NMAX * (sizeof(FSq) + 5 * sizeof(double) + sizeof(int16_t));
+    const size_t smem = packing_smem(NMAX);
     SQS_CUDA(cudaFuncSetAttribute(cert_packing_kernel<T, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return SQS_OK;
 }
@@ -1418,7 +1442,6 @@ static int static_setup(sqs_ctx* ctx) {
     const int64_t* d_s0 = (const int64_t*)(D + kSoS0);
     const Lit* d_lits = (const Lit*)(D + kSoLits);
     PkOut* d_out = (PkOut*)(D + kSoOut);
-    if (int r = launch_fp64(ctx, pa, cnt, 0, nullptr, nullptr, 0, d_s0, d_lits, D, d_out, 1)) return r;
     if (int r = launch_stage<7>(ctx, pa, cnt, 0, nullptr, nullptr, 0, d_s0, d_lits, D, d_out, 1)) return r;
     if (int r = launch_stage<15>(ctx, pa, cnt, 0, nullptr, nullptr, 0, d_s0, d_lits, D, d_out, 1)) return r;
     if (int r = launch_stage<58>(ctx, pa, cnt, 0, nullptr, nullptr, 0, d_s0, d_lits, D, d_out, 1)) return r;
@@ -1563,11 +1586,10 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
                                           d_out, pa, cnt, cap))
         return r;
     const int blocks = ctx->sm_count * 8;
-    if (int r = launch_fp64(ctx, pa, cnt, cap, pb, cnt + 5, cap, d_s0, d_lits, d_text, d_out, blocks)) return r;
-    if (int r = launch_stage<7>(ctx, pb, cnt + 5, cap, pa, cnt + 1, cap, d_s0, d_lits, d_text, d_out, blocks)) return r;
-    if (int r = launch_stage<15>(ctx, pa, cnt + 1, cap, pb, cnt + 2, cap, d_s0, d_lits, d_text, d_out, blocks))
+    if (int r = launch_stage<7>(ctx, pa, cnt, cap, pb, cnt + 1, cap, d_s0, d_lits, d_text, d_out, blocks)) return r;
+    if (int r = launch_stage<15>(ctx, pb, cnt + 1, cap, pa, cnt + 2, cap, d_s0, d_lits, d_text, d_out, blocks))
         return r;
-    if (int r = launch_stage<58>(ctx, pb, cnt + 2, cap, nullptr, nullptr, 0, d_s0, d_lits, d_text, d_out, blocks))
+    if (int r = launch_stage<58>(ctx, pa, cnt + 2, cap, nullptr, nullptr, 0, d_s0, d_lits, d_text, d_out, blocks))
         return r;
     SQS_CUDA(cudaMemcpyAsync(s_out, d_out, sizeof(PkOut) * (size_t)count, cudaMemcpyDeviceToHost, st));
     SQS_CUDA(cudaStreamSynchronize(st));

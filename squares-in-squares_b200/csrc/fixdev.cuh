@@ -371,6 +371,10 @@ FX_HEAVY Fix<F> parse(const char* text, const Lit& L, int rnd) {
     for (int l = 1; l <= F; ++l) {
         uint32_t v = 0;
         const long long base = (long long)L.point + (long long)(l - 1) * 9;
+        if (base >= L.ndig) {  // past the literal's digits
+            r.d[l] = 0;
+            continue;
+        }
         for (int k = 0; k < 9; ++k) v = v * 10u + (uint32_t)lit_digit(text, L, base + k);
         r.d[l] = v;
     }
@@ -425,14 +429,35 @@ FX_HD double round_half_away(double v) {
 #endif
 }
 
-// Point sin/cos (the side measurement): quadrant q from the double estimate.
+// One series of taylor() by itself (the same terms and roundings).
 template <int F>
-FX_HEAVY void sincos_point(const Fix<F>& a, const Fix<F>& half_pi, Fix<F>& sn, Fix<F>& cs) {
+FX_HEAVY Fix<F> taylor_one(const Fix<F>& x, int terms, int sine) {
+    const Fix<F> x2 = mul(x, x, 0);
+    Fix<F> t = sine ? x : of_int<F>(1);
+    Fix<F> sum = t;
+    for (int m = 1; m <= terms; ++m) {
+        t = div_small(mul(t, x2, 0), (uint32_t)((2 * m) * (sine ? 2 * m + 1 : 2 * m - 1)));
+        t.neg = (uint32_t)(m & 1) ^ (sine ? x.neg : 0u);
+        fix_zero(t);
+        sum = add(sum, t);
+        if (is_zero(t)) break;
+    }
+    return sum;
+}
+
+// Point sin/cos (the side measurement): quadrant q from the double estimate,
+// the cos (which = 0) or sin (1) series of the reduced angle, and the two
+// put together.
+template <int F>
+FX_HEAVY void sincos_series(const Fix<F>& a, const Fix<F>& half_pi, int which, Fix<F>& out, int& quad) {
     const long long q = (long long)round_half_away(approx(a) / 1.57079632679489661923);
     const Fix<F> r = sub(a, mul(of_int<F>(q), half_pi, 0));
-    Fix<F> s0, c0;
-    taylor(r, s0, c0, F <= 10 ? 32 : 115);
-    switch ((int)((q % 4 + 4) % 4)) {
+    out = taylor_one(r, F <= 10 ? 32 : 115, which);
+    quad = (int)((q % 4 + 4) % 4);
+}
+template <int F>
+FX_HD void sincos_quadrant(const Fix<F>& s0, const Fix<F>& c0, int quad, Fix<F>& sn, Fix<F>& cs) {
+    switch (quad) {
         case 0: sn = s0; cs = c0; break;
         case 1: sn = c0; cs = neg(s0); break;
         case 2: sn = neg(s0); cs = neg(c0); break;

@@ -170,3 +170,44 @@ def test_full_seed42_corpus_equals_reference(ctx, oracle):
     assert not bad, (len(bad), bad[:3])
     assert 0 < ok.sum() < len(items)
     assert max(n for n, _ in items) > 900
+
+
+@pytest.mark.parametrize("kind", ["gap", "turns", "far", "flat_shift", "flat_nudge", "mixed", "random"])
+def test_pair_decision_matches_oracle(ctx, oracle, kind):
+    """The FP64 pair decision at its edges -- gaps and overlaps down to 1e-17,
+    angles outside [0, 2 pi), coordinates near the bound, touching edges with
+    exact, dyadic and rounded offsets, mixed flat and tilted squares -- against
+    the oracle certifier: every verdict, reason, score and side."""
+    import numpy as np
+
+    from sqs import core
+    from sqs.workloads import grid_rows, rows_of, tilted_lattice
+
+    rng = np.random.default_rng(11)
+    items = []
+    for k in range(60):
+        n = int(rng.choice([2, 3, 31, 64, 65, 90]))
+        q = tilted_lattice(n, 10 ** rng.uniform(-16, -7), float(rng.uniform(0.05, 1.5)))
+        flat = np.array([[float(r["x"]), float(r["y"]), 0.0] for r in grid_rows(n)])
+        i = int(rng.integers(n))
+        if kind == "turns":
+            q[:, 2] -= int(rng.integers(-15, 15)) * 2 * np.pi
+        elif kind == "far":
+            q[:, :2] += rng.uniform(-9000, 9000)
+        elif kind == "flat_shift":
+            q = flat + [[rng.choice([0.125, 0.3, 2.0 ** -20, 2.0 ** -30]), rng.choice([0.5, 1e-3]), 0.0]]
+        elif kind == "flat_nudge":
+            q = flat
+            q[i, int(rng.integers(2))] += rng.choice([-1, 1]) * 10 ** rng.uniform(-17, -5)
+        elif kind == "mixed":
+            q = flat * [[1.0000001, 1.0000001, 1.0]]
+            q[:, 2] = rng.choice([0.0, 1e-300, 1e-8, 3e-8, np.pi / 2], n)
+        elif kind == "random":
+            q = rng.uniform(0, 1.6 * np.sqrt(n), (n, 3))
+        items.append((n, rows_of(q, str(rng.choice([".17g", ".25f", ".20e", ".9f"])))))
+    arrs = core.pack_batch(items)
+    out = core.certify_arrays(*arrs, ctx=ctx)
+    ok, score, sides, reasons = oracle.certify_batch_text(*arrs, which="oracle")
+    for p in range(len(items)):
+        assert (int(out[p].ok), float(out[p].score), out[p].L.decode(), out[p].reason.decode()) == \
+            (int(ok[p]), float(score[p]), sides[p], reasons[p])
