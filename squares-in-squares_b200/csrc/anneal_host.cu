@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <charconv>
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -510,8 +511,8 @@ int certify_states(sqs_ctx* ctx, const std::vector<int>& ns, const std::vector<c
             for (int i = 0; i < n; ++i) {
                 const double v[3] = {b[3 * i] * ladder[step], b[3 * i + 1] * ladder[step], b[3 * i + 2]};
                 for (double x : v) {
-                    std::snprintf(buf, sizeof buf, "%.17g", x);
-                    text += buf;
+                    // printf's %.17g, several times faster
+                    text.append(buf, std::to_chars(buf, buf + sizeof buf, x, std::chars_format::general, 17).ptr);
                     lit_off.push_back((int64_t)text.size());
                 }
             }

@@ -23,6 +23,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <charconv>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -62,6 +63,12 @@ struct Pair {
     int32_t pk;
     int16_t u, v;
 };
+
+// A square's literals x, y, angle: back to back from text offset `off`.
+struct SqText {
+    uint32_t off, len[3];
+};
+constexpr uint32_t kLenMax = 1u << 20;  // a longer literal is read as far as this
 
 struct Consts {
     Fix<9> half_pi9, two_pi9, half9;
@@ -375,8 +382,8 @@ __device__ void fix_shfl_min_max(Fix<F>& v, bool& have, bool want_min) {
 template <int T, int NMAX>
 __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
     int count, const int32_t* __restrict__ bucket, const int32_t* __restrict__ pk_n,
-    const int64_t* __restrict__ pk_sq0, const char* __restrict__ text, const int64_t* __restrict__ raw_off,
-    const int32_t* __restrict__ raw_len, Lit* __restrict__ lits, PkOut* __restrict__ out,
+    const int64_t* __restrict__ pk_sq0, const char* __restrict__ text, const SqText* __restrict__ raw,
+    Lit* __restrict__ lits, PkOut* __restrict__ out,
     Pair* __restrict__ pairs, uint32_t* __restrict__ pair_count, uint32_t pair_cap) {
     constexpr int W = T / 32;
     constexpr int NP = NMAX;  // power of two
@@ -423,9 +430,10 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
     for (int i = tid; i < n; i += T) {
         uint32_t kind = kNoKey;
         Lit Ls[3];
-        for (int k = 0; k < 3; ++k) {
-            const int64_t r = 3 * (s0 + i) + k;
-            const bool ok = analyze(text + raw_off[r], raw_len[r], (uint32_t)raw_off[r], Ls[k]);
+        const SqText st = raw[s0 + i];
+        uint32_t off = st.off;
+        for (int k = 0; k < 3; off += st.len[k], ++k) {
+            const bool ok = analyze(text + off, (int)min(st.len[k], kLenMax), off, Ls[k]);
             if (!ok && kind == kNoKey) kind = kErrParse;
         }
         if (kind == kNoKey) {
@@ -969,16 +977,19 @@ static void fifty_into(const Fix<9>& v, char* dst, size_t cap) {
     }
     bool allz = true;
     for (uint64_t w : o) allz &= w == 0;
-    std::snprintf(dst, cap, "%s%llu.%09llu%09llu%09llu%09llu%09llu%05llu", (v.neg && !allz) ? "-" : "",
-                  (unsigned long long)o[0], (unsigned long long)o[1], (unsigned long long)o[2],
-                  (unsigned long long)o[3], (unsigned long long)o[4], (unsigned long long)o[5],
-                  (unsigned long long)o[6]);
-}
-
-static std::string fifty(const Fix<9>& v) {
-    char buf[128];
-    fifty_into(v, buf, sizeof buf);
-    return buf;
+    char buf[96];
+    char* c = buf;
+    if (v.neg && !allz) *c++ = '-';
+    c = std::to_chars(c, c + 20, o[0]).ptr;
+    *c++ = '.';
+    for (int i = 1; i <= 6; ++i) {  // 9 digits a limb, the last 5
+        const int nd = i == 6 ? 5 : 9;
+        uint64_t w = o[i];
+        for (int k = nd - 1; k >= 0; --k, w /= 10) c[k] = (char)('0' + w % 10);
+        c += nd;
+    }
+    *c = 0;
+    std::snprintf(dst, cap, "%s", buf);
 }
 
 static double grid_score(int n) { return std::ceil(std::sqrt((double)n)) / std::sqrt((double)n) - 1.0; }
@@ -988,8 +999,16 @@ static double grid_score(int n) { return std::ceil(std::sqrt((double)n)) / std::
 // as v, with ".0" appended to a plain integer; returns its length (< 40).
 static size_t roundtrip_into(double v, char out[40]) {
     for (int p = 15; p <= 17; ++p) {
-        std::snprintf(out, 40, "%.*g", p, v);
-        if (std::strtod(out, nullptr) == v) break;
+        if (std::isfinite(v)) {  // to_chars and from_chars are printf and strtod in the C locale, several times faster
+            char* e = std::to_chars(out, out + 39, v, std::chars_format::general, p).ptr;
+            *e = 0;
+            double back = 0.0;
+            std::from_chars(out, e, back);
+            if (back == v) break;
+        } else {
+            std::snprintf(out, 40, "%.*g", p, v);
+            if (std::strtod(out, nullptr) == v) break;
+        }
     }
     size_t len = std::strlen(out);
     if (std::strpbrk(out, ".eE") == nullptr) {
@@ -1017,8 +1036,7 @@ constexpr size_t packing_smem(int nmax) { return (size_t)nmax * (sizeof(FSq) + 7
 
 template <int T, int NMAX>
 static int launch_packing(sqs_ctx* ctx, cudaStream_t st, int count, const int32_t* bucket, const int32_t* pk_n,
-                          const int64_t* pk_sq0, const char* text, const int64_t* raw_off,
-                          const int32_t* raw_len, Lit* lits, PkOut* out, Pair* pairs, uint32_t* pair_count,
+                          const int64_t* pk_sq0, const char* text, const SqText* raw, Lit* lits, PkOut* out, Pair* pairs, uint32_t* pair_count,
                           uint32_t cap) {
     if (count == 0) return SQS_OK;
     const size_t smem = packing_smem(NMAX);
@@ -1028,8 +1046,8 @@ static int launch_packing(sqs_ctx* ctx, cudaStream_t st, int count, const int32_
                                       (int)smem));
         attr[ctx->device & 63] = true;
     }
-    cert_packing_kernel<T, NMAX><<<count, T, smem, st>>>(count, bucket, pk_n, pk_sq0, text, raw_off,
-                                                               raw_len, lits, out, pairs, pair_count, cap);
+    cert_packing_kernel<T, NMAX><<<count, T, smem, st>>>(count, bucket, pk_n, pk_sq0, text, raw, lits, out, pairs,
+                                                          pair_count, cap);
     SQS_CUDA(cudaGetLastError());
     ctx->launches += 1;
     return SQS_OK;
@@ -1041,8 +1059,7 @@ static int launch_packing(sqs_ctx* ctx, cudaStream_t st, int count, const int32_
 // 1.2 ms side by side).
 static int launch_buckets(sqs_ctx* ctx, int c0, int c1, int c2, const int32_t* b0, const int32_t* b1,
                           const int32_t* b2, const int32_t* pk_n, const int64_t* pk_sq0, const char* text,
-                          const int64_t* raw_off, const int32_t* raw_len, Lit* lits, PkOut* out, Pair* pairs,
-                          uint32_t* pair_count, uint32_t cap) {
+                          const SqText* raw, Lit* lits, PkOut* out, Pair* pairs, uint32_t* pair_count, uint32_t cap) {
     const int classes = (c0 > 0) + (c1 > 0) + (c2 > 0);
     cudaStream_t s0 = ctx->stream, s1 = ctx->stream;
     if (classes > 1) {
@@ -1051,14 +1068,12 @@ static int launch_buckets(sqs_ctx* ctx, int c0, int c1, int c2, const int32_t* b
         s1 = ctx->aux[1];
         for (int a = 0; a < 2; ++a) SQS_CUDA(cudaStreamWaitEvent(ctx->aux[a], ctx->fork, 0));
     }
-    int rc = launch_packing<256, 1024>(ctx, ctx->stream, c2, b2, pk_n, pk_sq0, text, raw_off, raw_len, lits, out, pairs,
+    int rc = launch_packing<256, 1024>(ctx, ctx->stream, c2, b2, pk_n, pk_sq0, text, raw, lits, out, pairs,
                                        pair_count, cap);
     if (!rc)
-        rc = launch_packing<128, 256>(ctx, s1, c1, b1, pk_n, pk_sq0, text, raw_off, raw_len, lits, out, pairs, pair_count,
-                                      cap);
+        rc = launch_packing<128, 256>(ctx, s1, c1, b1, pk_n, pk_sq0, text, raw, lits, out, pairs, pair_count, cap);
     if (!rc)
-        rc = launch_packing<64, 64>(ctx, s0, c0, b0, pk_n, pk_sq0, text, raw_off, raw_len, lits, out, pairs, pair_count,
-                                    cap);
+        rc = launch_packing<64, 64>(ctx, s0, c0, b0, pk_n, pk_sq0, text, raw, lits, out, pairs, pair_count, cap);
     if (classes > 1) {  // join the side streams, also after a failed launch
         for (int a = 0; a < 2; ++a) {
             SQS_CUDA(cudaEventRecord(ctx->join[a], ctx->aux[a]));
@@ -1172,10 +1187,9 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
     // staging: no zero fill, no page faults after the first call, and an
     // upload at the full host-link rate.  Every slot of a live packing is
     // written below; slots of packings found invalid are never read.
-    const size_t n3 = (size_t)(3 * S);
-    if (int r = ctx->h_cert.reserve(n3 * (sizeof(int64_t) + sizeof(int32_t)) + 16)) return r;
-    int64_t* const raw_off = (int64_t*)ctx->h_cert.p;
-    int32_t* const raw_len = (int32_t*)(raw_off + n3);
+    // One 16-byte record a square (its three literals lie back to back).
+    if (int r = ctx->h_cert.reserve((size_t)S * sizeof(SqText) + 16)) return r;
+    SqText* const raw = (SqText*)ctx->h_cert.p;
     const int nt = count >= 64 ? (int)std::max(1u, std::min(16u, std::thread::hardware_concurrency())) : 1;
     std::vector<int> p_lo((size_t)nt + 1, count);
     {
@@ -1222,21 +1236,20 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
             }
             for (int i = 0; i < n; ++i) {
                 const int64_t r = row_of[(size_t)i];
+                SqText& q = raw[pk_sq0[(size_t)p] + i];
+                q.off = (uint32_t)(do_rt ? (int64_t)rt[(size_t)t].size() : lit_off[3 * r]);
                 for (int k = 0; k < 3; ++k) {
                     const int64_t a = lit_off[3 * r + k], b = lit_off[3 * r + k + 1];
                     if (b < a) {
                         bad_row[(size_t)t] = r;
                         return;
                     }
-                    const size_t q = (size_t)(3 * (pk_sq0[(size_t)p] + i) + k);
                     if (do_rt) {
                         const std::string s2 = roundtrip(text + a, (size_t)(b - a));
-                        raw_off[q] = (int64_t)rt[(size_t)t].size();
-                        raw_len[q] = (int32_t)s2.size();
+                        q.len[k] = (uint32_t)s2.size();
                         rt[(size_t)t] += s2;
                     } else {
-                        raw_off[q] = a;
-                        raw_len[q] = (int32_t)std::min<int64_t>(b - a, 1 << 20);
+                        q.len[k] = (uint32_t)(b - a);
                     }
                 }
             }
@@ -1258,8 +1271,8 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
             if (base)
                 for (int p = p_lo[(size_t)t]; p < p_lo[(size_t)t + 1]; ++p) {
                     if (!live[(size_t)p]) continue;
-                    for (int64_t q = 3 * pk_sq0[(size_t)p]; q < 3 * (pk_sq0[(size_t)p] + pk_n[(size_t)p]); ++q)
-                        raw_off[(size_t)q] += (int64_t)base;
+                    for (int64_t q = pk_sq0[(size_t)p]; q < pk_sq0[(size_t)p] + pk_n[(size_t)p]; ++q)
+                        raw[q].off += (uint32_t)base;
                 }
             base += rt[(size_t)t].size();
         }
@@ -1281,7 +1294,7 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
     struct Seg { size_t off, bytes; };
     size_t tot = 0;
     auto seg = [&](size_t bytes) { Seg s{tot, bytes}; tot += (bytes + 255) & ~(size_t)255; return s; };
-    const Seg g_text = seg(blob_bytes), g_off = seg(n3 * 8 + 8), g_len = seg(n3 * 4 + 4);
+    const Seg g_text = seg(blob_bytes), g_raw = seg((size_t)S * sizeof(SqText) + 16);
     const Seg g_n = seg((size_t)count * 4), g_s0 = seg((size_t)count * 8);
     const Seg g_b0 = seg(bk[0].size() * 4 + 4), g_b1 = seg(bk[1].size() * 4 + 4), g_b2 = seg(bk[2].size() * 4 + 4);
     const Seg g_lits = seg((size_t)(3 * S + 3) * sizeof(Lit)), g_out = seg((size_t)count * sizeof(PkOut));
@@ -1294,8 +1307,7 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
         return SQS_OK;
     };
     if (int r = up(g_text, blob, do_rt ? rt_text.size() : (size_t)lit_off[3 * row_start[count]])) return r;
-    if (int r = up(g_off, raw_off, n3 * 8)) return r;
-    if (int r = up(g_len, raw_len, n3 * 4)) return r;
+    if (int r = up(g_raw, raw, (size_t)S * sizeof(SqText))) return r;
     if (int r = up(g_n, pk_n.data(), (size_t)count * 4)) return r;
     if (int r = up(g_s0, pk_sq0.data(), (size_t)count * 8)) return r;
     if (int r = up(g_b0, bk[0].data(), bk[0].size() * 4)) return r;
@@ -1308,15 +1320,13 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
     Pair* pb = (Pair*)(D + g_pb.off);
     uint32_t* cnt = (uint32_t*)(D + g_cnt.off);
     const char* d_text = D + g_text.off;
-    const int64_t* d_off = (const int64_t*)(D + g_off.off);
-    const int32_t* d_len = (const int32_t*)(D + g_len.off);
+    const SqText* d_raw = (const SqText*)(D + g_raw.off);
     const int32_t* d_n = (const int32_t*)(D + g_n.off);
     const int64_t* d_s0 = (const int64_t*)(D + g_s0.off);
     Lit* d_lits = (Lit*)(D + g_lits.off);
     if (int r = launch_buckets(ctx, (int)bk[0].size(), (int)bk[1].size(), (int)bk[2].size(),
                                (const int32_t*)(D + g_b0.off), (const int32_t*)(D + g_b1.off),
-                               (const int32_t*)(D + g_b2.off), d_n, d_s0, d_text, d_off, d_len, d_lits, d_out, pa, cnt,
-                               cap))
+                               (const int32_t*)(D + g_b2.off), d_n, d_s0, d_text, d_raw, d_lits, d_out, pa, cnt, cap))
         return r;
     int32_t* slot_of = (int32_t*)(D + g_slot.off);
     SqRef* list = (SqRef*)(D + g_list.off);
@@ -1346,7 +1356,6 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
         sqs_verdict& v = out[p];
         const PkOut& o = h[(size_t)p];
         const int n = pk_n[(size_t)p];
-        const std::string N = std::to_string(n);
         if (o.flags & kPairOverflow) {
             set_error("packing %d: undecided-pair list overflowed", p);
             return SQS_ENOMEM;
@@ -1355,7 +1364,7 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
             static const char* what[4] = {"cannot parse coordinates", "value out of range for a double",
                                           "coordinate out of bounds", "angle out of bounds"};
             put(v.reason, sizeof v.reason,
-                "n=" + N + ", square " + std::to_string(o.err_key / 4) + ": " + what[o.err_key % 4]);
+                "n=" + std::to_string(n) + ", square " + std::to_string(o.err_key / 4) + ": " + what[o.err_key % 4]);
             continue;
         }
         if (o.fkey != kNoPair) {
@@ -1379,7 +1388,7 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
         }
         v.ok = 1;
         put(v.reason, sizeof v.reason, "ok");
-        put(v.L, sizeof v.L, fifty(o.side));
+        fifty_into(o.side, v.L, sizeof v.L);
         v.score = std::max(0.0, sf / lb - 1.0);
     }
     return SQS_OK;
@@ -1403,8 +1412,7 @@ constexpr uint32_t kStaticPairCap = 16u * kStaticMaxSquares + 4096u;
 constexpr size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 constexpr size_t kSoText = 0;
 constexpr size_t kSoOff = kSoText + al256(kStaticMaxText);
-constexpr size_t kSoLen = kSoOff + al256(sizeof(int64_t) * 3 * kStaticMaxSquares);
-constexpr size_t kSoN = kSoLen + al256(sizeof(int32_t) * 3 * kStaticMaxSquares);
+constexpr size_t kSoN = kSoOff + al256(sizeof(SqText) * kStaticMaxSquares);
 constexpr size_t kSoS0 = kSoN + al256(sizeof(int32_t) * kStaticMaxPackings);
 constexpr size_t kSoBk = kSoS0 + al256(sizeof(int64_t) * kStaticMaxPackings);
 constexpr size_t kSoLits = kSoBk + al256(sizeof(int32_t) * kStaticMaxPackings);
@@ -1428,8 +1436,7 @@ static std::atomic_flag s_busy = ATOMIC_FLAG_INIT;
 
 // Host staging (static, not heap): literal slices in square-id order, packing
 // tables, round-tripped literals, the per-packing records read back.
-static int64_t s_raw_off[3 * kStaticMaxSquares];
-static int32_t s_raw_len[3 * kStaticMaxSquares];
+static SqText s_raw[kStaticMaxSquares];
 static int32_t s_pk_n[kStaticMaxPackings];
 static int64_t s_pk_sq0[kStaticMaxPackings];
 static int32_t s_bucket[kStaticMaxPackings];
@@ -1546,10 +1553,11 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
         s_pk_sq0[p] = S;
         for (int i = 0; i < n; ++i) {
             const int64_t r = s_row_of[i];
+            SqText& q = s_raw[S + i];
+            q.off = (uint32_t)(do_rt ? (int64_t)rt_used : lit_off[3 * r]);
             for (int k = 0; k < 3; ++k) {
                 const int64_t a = lit_off[3 * r + k], b = lit_off[3 * r + k + 1];
                 SQS_REQUIRE(b >= a, "literal offsets not monotone at row %lld", (long long)r);
-                const int64_t q = 3 * (S + i) + k;
                 if (do_rt) {
                     SQS_REQUIRE((size_t)(b - a) < sizeof(s_lit_tmp), "literal longer than %zu bytes",
                                 sizeof(s_lit_tmp) - 1);
@@ -1559,12 +1567,10 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
                     const size_t len = roundtrip_into(std::strtod(s_lit_tmp, nullptr), buf);
                     SQS_REQUIRE(rt_used + len <= kStaticMaxText, "literals exceed %zu bytes", kStaticMaxText);
                     std::memcpy(s_rt_text + rt_used, buf, len);
-                    s_raw_off[q] = (int64_t)rt_used;
-                    s_raw_len[q] = (int32_t)len;
+                    q.len[k] = (uint32_t)len;
                     rt_used += len;
                 } else {
-                    s_raw_off[q] = a;
-                    s_raw_len[q] = (int32_t)std::min<int64_t>(b - a, 1 << 20);
+                    q.len[k] = (uint32_t)(b - a);
                 }
             }
         }
@@ -1585,8 +1591,7 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
     cudaStream_t st = ctx->stream;
     if (text_bytes)
         SQS_CUDA(cudaMemcpyAsync(D + kSoText, do_rt ? s_rt_text : text, text_bytes, cudaMemcpyHostToDevice, st));
-    SQS_CUDA(cudaMemcpyAsync(D + kSoOff, s_raw_off, sizeof(int64_t) * 3 * (size_t)S, cudaMemcpyHostToDevice, st));
-    SQS_CUDA(cudaMemcpyAsync(D + kSoLen, s_raw_len, sizeof(int32_t) * 3 * (size_t)S, cudaMemcpyHostToDevice, st));
+    SQS_CUDA(cudaMemcpyAsync(D + kSoOff, s_raw, sizeof(SqText) * (size_t)S, cudaMemcpyHostToDevice, st));
     SQS_CUDA(cudaMemcpyAsync(D + kSoN, s_pk_n, sizeof(int32_t) * (size_t)count, cudaMemcpyHostToDevice, st));
     SQS_CUDA(cudaMemcpyAsync(D + kSoS0, s_pk_sq0, sizeof(int64_t) * (size_t)count, cudaMemcpyHostToDevice, st));
     SQS_CUDA(cudaMemcpyAsync(D + kSoBk, s_bucket, sizeof(int32_t) * (size_t)(nb[0] + nb[1] + nb[2]),
@@ -1595,8 +1600,7 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
     SQS_CUDA(cudaMemsetAsync(D + kSoOut, 0, sizeof(PkOut) * (size_t)count, st));
     SQS_CUDA(cudaMemsetAsync(D + kSoCnt, 0, 64, st));
     const char* d_text = D + kSoText;
-    const int64_t* d_off = (const int64_t*)(D + kSoOff);
-    const int32_t* d_len = (const int32_t*)(D + kSoLen);
+    const SqText* d_raw = (const SqText*)(D + kSoOff);
     const int32_t* d_n = (const int32_t*)(D + kSoN);
     const int64_t* d_s0 = (const int64_t*)(D + kSoS0);
     const int32_t* d_bk = (const int32_t*)(D + kSoBk);
@@ -1607,7 +1611,7 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
     uint32_t* cnt = (uint32_t*)(D + kSoCnt);
     const uint32_t cap = kStaticPairCap;
     if (int r = launch_buckets(ctx, nb[0], nb[1], nb[2], d_bk, d_bk + nb[0], d_bk + nb[0] + nb[1], d_n, d_s0, d_text,
-                               d_off, d_len, d_lits, d_out, pa, cnt, cap))
+                               d_raw, d_lits, d_out, pa, cnt, cap))
         return r;
     const int blocks = ctx->sm_count * 8;
     if (int r = launch_stage<7>(ctx, pa, cnt, cap, pb, cnt + 1, cap, d_s0, d_lits, d_text, d_out, blocks)) return r;
