@@ -1,21 +1,23 @@
 // FP32 cell-list SAT overlap + wall energy and gradient of many independent
-// configurations: one CTA per configuration.
+// configurations: one CTA, or for n <= 256 one warp, per configuration.
 //
-// Per CTA (all in shared memory):
-//   1. load the n squares (coalesced 12-byte records), cos/sin, wall term,
-//      cell id on a G x G grid of cells with side >= sqrt(2.000001) (so every
-//      interacting pair sits in the same or adjacent cells), per-cell counts;
-//   2. exclusive scan of the counts, counting-sort scatter, each cell's few
-//      entries ordered by square index (deterministic pair order);
+// Per configuration:
+//   1. load the n squares, cos/sin, wall term, cell on a G x G grid of cells
+//      with side >= sqrt(2.000001) (so every interacting pair sits in the same
+//      or adjacent cells), rank within the cell; a thread keeps its squares in
+//      registers until the scatter;
+//   2. exclusive scan of the cell counts, scatter to cell order;
 //   3. broad phase: every square scans two contiguous ranges of the
 //      cell-sorted array -- the rest of its own cell plus the east cell, and
 //      the three cells of the row above -- which visits each unordered
-//      neighbour pair exactly once.  Pairs inside the cut-off are appended
-//      to a per-warp queue (ballot + popc), and every time 32 are queued the
-//      whole warp evaluates them (narrow phase at full SIMT width), adding
-//      both squares' gradients with shared-memory atomics;
-//   4. warp-shuffle + shared reduction of the energy and candidate count,
-//      coalesced store of the gradient.
+//      neighbour pair exactly once, and keeps the hits of up to 32 candidates
+//      as bits.  The set bits (a third of the candidates) are then appended
+//      to a per-warp queue, one a lane a round, and every time 32 pairs are
+//      queued the warp evaluates them (narrow phase at full SIMT width),
+//      adding both squares' gradients with shared-memory integer atomics;
+//   4. exact integer reduction of the energy, store of the gradient.
+// Energies and gradients are integer sums, so results do not depend on the
+// order in which pairs are found and the cells need no sorting.
 // Reference: total_cached (seeded.cu:148-162) is the all-pairs O(n^2) form
 // of the same energy; the legacy FP32 path's 16x16 cell grid of width 2
 // (packing.cu:22-47) is the reference's own cell-list idea.
@@ -31,21 +33,43 @@ namespace sqs {
 
 constexpr int kSatMaxN = 1024;
 constexpr float kCellMin = 1.41422f;  // > sqrt(2.000001) = 1.4142139
-constexpr int kQueue = 64;            // per-warp pair queue entries
+constexpr int kQueue = 256, kCtaQueue = 128;  // pair queue entries of a warp: warp form, CTA form
+
+// Pair energies are summed as 64-bit integers in units of 2^-40: every term
+// is rounded once (error below 5e-13), the sum is exact, and 1024 squares'
+// pairs stay far below 2^23, so below 2^63 units.  The warp form sums its wall
+// terms the same way; the CTA form in double, in thread order.
+constexpr double kEUnit = 1099511627776.0;  // 2^40
+__device__ __forceinline__ long long e_units(float e) { return __float2ll_rn(e * 1099511627776.0f); }
+
+// Exact 64-bit warp sum: the 26 low bits, the next 26 and the signed rest
+// each sum within 32 bits.
+__device__ __forceinline__ long long warp_sum_units(long long v) {
+    const unsigned s0 = __reduce_add_sync(0xffffffffu, (unsigned)v & 0x3ffffffu);
+    const unsigned s1 = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 26) & 0x3ffffffu);
+    const int s2 = __reduce_add_sync(0xffffffffu, (int)(v >> 52));
+    return (long long)(((unsigned long long)(long long)s2 << 52) + ((unsigned long long)s1 << 26) + s0);
+}
+
+// Nearest integer (ties to even) of |x| < 2^22 on the FMA pipe: x + 1.5 * 2^23
+// lands in [2^23, 2^24), where one float ulp is 1, so its bit pattern minus
+// that of 1.5 * 2^23 is the rounded integer.
+constexpr float kMagic = 12582912.0f;
+__device__ __forceinline__ int magic_int(float shifted) { return __float_as_int(shifted) - 0x4B400000; }
 
 // Gradient accumulation with native 32-bit integer shared-memory atomics
 // (shared-memory float atomics are several times slower): a contribution v
-// is split into floor(v * 2^12) and the remaining fraction in units of 2^-32,
-// two integer sums that cannot overflow for n <= 1024 (|v| < 6 per pair) and
-// that do not depend on the order of the additions.
+// is split into round(v * 2^12) and the signed rest in units of 2^-32, two
+// integer sums that cannot overflow for n <= 1024 (|v| < 6 per pair) and that
+// do not depend on the order of the additions.
 struct GradFix {
-    int* hi;        // [3n]
-    unsigned* lo;   // [3n]
+    int* hi;  // [3n]
+    int* lo;  // [3n]
     __device__ __forceinline__ void add(int k, float v) const {
         const float s = v * 4096.0f;
-        const float f = floorf(s);
-        atomicAdd(hi + k, (int)f);
-        atomicAdd(lo + k, __float2uint_rn((s - f) * 1048576.0f));
+        const float h = s + kMagic;
+        atomicAdd(hi + k, magic_int(h));
+        atomicAdd(lo + k, magic_int(fmaf(s - (h - kMagic), 1048576.0f, kMagic)));
     }
     __device__ __forceinline__ float value(int k) const {
         return (float)(((double)hi[k] + (double)lo[k] * (1.0 / 1048576.0)) * (1.0 / 4096.0));
@@ -61,39 +85,91 @@ __host__ __device__ inline int sat_grid_cap(int n) {
 __host__ __device__ inline size_t sat_smem_bytes(int n, int threads) {
     const int G = sat_grid_cap(n);
     size_t b = 0;
-    b += (size_t)n * 16;                      // stash (x, y, c, s) by original index
     b += (size_t)n * 16;                      // cell-sorted (x, y) and (c, s)
-    b += (size_t)n * 12;                      // wall gradient by original index
     b += (size_t)n * 24;                      // pair gradient accumulators (GradFix)
+    b += (size_t)(threads / 32) * kCtaQueue * 4;  // warp pair queues
+    b += ((size_t)(G * G + 1) * 2 + 3) & ~(size_t)3;  // cell counts / starts
     b += (size_t)n * 4;                       // sorted -> (original index, cell)
-    b += (size_t)n * 4;                       // original -> (cell, rank)
-    b += (size_t)(G * G + 1) * 4;             // cell counts / starts
-    b += (size_t)(threads / 32) * kQueue * 4; // warp pair queues
-    b += 64;                                  // reduction scratch
+    b += 8 + (size_t)(threads / 32) * 24;     // reduction scratch
     return (b + 15) & ~(size_t)15;
 }
 
+// Broad phase of one warp's 32 squares p = base + lane over the cell-sorted
+// centres: the two candidate ranges of each, 32 candidates at a time as hit
+// bits; then every lane writes its hits at its place in the warp's queue (a
+// prefix sum of the hit counts), and `flush(entry)` takes 32 queued pairs at a
+// time off its end.  `qn`: queued pairs (below 32 on entry and exit).  Testing
+// a candidate costs about ten instructions.  At 4,096 x 200: 41.0 us, the same
+// as a ballot and a queue position for every candidate, and 43.0 with a ballot
+// per hit; at 1,500 x 999 with the queue's size below 88.6 us (90.1 with a
+// ballot per hit).
+template <bool COUNT, int CAP, class E, class Flush>
+__device__ __forceinline__ void broad_phase(const float2* sxy, int p, float px, float py, int a1, int len1, int a2,
+                                            int len, int lane, E* queue, int& qn, uint32_t& cand_loc, Flush&& flush) {
+    constexpr int kShift = sizeof(E) * 4;  // an entry is p | q << kShift
+    const int maxlen = __reduce_max_sync(0xffffffffu, len);
+    for (int t0 = 0; t0 < maxlen; t0 += 32) {
+        uint32_t hits = 0u;
+        const int end = min(maxlen - t0, 32);
+#pragma unroll 4
+        for (int k = 0; k < end; ++k) {
+            const int t = t0 + k;
+            if (t < len) {
+                const float2 Q = sxy[(t < len1 ? a1 : a2) + t];
+                const float dx = Q.x - px, dy = Q.y - py;
+                const float d2 = dx * dx + dy * dy;
+                hits |= d2 < kPairCut2 ? 1u << k : 0u;
+                if (COUNT) cand_loc += d2 < 2.0f;
+            }
+        }
+        int left;  // hits of the warp not queued yet
+        do {
+            const int mine = __popc(hits);
+            int incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            int at = qn + incl - mine;
+            while (hits && at < CAP) {
+                const int t = t0 + __ffs(hits) - 1;
+                hits &= hits - 1u;
+                queue[at++] = (E)((uint32_t)p | ((uint32_t)((t < len1 ? a1 : a2) + t) << kShift));
+            }
+            __syncwarp();
+            left = max(qn + total - CAP, 0);
+            for (qn = min(qn + total, CAP); qn >= 32; qn -= 32) flush((uint32_t)queue[qn - 32 + lane]);
+            __syncwarp();
+        } while (left > 0);
+    }
+}
+
+// One CTA per configuration.  n = 999 holds 54 KB of shared memory, so four
+// CTAs of 256 threads share an SM.  The form before kept an original-order copy
+// of the squares and the wall gradients there and summed energies in float,
+// for which every cell was sorted: 76 KB, eight warps an SM, 243 us at
+// 1,500 x 999 against 88.6 (queues of 64 or 256 pairs a warp: 96 us, the one
+// for its rounds, the other for a CTA less an SM; 512 threads: 97 us).
 template <int T>
-__global__ void __launch_bounds__(T) sat_energy_kernel(int n, const float* __restrict__ xya,
+__global__ void __launch_bounds__(T, T == 256 ? 4 : 1) sat_energy_kernel(int n, const float* __restrict__ xya,
                                                         const float* __restrict__ side,
                                                         float* __restrict__ energy,
                                                         float* __restrict__ grad,
                                                         uint32_t* __restrict__ cand) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int W = T / 32;
+    constexpr int W = T / 32, NPT = kSatMaxN / T;
     const int cfg = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Gcap = sat_grid_cap(n);
-    float4* stash = reinterpret_cast<float4*>(smem);
-    float2* sxy = reinterpret_cast<float2*>(stash + n);             // cell-sorted centres
+    float2* sxy = reinterpret_cast<float2*>(smem);                  // cell-sorted centres
     float2* scs = sxy + n;                                          // cell-sorted cos/sin
-    float* gacc = reinterpret_cast<float*>(scs + n);                // wall gradient
-    GradFix gf{reinterpret_cast<int*>(gacc + 3 * n), reinterpret_cast<unsigned*>(gacc + 6 * n)};
-    short2* sorted_meta = reinterpret_cast<short2*>(gacc + 9 * n);  // (orig, cell)
-    short2* orig_meta = sorted_meta + n;                            // (cell, rank)
-    int* cells = reinterpret_cast<int*>(orig_meta + n);             // G*G + 1
-    uint32_t* queues = reinterpret_cast<uint32_t*>(cells + Gcap * Gcap + 1);
-    float* red = reinterpret_cast<float*>(queues + W * kQueue);
+    const GradFix gf{reinterpret_cast<int*>(scs + n), reinterpret_cast<int*>(scs + n) + 3 * n};
+    uint32_t* queues = reinterpret_cast<uint32_t*>(gf.lo + 3 * n);
+    uint16_t* cells = reinterpret_cast<uint16_t*>(queues + W * kCtaQueue);  // G*G + 1
+    short2* sorted_meta = reinterpret_cast<short2*>(cells + ((Gcap * Gcap + 2) & ~1));  // (orig, cell)
+    long long* red = reinterpret_cast<long long*>(((uintptr_t)(sorted_meta + n) + 7) & ~(uintptr_t)7);
 
     const float L = side[cfg];
     int G = (int)(L / kCellMin);
@@ -102,27 +178,39 @@ __global__ void __launch_bounds__(T) sat_energy_kernel(int n, const float* __res
     const int ncell = G * G;
 
     for (int c = tid; c <= ncell; c += T) cells[c] = 0;
+    for (int k = tid; k < 6 * n; k += T) gf.hi[k] = 0;
     __syncthreads();
 
     // 1. load, trig, walls, cell binning
-    float e_loc = 0.f;
+    long long e_loc = 0;
+    double e_wall = 0.0;
     const float* src = xya + (size_t)cfg * 3 * n;
-    for (int i = tid; i < n; i += T) {
-        const float x = src[3 * i], y = src[3 * i + 1], a = src[3 * i + 2];
-        float s, c;
-        sincosf(a, &s, &c);
-        float gx = 0.f, gy = 0.f, ga = 0.f;
-        e_loc += wall_energy_grad(x, y, c, s, L, gx, gy, ga);
-        gacc[3 * i] = gx;
-        gacc[3 * i + 1] = gy;
-        gacc[3 * i + 2] = ga;
-        int cx = (int)floorf(x * inv_cell), cy = (int)floorf(y * inv_cell);
-        cx = cx < 0 ? 0 : (cx >= G ? G - 1 : cx);
-        cy = cy < 0 ? 0 : (cy >= G ? G - 1 : cy);
-        const int cell = cy * G + cx;
-        const int rank = atomicAdd(&cells[cell], 1);
-        stash[i] = make_float4(x, y, c, s);
-        orig_meta[i] = make_short2((short)cell, (short)rank);
+    float sx[NPT], sy[NPT], sc[NPT], ss[NPT], wx[NPT], wy[NPT], wa[NPT];
+    int cr[NPT];  // cell << 16 | rank
+#pragma unroll
+    for (int k = 0; k < NPT; ++k) {
+        const int i = tid + k * T;
+        if (i < n) {
+            const float x = src[3 * i], y = src[3 * i + 1], a = src[3 * i + 2];
+            float s, c;
+            sincosf(a, &s, &c);
+            float gx = 0.f, gy = 0.f, ga = 0.f;
+            e_wall += (double)wall_energy_grad(x, y, c, s, L, gx, gy, ga);
+            wx[k] = gx;
+            wy[k] = gy;
+            wa[k] = ga;
+            int cx = (int)floorf(x * inv_cell), cy = (int)floorf(y * inv_cell);
+            cx = cx < 0 ? 0 : (cx >= G ? G - 1 : cx);
+            cy = cy < 0 ? 0 : (cy >= G ? G - 1 : cy);
+            const int cell = cy * G + cx;
+            // per-cell counts in 16-bit halves of 32-bit words (native integer atomics)
+            const unsigned old = atomicAdd(reinterpret_cast<unsigned*>(cells) + (cell >> 1), 1u << (16 * (cell & 1)));
+            cr[k] = (cell << 16) | (int)((old >> (16 * (cell & 1))) & 0xffffu);
+            sx[k] = x;
+            sy[k] = y;
+            sc[k] = c;
+            ss[k] = s;
+        }
     }
     __syncthreads();
 
@@ -140,55 +228,34 @@ __global__ void __launch_bounds__(T) sat_energy_kernel(int n, const float* __res
         int run = incl - sum;
         for (int c = lo; c < hi; ++c) {
             int k = cells[c];
-            cells[c] = run;
+            cells[c] = (uint16_t)run;
             run += k;
         }
-        if (tid == 31) cells[ncell] = incl;
+        if (tid == 31) cells[ncell] = (uint16_t)incl;
     }
     __syncthreads();
-    for (int i = tid; i < n; i += T) {
-        const short2 m = orig_meta[i];
-        const int pos = cells[m.x] + m.y;
-        const float4 v = stash[i];
-        sxy[pos] = make_float2(v.x, v.y);
-        scs[pos] = make_float2(v.z, v.w);
-        sorted_meta[pos] = make_short2((short)i, m.x);
-    }
-    __syncthreads();
-    // order each cell's entries by original index (cells hold a few squares)
-    for (int c = tid; c < ncell; c += T) {
-        const int a = cells[c], b = cells[c + 1];
-        for (int u = a + 1; u < b; ++u) {
-            const float2 kxy = sxy[u], kcs = scs[u];
-            const short2 km = sorted_meta[u];
-            int w = u - 1;
-            while (w >= a && sorted_meta[w].x > km.x) {
-                sxy[w + 1] = sxy[w];
-                scs[w + 1] = scs[w];
-                sorted_meta[w + 1] = sorted_meta[w];
-                --w;
-            }
-            sxy[w + 1] = kxy;
-            scs[w + 1] = kcs;
-            sorted_meta[w + 1] = km;
+#pragma unroll
+    for (int k = 0; k < NPT; ++k) {
+        const int i = tid + k * T;
+        if (i < n) {
+            const int cell = cr[k] >> 16, pos = cells[cell] + (cr[k] & 0xffff);
+            sxy[pos] = make_float2(sx[k], sy[k]);
+            scs[pos] = make_float2(sc[k], ss[k]);
+            sorted_meta[pos] = make_short2((short)i, (short)cell);
         }
-    }
-    for (int k = tid; k < 3 * n; k += T) {
-        gf.hi[k] = 0;
-        gf.lo[k] = 0u;
     }
     __syncthreads();
 
     // 3. broad phase into warp queues, narrow phase 32 pairs at a time
     uint32_t cand_loc = 0;
-    uint32_t* queue = queues + warp * kQueue;
+    uint32_t* queue = queues + warp * kCtaQueue;
     int qn = 0;  // warp-uniform queue length
     auto narrow = [&](uint32_t entry) {
         const int p = (int)(entry & 0xffffu), q = (int)(entry >> 16);
         const float2 P = sxy[p], Q = sxy[q], Pc = scs[p], Qc = scs[q];
         PairGrad g;
         if (sat_pair_grad(Q.x - P.x, Q.y - P.y, Pc.x, Pc.y, Qc.x, Qc.y, g)) {
-            e_loc += g.e;
+            e_loc += e_units(g.e);
             const int i = sorted_meta[p].x, j = sorted_meta[q].x;
             gf.add(3 * i, g.px);
             gf.add(3 * i + 1, g.py);
@@ -217,72 +284,60 @@ __global__ void __launch_bounds__(T) sat_energy_kernel(int n, const float* __res
                 len2 = cells[(cy + 1) * G + min(cx + 2, G)] - a2;
             }
             len = len1 + len2;
+            a2 -= len1;  // q = a2 + t for t >= len1
         }
-        const int maxlen = __reduce_max_sync(0xffffffffu, len);
-        for (int t = 0; t < maxlen; ++t) {
-            bool pass = false;
-            int q = 0;
-            if (t < len) {
-                q = t < len1 ? a1 + t : a2 + (t - len1);
-                const float2 Q = sxy[q];
-                const float dx = Q.x - px, dy = Q.y - py;
-                const float d2 = dx * dx + dy * dy;
-                pass = d2 < kPairCut2;
-                cand_loc += d2 < 2.0f;
-            }
-            const uint32_t m = __ballot_sync(0xffffffffu, pass);
-            if (pass) queue[qn + __popc(m & ((1u << lane) - 1u))] = (uint32_t)p | ((uint32_t)q << 16);
-            qn += __popc(m);
-            if (qn >= 32) {
-                __syncwarp();
-                narrow(queue[lane]);
-                __syncwarp();
-                if (lane < qn - 32) queue[lane] = queue[32 + lane];
-                __syncwarp();
-                qn -= 32;
-            }
-        }
+        if (cand) broad_phase<true, kCtaQueue>(sxy, p, px, py, a1, len1, a2, len, lane, queue, qn, cand_loc, narrow);
+        else broad_phase<false, kCtaQueue>(sxy, p, px, py, a1, len1, a2, len, lane, queue, qn, cand_loc, narrow);
     }
     __syncwarp();
     if (lane < qn) narrow(queue[lane]);
     __syncthreads();
 
     // 4. reductions and stores
-    for (int o = 16; o > 0; o >>= 1) {
-        e_loc += __shfl_xor_sync(0xffffffffu, e_loc, o);
-        cand_loc += __shfl_xor_sync(0xffffffffu, cand_loc, o);
-    }
+    e_loc = warp_sum_units(e_loc);
+    cand_loc = __reduce_add_sync(0xffffffffu, cand_loc);
+    for (int o = 16; o > 0; o >>= 1) e_wall += __shfl_xor_sync(0xffffffffu, e_wall, o);
     if (lane == 0) {
-        red[warp] = e_loc;
-        reinterpret_cast<uint32_t*>(red)[W + warp] = cand_loc;
+        red[3 * warp] = e_loc;
+        red[3 * warp + 1] = cand_loc;
+        red[3 * warp + 2] = __double_as_longlong(e_wall);
     }
     __syncthreads();
     if (tid == 0) {
-        float e = 0.f;
-        uint32_t cc = 0;
+        long long e = 0, cc = 0;
+        double walls = 0.0;
         for (int w = 0; w < W; ++w) {
-            e += red[w];
-            cc += reinterpret_cast<uint32_t*>(red)[W + w];
+            e += red[3 * w];
+            cc += red[3 * w + 1];
+            walls += __longlong_as_double(red[3 * w + 2]);
         }
-        energy[cfg] = e;
-        if (cand) cand[cfg] = cc;
+        energy[cfg] = (float)(walls + (double)e * (1.0 / kEUnit));
+        if (cand) cand[cfg] = (uint32_t)cc;
     }
     if (grad) {
         float* dst = grad + (size_t)cfg * 3 * n;
-        for (int k = tid; k < 3 * n; k += T) dst[k] = gacc[k] + gf.value(k);
+#pragma unroll
+        for (int k = 0; k < NPT; ++k) {
+            const int i = tid + k * T;
+            if (i < n) {
+                dst[3 * i] = wx[k] + gf.value(3 * i);
+                dst[3 * i + 1] = wy[k] + gf.value(3 * i + 1);
+                dst[3 * i + 2] = wa[k] + gf.value(3 * i + 2);
+            }
+        }
     }
 }
 
 // ---------------------------------------------------------------------------
 // Warp-per-configuration form for n <= 256: the same phases as above run by
-// one warp without block barriers, several configurations per CTA, except that
-// energies are summed exactly as integers, so a cell's entries need no ordering.  A lane
-// keeps its (up to 8) squares in registers from the load to the scatter, all
-// loads are issued before any is used, and the cell grid is sized from n, so
-// ~7.7 KB of shared memory per configuration lets a whole 4,096-configuration
-// batch be resident in one wave.
+// one warp without block barriers, several configurations per CTA.  A lane
+// keeps its squares (NPL of them, the kernel is instantiated for each number)
+// in registers from the load to the scatter, all loads are issued before any
+// is used, and the cell grid is sized from n, so ~7.7 KB of shared memory per
+// configuration lets a whole 4,096-configuration batch of n = 200 be resident
+// in one wave.  Bound by issue slots (70% issuing at 4,096 x 200).  An instance
+// sized for n = 17 takes 6.15 us a call of 48 against 8.2 for the largest's.
 constexpr int kWarpMaxN = 256;
-constexpr int kWarpNpl = kWarpMaxN / 32;
 
 __host__ __device__ inline int warp_grid_cap(int n) {
     int g = (int)sqrtf((float)n) + 2;
@@ -294,7 +349,7 @@ __host__ __device__ inline size_t warp_smem_bytes(int n) {
     // sorted (x, y) + (c, s), pair-gradient accumulators, original index (byte),
     // cell starts (uint16), pair queue
     size_t b = (size_t)n * 16 + (size_t)n * 12 + (((size_t)n + 3) & ~(size_t)3) +
-               (((size_t)(G * G + 1) * 2 + 3) & ~(size_t)3) + kQueue * 4;
+               (((size_t)(G * G + 1) * 2 + 3) & ~(size_t)3) + kQueue * 2;
     return (b + 15) & ~(size_t)15;
 }
 
@@ -305,27 +360,13 @@ __host__ __device__ inline size_t warp_smem_bytes(int n) {
 // sum is exact and order-free.
 constexpr float kGScale = 524288.0f;
 
-// Energies of the warp kernel are summed as 64-bit integers in units of
-// 2^-40: every wall and pair term is rounded once (error below 5e-13), the
-// sum is exact, and so it does not depend on the order in which the pairs are
-// found -- cell lists built with atomics need no sorting for a deterministic
-// result.  A configuration's energy is far below 2^23, so the sum stays
-// below 2^63 units.
-constexpr double kEUnit = 1099511627776.0;  // 2^40
-__device__ __forceinline__ long long e_units(float e) { return __float2ll_rn(e * 1099511627776.0f); }
-
-// round(v * kGScale) to the nearest integer (ties to even) on the FMA pipe:
-// for |v * kGScale| < 2^22 the fused v * 2^19 + 1.5 * 2^23 lands in
-// [2^23, 2^24), where one float ulp is 1, so its bit pattern minus that of
-// 1.5 * 2^23 is the rounded integer.  |v| < 5.13 keeps it within range.
-__device__ __forceinline__ int gq_units(float v) {
-    return __float_as_int(fmaf(v, kGScale, 12582912.0f)) - 0x4B400000;
-}
+// round(v * kGScale) on the FMA pipe: |v| < 5.13 keeps v * 2^19 below 2^22.
+__device__ __forceinline__ int gq_units(float v) { return magic_int(fmaf(v, kGScale, kMagic)); }
 
 // 28 / W CTAs of W warps per SM (72 registers a thread at W = 4; the default
 // is W = 2, measured 2% faster than 4 and 20% faster than 8): with the
 // shared memory of n = 200 that keeps 4,096 configurations in one wave.
-template <int W, bool COUNT>
+template <int W, bool COUNT, int NPL>
 __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int configs, int n, const float* __restrict__ xya,
                                                                  const float* __restrict__ side,
                                                                  float* __restrict__ energy, float* __restrict__ grad,
@@ -342,7 +383,7 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
     int* gq = reinterpret_cast<int*>(scs + n);                 // pair-gradient sums (kGScale units)
     uint8_t* orig = reinterpret_cast<uint8_t*>(gq + 3 * n);    // sorted -> original index
     uint16_t* cells = reinterpret_cast<uint16_t*>(orig + ((n + 3) & ~3));  // G*G + 1 starts
-    uint32_t* queue = reinterpret_cast<uint32_t*>(cells + (((Gcap * Gcap + 1) + 1) & ~1));
+    uint16_t* queue = cells + (((Gcap * Gcap + 1) + 1) & ~1);  // p | q << 8
 
     const float L = side[cfg];
     int G = (int)(L / kCellMin);
@@ -354,9 +395,9 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
 
     // 1. all loads first, then trig, walls and cell ranks
     const float* src = xya + (size_t)cfg * 3 * n;
-    float px[kWarpNpl], py[kWarpNpl], pa[kWarpNpl];
+    float px[NPL], py[NPL], pa[NPL];
 #pragma unroll
-    for (int k = 0; k < kWarpNpl; ++k) {
+    for (int k = 0; k < NPL; ++k) {
         const int i = lane + 32 * k;
         if (i < n) {
             px[k] = src[3 * i];
@@ -366,17 +407,25 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
     }
     __syncwarp();
     long long e_loc = 0;  // kEUnit units: exact, so the sum does not depend on the order of the pairs
-    float pc[kWarpNpl], ps[kWarpNpl];
-    int cr[kWarpNpl];  // cell << 16 | rank
+    // Wall gradients wait in registers for the pair sums; with many squares a
+    // lane there is no room, and they go straight out and are read back.
+    constexpr bool kKeepWalls = NPL <= 2;
+    float wx[kKeepWalls ? NPL : 1], wy[kKeepWalls ? NPL : 1], wa[kKeepWalls ? NPL : 1];
+    float pc[NPL], ps[NPL];
+    int cr[NPL];  // cell << 16 | rank
 #pragma unroll
-    for (int k = 0; k < kWarpNpl; ++k) {
+    for (int k = 0; k < NPL; ++k) {
         const int i = lane + 32 * k;
         if (i < n) {
             sincosf(pa[k], &ps[k], &pc[k]);
             float gx = 0.f, gy = 0.f, ga = 0.f;
             e_loc += e_units(wall_energy_grad(px[k], py[k], pc[k], ps[k], L, gx, gy, ga));
-            if (gdst) {  // the wall term goes straight out (unbounded for squares far outside
-                         // the box); pair terms are added at the end
+            // (kept apart from the pair sums: unbounded for squares far outside the box)
+            if (kKeepWalls) {
+                wx[k % (kKeepWalls ? NPL : 1)] = gx;
+                wy[k % (kKeepWalls ? NPL : 1)] = gy;
+                wa[k % (kKeepWalls ? NPL : 1)] = ga;
+            } else if (gdst) {
                 gdst[3 * i] = gx;
                 gdst[3 * i + 1] = gy;
                 gdst[3 * i + 2] = ga;
@@ -414,7 +463,7 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
     }
     __syncwarp();
 #pragma unroll
-    for (int k = 0; k < kWarpNpl; ++k) {
+    for (int k = 0; k < NPL; ++k) {
         const int i = lane + 32 * k;
         if (i < n) {
             const int cell = cr[k] >> 16;
@@ -430,7 +479,7 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
     uint32_t cand_loc = 0;
     int qn = 0;
     auto narrow = [&](uint32_t entry) {
-        const int p = (int)(entry & 0xffffu), q = (int)(entry >> 16);
+        const int p = (int)(entry & 0xffu), q = (int)(entry >> 8);
         const float2 P = sxy[p], Q = sxy[q], Pc = scs[p], Qc = scs[q];
         PairGrad g;
         if (sat_pair_grad(Q.x - P.x, Q.y - P.y, Pc.x, Pc.y, Qc.x, Qc.y, g)) {
@@ -465,73 +514,75 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
             len = len1 + len2;
             a2 -= len1;  // q = a2 + t for t >= len1
         }
-        const int maxlen = __reduce_max_sync(0xffffffffu, len);
-        for (int t = 0; t < maxlen; ++t) {
-            bool pass = false;
-            int q = 0;
-            if (t < len) {
-                q = (t < len1 ? a1 : a2) + t;
-                const float2 Q = sxy[q];
-                const float dx = Q.x - qx0, dy = Q.y - qy0;
-                const float d2 = dx * dx + dy * dy;
-                pass = d2 < kPairCut2;
-                if (COUNT) cand_loc += d2 < 2.0f;
-            }
-            const uint32_t m = __ballot_sync(0xffffffffu, pass);
-            if (pass) queue[qn + __popc(m & ((1u << lane) - 1u))] = (uint32_t)p | ((uint32_t)q << 16);
-            qn += __popc(m);
-            if (qn >= 32) {
-                __syncwarp();
-                narrow(queue[lane]);
-                __syncwarp();
-                if (lane < qn - 32) queue[lane] = queue[32 + lane];
-                __syncwarp();
-                qn -= 32;
-            }
-        }
+        broad_phase<COUNT, kQueue>(sxy, p, qx0, qy0, a1, len1, a2, len, lane, queue, qn, cand_loc, narrow);
     }
     __syncwarp();
     if (lane < qn) narrow(queue[lane]);
     __syncwarp();
 
-    // 4. reductions and the coalesced gradient store
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        e_loc += __shfl_xor_sync(0xffffffffu, e_loc, o);
-        cand_loc += __shfl_xor_sync(0xffffffffu, cand_loc, o);
-    }
+    // 4. reductions and the gradient store
+    e_loc = warp_sum_units(e_loc);
+    if (COUNT) cand_loc = __reduce_add_sync(0xffffffffu, cand_loc);
     if (lane == 0) {
         energy[cfg] = (float)((double)e_loc * (1.0 / kEUnit));
         if (COUNT) cand[cfg] = cand_loc;
     }
-    if (gdst) {
+    if (!gdst) return;
+    if (kKeepWalls) {
+#pragma unroll
+        for (int k = 0; k < NPL; ++k) {
+            const int i = lane + 32 * k;
+            if (i < n) {
+                gdst[3 * i] = wx[k % (kKeepWalls ? NPL : 1)] + (float)gq[3 * i] * (1.0f / kGScale);
+                gdst[3 * i + 1] = wy[k % (kKeepWalls ? NPL : 1)] + (float)gq[3 * i + 1] * (1.0f / kGScale);
+                gdst[3 * i + 2] = wa[k % (kKeepWalls ? NPL : 1)] + (float)gq[3 * i + 2] * (1.0f / kGScale);
+            }
+        }
+    } else {
         for (int k = lane; k < 3 * n; k += 32) gdst[k] += (float)gq[k] * (1.0f / kGScale);
     }
 }
 
-template <int W>
-static int launch_warp(sqs_ctx* ctx, cudaStream_t st, int configs, int n, const float* xya, const float* side,
-                       float* energy, float* grad, uint32_t* cand) {
+template <int W, int NPL>
+static int launch_warp_npl(sqs_ctx* ctx, cudaStream_t st, int configs, int n, const float* xya, const float* side,
+                           float* energy, float* grad, uint32_t* cand) {
     const size_t smem = warp_smem_bytes(n) * W;
     static bool attr_set[64] = {false};
     const int dev = ctx->device & 63;
     if (!attr_set[dev]) {
-        SQS_CUDA(cudaFuncSetAttribute(sat_energy_warp_kernel<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        SQS_CUDA(cudaFuncSetAttribute(sat_energy_warp_kernel<W, true, NPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       200 * 1024));
-        SQS_CUDA(cudaFuncSetAttribute(sat_energy_warp_kernel<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      200 * 1024));
+        SQS_CUDA(cudaFuncSetAttribute(sat_energy_warp_kernel<W, false, NPL>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set[dev] = true;
     }
     const unsigned blocks = (unsigned)((configs + W - 1) / W);
     if (cand)
-        sat_energy_warp_kernel<W, true><<<blocks, W * 32, smem, st>>>(configs, n, xya, side, energy, grad,
-                                                                               cand);
+        sat_energy_warp_kernel<W, true, NPL><<<blocks, W * 32, smem, st>>>(configs, n, xya, side, energy, grad, cand);
     else
-        sat_energy_warp_kernel<W, false><<<blocks, W * 32, smem, st>>>(configs, n, xya, side, energy, grad,
-                                                                                nullptr);
+        sat_energy_warp_kernel<W, false, NPL><<<blocks, W * 32, smem, st>>>(configs, n, xya, side, energy, grad,
+                                                                            nullptr);
     SQS_CUDA(cudaGetLastError());
     ctx->launches += 1;
     return SQS_OK;
+}
+
+// W warps per CTA; the instance with the squares a lane has, rounded up (the
+// widths other than the default keep one instance for every n).
+template <int W>
+static int launch_warp(sqs_ctx* ctx, cudaStream_t st, int configs, int n, const float* xya, const float* side,
+                       float* energy, float* grad, uint32_t* cand) {
+    if (W != 2) return launch_warp_npl<W, 8>(ctx, st, configs, n, xya, side, energy, grad, cand);
+    switch ((n + 31) / 32) {
+        case 1: return launch_warp_npl<2, 1>(ctx, st, configs, n, xya, side, energy, grad, cand);
+        case 2: return launch_warp_npl<2, 2>(ctx, st, configs, n, xya, side, energy, grad, cand);
+        case 3: return launch_warp_npl<2, 3>(ctx, st, configs, n, xya, side, energy, grad, cand);
+        case 4: return launch_warp_npl<2, 4>(ctx, st, configs, n, xya, side, energy, grad, cand);
+        case 5: return launch_warp_npl<2, 5>(ctx, st, configs, n, xya, side, energy, grad, cand);
+        case 6: return launch_warp_npl<2, 6>(ctx, st, configs, n, xya, side, energy, grad, cand);
+        case 7: return launch_warp_npl<2, 7>(ctx, st, configs, n, xya, side, energy, grad, cand);
+        default: return launch_warp_npl<2, 8>(ctx, st, configs, n, xya, side, energy, grad, cand);
+    }
 }
 
 template <int T>
@@ -557,7 +608,7 @@ static int sat_energy_launch_on(sqs_ctx* ctx, cudaStream_t st, int configs, int 
     SQS_REQUIRE(n >= 1 && n <= kSatMaxN, "n %d out of 1..%d", n, kSatMaxN);
     SQS_REQUIRE(xya && side && energy, "null device pointer");
     if (configs == 0) return SQS_OK;
-    if (threads == 0) threads = n <= kWarpMaxN ? -2 : 128;
+    if (threads == 0) threads = n <= kWarpMaxN ? -2 : 256;
     if (threads < 0) {  // warp-per-configuration kernel, -threads warps per CTA
         SQS_REQUIRE(n <= kWarpMaxN, "the warp-per-configuration kernel takes n <= %d", kWarpMaxN);
         switch (-threads) {
