@@ -132,6 +132,17 @@ int prepare_job(const sqs_job& J, int j, JobDev& d, JobMut& m, Plan& p, const Sh
     return SQS_OK;
 }
 
+bool replan(const sqs_job& J, int rl, JobDev& d, Plan& p) {
+    Plan q;
+    const int want = std::min(16, (J.replicas + rl - 1) / rl);
+    if (!plan_job(J.n, J.replicas, J.L0, p.cell, want, q) && !plan_job(J.n, J.replicas, J.L0, p.cell, 1, q)) return false;
+    if (q.cs == p.cs) return false;
+    p = q;
+    d.cs = q.cs;
+    d.Rl = q.Rl;
+    return true;
+}
+
 // replicas, then the quench scratch of up to one CTA per replica
 int64_t job_pos_elems(const sqs_job& J) { return (int64_t)J.replicas * J.n * (1 + kQuenchScr); }
 

@@ -58,6 +58,7 @@ struct SJob {
     JobDev jd{};
     JobMut jm{};
     Plan plan{};
+    bool free_shape = false;    // neither pinned nor tuned: the server picks the shape slice by slice
     int64_t left = 0;           // sweeps not yet launched
     size_t off = 0, bytes = 0;  // arena block
     sqs_job_result res{};
@@ -381,6 +382,7 @@ extern "C" int sqs_server_submit(sqs_server* s, const sqs_job* job, int64_t* id)
         j.job.xya_rep = j.xya_rep.data();
     }
     if (int r = prepare_job(j.job, 0, j.jd, j.jm, j.plan, &shape)) return r;
+    j.free_shape = shape.cs == 0;
     j.left = job_sweeps(j.job);
     SQS_REQUIRE(job_bytes(j.job) <= s->arena_bytes, "job state (%zu bytes) exceeds the server's HBM budget",
                 job_bytes(j.job));
@@ -452,14 +454,33 @@ int launch_idle(sqs_server* s, const std::vector<int32_t>& fin, int& launched) {
     std::map<Key, int> nmax;
     std::vector<uint8_t> retiring((size_t)s->max_active, 0);
     for (int32_t k : fin) retiring[(size_t)k] = 1;
+    // Replicas a CTA of the slices started now.  Few replicas on the whole GPU
+    // run faster spread out: a warp's proposals are a chain, and 16 of them on
+    // an SM get in each other's way.  One job of n = 295 with 64 replicas took
+    // 15.8 / 13.0 / 12.6 ms on CTAs of 16 / 8 / 4, 64 jobs (2,048 replicas of
+    // n 150..250) 7.5 / 8.1 / 8.9; the lines lie where the order changes
+    // (8 below 900 to 1,000 replicas, 4 below about 300, on 148 SMs).  The
+    // shape does not change a job's trajectory, so it follows the load from
+    // slice to slice.
+    int replicas = 0;
+    for (int k = 0; k < s->max_active; ++k)
+        if (s->slot_job[(size_t)k] >= 0 && !retiring[(size_t)k] && !s->retiring[(size_t)k])
+            replicas += s->jobs[s->slot_job[(size_t)k]].job.replicas;
+    const int rl = replicas <= 2 * s->ctx->sm_count ? 4 : (replicas <= 6 * s->ctx->sm_count ? 8 : kMaxRl);
+    bool reshaped = false;
     for (int k = 0; k < s->max_active; ++k) {
         if (s->slot_job[(size_t)k] < 0 || s->flying[(size_t)k] || retiring[(size_t)k] || s->retiring[(size_t)k]) continue;
-        const SJob& j = s->jobs[s->slot_job[(size_t)k]];
+        SJob& j = s->jobs[s->slot_job[(size_t)k]];
+        if (j.free_shape && replan(j.job, rl, j.jd, j.plan)) {
+            SQS_CUDA(cudaMemcpyAsync(s->d_jd + k, &j.jd, sizeof(JobDev), cudaMemcpyHostToDevice, s->ast));
+            reshaped = true;
+        }
         const Key key = std::make_tuple(j.plan.cs, j.plan.Rl, (int)uses_moves(j.jd.flags));
         groups[key].push_back(k);
         rb[key] = std::max(rb[key], j.plan.rb);
         nmax[key] = std::max(nmax[key], j.job.n);
     }
+    if (reshaped) SQS_CUDA(cudaEventRecord(s->admitted, s->ast));
     auto work = [&](int32_t k) {
         const SJob& j = s->jobs[s->slot_job[(size_t)k]];
         return j.left * (int64_t)j.job.n;
