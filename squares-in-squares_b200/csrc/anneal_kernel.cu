@@ -124,7 +124,7 @@ __device__ bool build_cells(const Rep& R, int n, const Grid& g, int lane) {
 // two compares for its row and two for its cell.  Against nine guarded byte
 // loads, a nine-step sum and an eight-step search this halves the instructions
 // around a candidate.
-template <int kStride = 32, typename Fn>
+template <int kStride, typename Fn>
 __device__ __forceinline__ void for_block(const Rep& R, const Grid& g, int cx, int cy, int lane, Fn&& fn) {
     const unsigned mask = cx == g.G - 1 ? 0x00ffffu : 0xffffffu;
     const int xs = cx > 0 ? cx - 1 : 0;
@@ -823,10 +823,10 @@ __device__ int build_pair_list(const Rep& R, int n, const Grid& g, int lane, flo
 // lists are rebuilt only when a square changes cells.  A rejected move (or one
 // that overflows a cell) is undone from `scr`, the replica's scratch block
 // (n float4 undo copy, at 3 n the reference centres, from 4 n the pairs).
-// Returns whether it was accepted; *ovf counts overflows.
+// Returns whether it was accepted; an overflow adds `count` to *ovf.
 __device__ __forceinline__ bool collective_move(const Rep& rep, const Grid& g, int n, float L, int lane, int mode, int c,
                                              float tx, float ty, float th, float u, float invT, long long& E,
-                                             float4* __restrict__ scr, int& npl, int* ovf) {
+                                             float4* __restrict__ scr, int& npl, int count, int* ovf) {
     float4* save = scr;
     float2* ref = reinterpret_cast<float2*>(scr + 3 * n);
     uint32_t* pl = reinterpret_cast<uint32_t*>(scr + 4 * n);
@@ -888,7 +888,7 @@ __device__ __forceinline__ bool collective_move(const Rep& rep, const Grid& g, i
         acc = dq <= 0 || u < __expf(-((float)dq * (1.0f / kEScale)) * invT);
         if (acc) E = En;
     } else {
-        ++*ovf;
+        *ovf += count;
     }
     if (!acc) {
         for (int s = lane; s < n; s += 32) {
@@ -1088,20 +1088,24 @@ struct IntTag {
     static constexpr int value = V;
 };
 
-// A proposal's move: the square (-1: nothing moved) and its old and new
-// cells, one byte per coordinate (grids are at most 64 / 1.59 < 256 wide).
-struct Moved {
-    int i, cells;
-};
+// A proposal's old and new cells, one byte per coordinate (grids are at most
+// 64 / 1.59 < 256 wide).
 __device__ __forceinline__ int pack_cells(int ox, int oy, int nx, int ny) {
     return ox | (oy << 8) | (nx << 16) | (ny << 24);
 }
-// Did move (mi, mc) change what a proposal of square ik from cells ck read?
+// Whether two cells (16 bits a coordinate) are the same or adjacent: each
+// half of a + 0x8001 - b holds 0x8000 + difference + 1, without borrows, and
+// the difference + 1 must be 0, 1 or 2.
+__device__ __forceinline__ bool near_cells(unsigned a, unsigned b) {
+    const unsigned d = (a + 0x80018001u - b) ^ 0x80008000u;
+    return ((d & 0xfffcfffcu) | (d & (d >> 1) & 0x00010001u)) == 0u;
+}
+// Did the move of square mi (-1: none) between cells mc change what a
+// proposal of square ik from cells ck read?
 __device__ __forceinline__ bool touches(int mi, int mc, int ik, int ck) {
-    if (mi < 0) return false;
-    const int bx = ck & 0xff, by = (ck >> 8) & 0xff;
-    const int ox = mc & 0xff, oy = (mc >> 8) & 0xff, nx = (mc >> 16) & 0xff, ny = (int)((unsigned)mc >> 24);
-    return mi == ik || (abs(ox - bx) <= 1 && abs(oy - by) <= 1) || (abs(nx - bx) <= 1 && abs(ny - by) <= 1);
+    const unsigned b = __byte_perm((unsigned)ck, 0u, 0x4140);
+    const unsigned o = __byte_perm((unsigned)mc, 0u, 0x4140), n = __byte_perm((unsigned)mc, 0u, 0x4342);
+    return mi >= 0 && (mi == ik || near_cells(o, b) || near_cells(n, b));
 }
 
 template <bool MOVES>
@@ -1168,8 +1172,10 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
     if (active) {
         E = S.jm.done == 0 ? full_energy(rep, n, g, Lr, lane) : S.jm.E[r];
     }
-    unsigned long long props = 0, accs = 0;
+    // sums of a lane's share, added up at the end (Epart: at each checkpoint)
+    unsigned accs = 0;
     int ovf = 0;
+    long long Epart = 0;
     // move-set options: step adaptation with a cooling cycle of 200 exchange
     // rounds (temperatures x 0.002^(k/199), steps x its square root)
     const bool adaptive = MOVES && (jd.flags & kMoveAdapt) != 0;
@@ -1283,10 +1289,8 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     form_trial(fminf(kMaxStep, fmaxf(-kMaxStep, ddx)), fminf(kMaxStep, fmaxf(-kMaxStep, ddy)), dda);
                 };
                 if (!MOVES) form_plain();
-                // proposal q of this batch, evaluated by the whole warp; returns
-                // the square it moved (-1: none) and its old and new cells
-                auto single = [&](int q) -> Moved {
-                    Moved mv{-1, 0};
+                // proposal q of this batch, evaluated by the whole warp
+                auto single = [&](int q) {
                     const int dpk = __shfl_sync(0xffffffffu, di, q);
                     const int i = dpk & 0xffff, mode = dpk >> 16;
                     const float u_acc = __shfl_sync(0xffffffffu, du, q);
@@ -1305,9 +1309,8 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     }
                     if (MOVES && mode != 0) {
                         acc = collective_move(rep, g, n, Lr, lane, mode, i, dx, dy, da, u_acc, invT, E, scr_own, npl,
-                                              &ovf);
-                        ++props;
-                        accs += acc;
+                                              lane == 0, &ovf);
+                        if (lane == 0) accs += acc;
                     } else {
                         if (MOVES) {
                             if (lane == q) form_trial(dx, dy, da);
@@ -1322,7 +1325,7 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                                   ncy = (int)((unsigned)cells >> 24);
                         const float4 P = rep.sq[i];
                         long long dq = lane == q ? tw : 0;
-                        for_block(rep, g, ocx, ocy, lane, [&](int j) {
+                        for_block<32>(rep, g, ocx, ocy, lane, [&](int j) {
                             const long long d = pair_delta(rep.sq[j], nx, ny, nc, ns, P);
                             dq += j != i ? d : 0;
                         });
@@ -1332,19 +1335,18 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                         const int oc = ocy * g.G + ocx, ncell = ncy * g.G + ncx;
                         if (acc && oc != ncell && rep.cnt[ncell] >= kCellK) {
                             acc = false;
-                            ++ovf;
+                            if (lane == 0) ++ovf;
                         }
-                        ++props;
                         if (acc) {
-                            ++accs;
-                            E += dq;
+                            if (lane == 0) ++accs;
+                            if (MOVES) E += dq;
+                            else if (lane == 0) Epart += dq;
                             if (lane == q) apply_move(i, tx, ty, tc, ts, ta, oc, ncell);
                             stale |= (di & 0xffff) == i;
                             if (MOVES && npl >= 0) {  // out of the pair list's reach?
                                 const float2 o = reinterpret_cast<const float2*>(scr_own + 3 * n)[i];
                                 if (!(fabsf(nx - o.x) <= kListStep && fabsf(ny - o.y) <= kListStep)) npl = -1;
                             }
-                            mv = Moved{i, cells};
                         }
                     }
                     if (adaptive) {  // every 16 proposals: steer toward 25% acceptance
@@ -1355,7 +1357,6 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                         }
                     }
                     __syncwarp();
-                    return mv;
                 };
                 // Proposals q .. q + M - 1 evaluated at once, one per group of
                 // 32 / M lanes, all against the current state.  A proposal's
@@ -1364,15 +1365,15 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                 // new cell of that move inside its 3x3 block (cells are wider
                 // than a step, so a move changes a square's cell by at most one;
                 // every other read -- counts and slots of the block, squares in
-                // it, the count of its target cell -- lies in that block).
-                // When no accepted move touches a later proposal, all decisions
-                // stand, the accepted moves lie in distinct cells, and each
-                // proposal's own lane applies its move at the same time.
-                // Otherwise they are decided in order, and a proposal that was
-                // touched is evaluated again by the whole warp on the current
-                // state.  Energies are exact and order-free, so the trajectory
-                // is the one-at-a-time trajectory, bit for bit.
-                auto group = [&](int q, auto mtag) {
+                // it, the count of its target cell -- lies in that block).  The
+                // proposals before the first that was touched are settled: their
+                // accepted moves lie in distinct cells, and each proposal's own
+                // lane applies its move at the same time; the next group starts
+                // at the touched one.  Energies are exact and order-free, so the
+                // trajectory is the one-at-a-time trajectory, bit for bit.
+                // Energy, acceptances and overflows are summed a lane each and
+                // added up after the batch.  Returns the proposals settled.
+                auto group = [&](int q, auto mtag) -> int {
                     constexpr int M = decltype(mtag)::value, W = 32 / M;
                     const int grp = lane / W, gl = lane % W;
                     const int qs = q + grp;
@@ -1407,12 +1408,16 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     const long long mine = (long long)hi * 1048576ll + (long long)lo +
                                            (long long)(((unsigned long long)(unsigned)whi << 32) | wlo);
                     const float de = (float)mine * (1.0f / kEScale);
-                    const int oc = ocy * g.G + ocx, ncell = ncy * g.G + ncx;
-                    int acc = mine <= 0 || u_acc < __expf(-de * invT);
-                    int ov = 0;
-                    if (acc && oc != ncell && rep.cnt[ncell] >= kCellK) {
-                        acc = 0;
-                        ov = 1;
+                    bool acc = mine <= 0 || u_acc < __expf(-de * invT), full = false;
+                    if (acc && ((cells ^ (cells >> 16)) & 0xffff)) {  // a new cell: has it room?
+                        full = rep.cnt[ncy * g.G + ncx] >= kCellK;
+                        acc = !full;
+                    }
+                    unsigned am = __ballot_sync(0xffffffffu, acc && gl == 0);
+                    if (am == 0u) {  // nothing moves
+                        ovf += full && gl == 0;
+                        __syncwarp();
+                        return M;
                     }
                     // does an accepted move of an earlier proposal touch this one?
                     const int mv_i = acc ? i : -1;
@@ -1423,53 +1428,23 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                         const int ocl = __shfl_up_sync(0xffffffffu, cells, d * W);
                         hit |= grp >= d && touches(oi, ocl, i, cells);
                     }
-                    if (!__any_sync(0xffffffffu, hit)) {
-                        const unsigned am = __ballot_sync(0xffffffffu, acc && gl == 0);
-                        ovf += __popc(__ballot_sync(0xffffffffu, ov && gl == 0));
-                        props += M;
-                        if (am) {
-                            accs += __popc(am);
-                            E += warp_sum_ll(acc && gl == 0 ? mine : 0);
-                            if (lane >= q && lane < q + M && (am >> ((lane - q) * W) & 1u))
-                                apply_move(di, tx, ty, tc, ts, ta, ((tcells >> 8) & 0xff) * g.G + (tcells & 0xff),
-                                           (int)((unsigned)tcells >> 24) * g.G + ((tcells >> 16) & 0xff));
-#pragma unroll
-                            for (int k = 0; k < M; ++k) stale |= (am >> (k * W) & 1u) && di == __shfl_sync(0xffffffffu, i, k * W);
+                    const unsigned hm = __ballot_sync(0xffffffffu, hit);
+                    const int take = hm ? (__ffs(hm) - 1) / W : M;  // (the first proposal is never touched)
+                    if (gl == 0 && grp < take) {
+                        if (acc) {
+                            Epart += mine;
+                            ++accs;
                         }
-                        __syncwarp();
-                        return;
+                        ovf += full;
                     }
-                    int mi[M], mc[M];  // the group's moves so far: square (-1: none), cells
+                    if (take < M) am &= (1u << (take * W)) - 1u;
+                    if (lane >= q && lane < q + take && (am >> ((lane - q) * W) & 1u))
+                        apply_move(di, tx, ty, tc, ts, ta, ((tcells >> 8) & 0xff) * g.G + (tcells & 0xff),
+                                   (int)((unsigned)tcells >> 24) * g.G + ((tcells >> 16) & 0xff));
 #pragma unroll
-                    for (int k = 0; k < M; ++k) {
-                        const int src = k * W;
-                        const int ik = __shfl_sync(0xffffffffu, i, src), ck = __shfl_sync(0xffffffffu, cells, src);
-                        bool redo = false;
-#pragma unroll
-                        for (int m = 0; m < k; ++m) redo |= touches(mi[m], mc[m], ik, ck);
-                        if (redo) {
-                            const Moved mv = single(q + k);
-                            mi[k] = mv.i;
-                            mc[k] = mv.cells;
-                        } else {
-                            const int ak = __shfl_sync(0xffffffffu, acc, src), ovk = __shfl_sync(0xffffffffu, ov, src);
-                            const unsigned dlo = __shfl_sync(0xffffffffu, (unsigned)(unsigned long long)mine, src);
-                            const int dhi = __shfl_sync(0xffffffffu, (int)(mine >> 32), src);
-                            ++props;
-                            accs += ak;
-                            ovf += ovk;
-                            if (ak) {
-                                E += (long long)(((unsigned long long)(unsigned)dhi << 32) | dlo);
-                                if (lane == q + k)
-                                    apply_move(di, tx, ty, tc, ts, ta, ((tcells >> 8) & 0xff) * g.G + (tcells & 0xff),
-                                               (int)((unsigned)tcells >> 24) * g.G + ((tcells >> 16) & 0xff));
-                                stale |= di == ik;
-                            }
-                            __syncwarp();
-                            mi[k] = ak ? ik : -1;
-                            mc[k] = ck;
-                        }
-                    }
+                    for (int k = 0; k < M; ++k) stale |= (am >> (k * W) & 1u) && di == __shfl_sync(0xffffffffu, i, k * W);
+                    __syncwarp();
+                    return take;
                 };
                 // A replica of up to 32 squares without move-set options holds
                 // square `lane` in registers and tests a proposal against every
@@ -1489,21 +1464,22 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     const float4 P = rep.sq[i];
                     const long long d = pair_delta(own, nx, ny, nc, ns, P);
                     const long long dq = warp_sum_dq((lane != i && lane < n ? d : 0) + (lane == q ? tw : 0));
-                    ++props;
-                    bool acc = dq <= 0 || u_acc < __expf(-((float)dq * (1.0f / kEScale)) * invT);
+                    const bool acc = dq <= 0 || u_acc < __expf(-((float)dq * (1.0f / kEScale)) * invT);
                     if (!acc) return;
                     if (n > kCellK) {
                         const int cells = __shfl_sync(0xffffffffu, tcells, q);
                         const int ncell = (int)((unsigned)cells >> 24) * g.G + ((cells >> 16) & 0xff);
                         const int there = __popc(__ballot_sync(0xffffffffu, own_cell == ncell));
                         if (ncell != ((cells >> 8) & 0xff) * g.G + (cells & 0xff) && there >= kCellK) {
-                            ++ovf;
+                            if (lane == 0) ++ovf;
                             return;
                         }
                         if (lane == i) own_cell = ncell;
                     }
-                    ++accs;
-                    E += dq;
+                    if (lane == 0) {
+                        ++accs;
+                        Epart += dq;
+                    }
                     if (lane == i) own = make_float4(nx, ny, nc, ns);
                     if (lane == q) {
                         rep.sq[i] = make_float4(nx, ny, nc, ns);
@@ -1513,19 +1489,19 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     __syncwarp();
                 };
                 // groups need room: on small grids most proposals would be
-                // evaluated twice; the move-set instance keeps one at a time
-                // (its step scale follows the acceptance of the previous move)
-                const bool fours = !MOVES && g.G >= 8, twos = !MOVES && g.G >= 4;
+                // evaluated twice (fours from G = 6 on against 8: 16 replicas of
+                // n = 120 take 14.2 against 15.1 ms, n = 60 is the same); the
+                // move-set instance keeps one at a time (its step scale follows
+                // the acceptance of the previous move)
+                const bool fours = !MOVES && g.G >= 6, twos = !MOVES && g.G >= 4;
                 for (int q = 0; q < kn;) {
                     if (small) {
                         tiny(q);
                         ++q;
                     } else if (fours && q + 3 < kn) {
-                        group(q, IntTag<4>{});
-                        q += 4;
+                        q += group(q, IntTag<4>{});
                     } else if (twos && q + 1 < kn) {
-                        group(q, IntTag<2>{});
-                        q += 2;
+                        q += group(q, IntTag<2>{});
                     } else {
                         single(q);
                         ++q;
@@ -1533,6 +1509,10 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                 }
             }
             if (small) build_cells(rep, n, g, lane);  // every cell within its capacity
+            if (!MOVES) {
+                E += warp_sum_ll(Epart);
+                Epart = 0;
+            }
         }
         p_at = stop;
         // ---- checkpoint: best-state search, shrink, replica exchange.  Only
@@ -1760,6 +1740,8 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
 
     // ---- write the slice back
     if (active) {
+        const long long accs_all = warp_sum_ll(accs);
+        const int ovf_all = __reduce_add_sync(0xffffffffu, ovf);
         float4* dst = pos + jd.pos_off + (int64_t)r * n;
         for (int i = lane; i < n; i += 32) dst[i] = make_float4(rep.sq[i].x, rep.sq[i].y, rep.ang[i], 0.f);
         if (lane == 0) {
@@ -1768,9 +1750,9 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                 jmut[job].adapt[r] = adapt;
                 jmut[job].win[r] = win;
             }
-            atomicAdd(reinterpret_cast<unsigned long long*>(&jmut[job].proposals), props);
-            atomicAdd(reinterpret_cast<unsigned long long*>(&jmut[job].accepted), accs);
-            if (ovf) atomicAdd(&jmut[job].overflows, ovf);
+            atomicAdd(reinterpret_cast<unsigned long long*>(&jmut[job].proposals), (unsigned long long)(p_at - S.jm.done));
+            atomicAdd(reinterpret_cast<unsigned long long*>(&jmut[job].accepted), (unsigned long long)accs_all);
+            if (ovf_all) atomicAdd(&jmut[job].overflows, ovf_all);
         }
     }
     if (rank == 0 && tid == 0) {
@@ -1951,14 +1933,14 @@ int anneal_max_clusters(int cs, int Rl, size_t smem, bool moves, int* out) {
     return max_clusters_gw(cs, Rl, smem, moves, 1, out);
 }
 
-// Warps a replica for a launch of njobs clusters: 1 (the replica's own warp),
-// or with the move-set options the most, up to kMaxRl / Rl, that keep as
-// many of the launch's clusters resident at once.  The extra warps idle
-// while their CTA anneals and join the checkpoint quench, which
-// SQS_JOB_QUENCH_ALL runs for every replica at once (same results: the
-// quench's sums are integers).
+// Warps a replica for a launch of njobs clusters: the most, up to
+// kMaxRl / Rl, that keep as many of the launch's clusters resident at once.
+// The extra warps idle while their CTA anneals and join the checkpoint quench
+// (same results: the quench's sums are integers), be it of every replica
+// (SQS_JOB_QUENCH_ALL) or of the coldest: with 4 replicas a CTA the quench of
+// n = 200 went from 4 to 13 warps and 100 sweeps from 12.5 to 11.4 ms.
 static int quench_warps(int njobs, int cs, int Rl, size_t smem, bool moves) {
-    if (!moves || Rl >= kMaxRl) return 1;
+    if (Rl >= kMaxRl) return 1;
     int base = 0;
     if (max_clusters_gw(cs, Rl, smem, moves, 1, &base) != SQS_OK) return 1;
     const int need = std::min(njobs, base);
