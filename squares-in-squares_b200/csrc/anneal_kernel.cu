@@ -746,11 +746,12 @@ __device__ long long quench_grp(const Grp& gp, const Rep& R, int n, const Grid& 
 }
 
 // Quench of replica view R by warps 0 .. gw - 1 of a group that starts at
-// thread t0 (all of them call this): one warp a 16 squares, at most gw.  More
-// warps than that add barrier latency and no parallelism (n = 10: one warp
-// against eight, with the phases above, took 400 checkpoints from 87 to 76 ms;
-// n = 50, 64 chains: 55.8 ms, 56.0 with 8 squares a warp, 61.1 with 32).
-constexpr int kQuenchSquares = 16;
+// thread t0 (all of them call this): one warp for 8 squares, at most gw.  More
+// warps than that add barrier latency and no parallelism.  400 checkpoints of
+// n = 10: 53.9 ms with 16 squares a warp, 51.8 with 8, 51.1 with 4; 16
+// replicas of n = 60: 16.6, 16.1, 16.6; n = 50 with 64 chains, whose groups
+// have 4 warps: 48.4 each.
+constexpr int kQuenchSquares = 8;
 __device__ __forceinline__ long long quench_group(int id, int gw, int t0, long long* red, const Rep& R, int n,
                                                   const Grid& g, float L, int iters, int stall_limit, float4* scr,
                                                   long long E) {
