@@ -366,16 +366,29 @@ __device__ __forceinline__ int decide_pair(const FSq* sq, const PairSq& ps, int 
     return lo > 0.0 ? -2 : 2;
 }
 
+// The warp's largest (or smallest) value among the lanes that have one, on
+// every lane: lanes drop out limb by limb, sign first, one warp reduction a
+// limb (five rounds of exchanging and comparing whole values took 20,000
+// cycles for the four extremes, most of it local memory).
 template <int F>
-__device__ void fix_shfl_min_max(Fix<F>& v, bool& have, bool want_min) {
-    for (int o = 16; o > 0; o >>= 1) {
-        Fix<F> w;
-        for (int i = 0; i <= F; ++i) w.d[i] = __shfl_xor_sync(0xffffffffu, v.d[i], o);
-        w.neg = __shfl_xor_sync(0xffffffffu, v.neg, o);
-        const bool wh = __shfl_xor_sync(0xffffffffu, (int)have, o) != 0;
-        if (wh && (!have || (want_min ? fx::cmp(w, v) < 0 : fx::cmp(w, v) > 0))) v = w;
-        have = have || wh;
+__device__ __forceinline__ bool warp_extreme(Fix<F>& v, bool have, bool want_min) {
+    if (!__any_sync(0xffffffffu, have)) return false;
+    const bool flip = (v.neg != 0) != want_min;  // larger magnitude is worse
+    bool in = have;
+    const uint32_t s = (v.neg != 0) == want_min ? 2u : 1u;  // the wanted sign first
+    const uint32_t best = __reduce_max_sync(0xffffffffu, in ? s : 0u);
+    in = in && s == best;
+#pragma unroll
+    for (int i = 0; i <= F; ++i) {
+        const uint32_t k = flip ? ~v.d[i] : v.d[i];
+        const uint32_t m = __reduce_max_sync(0xffffffffu, in ? k : 0u);
+        in = in && k == m;
     }
+    const int src = __ffs(__ballot_sync(0xffffffffu, in)) - 1;
+#pragma unroll
+    for (int i = 0; i <= F; ++i) v.d[i] = __shfl_sync(0xffffffffu, v.d[i], src);
+    v.neg = __shfl_sync(0xffffffffu, v.neg, src);
+    return true;
 }
 
 // One CTA per packing: checks, side measurement, sort and sweep.
@@ -406,7 +419,7 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
     __shared__ double box[W][4];
     __shared__ int s_cand;
     __shared__ Fix<9> ext[W][4];
-    __shared__ int ext_have[W];
+    __shared__ int ext_have[W][4];
     __shared__ Fix<9> org[2];
     __shared__ uint32_t s_err;
     __shared__ unsigned long long s_fkey;
@@ -543,12 +556,11 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
             idx[atomicAdd(&s_cand, 1)] = (int16_t)i;
     }
     __syncthreads();
-    Fix<9> mnx, mxx, mny, mxy;
-    fx::set_zero(mnx);
-    fx::set_zero(mxx);
-    fx::set_zero(mny);
-    fx::set_zero(mxy);
-    bool have = false;
+    Fix<9> ex[2];  // smallest and largest corner coordinate of this thread (an even one's x, an odd one's y)
+    fx::set_zero(ex[0]);
+    fx::set_zero(ex[1]);
+    bool have[2] = {false, false};
+    const double gext[4] = {gx0, gx1, gy0, gy1};
     const int ncand = s_cand;
     for (int base = 0; base < ncand; base += T / 2) {
         const int k = base + tid / 2;
@@ -560,53 +572,48 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
         int quad = 0;
         if (turned) fx::sincos_series(A, C.half_pi9, tid & 1, series[tid], quad);
         __syncwarp();
-        if (in && !(tid & 1)) {
+        if (in) {  // the even thread takes the x extremes, the odd one the y extremes
             Fix<9> hc = C.half9, hs;  // halves of cos and sin (an untilted square's are 1/2 and 0)
             fx::set_zero(hs);
             if (turned) {
                 Fix<9> sn, cs;
-                fx::sincos_quadrant(series[tid + 1], series[tid], quad, sn, cs);
+                fx::sincos_quadrant(series[tid | 1], series[tid & ~1], quad, sn, cs);
                 hc = fx::mul(C.half9, cs, 0);
                 hs = fx::mul(C.half9, sn, 0);
             }
-            const Fix<9> X = fx::sub<9, true>(fx::parse<9>(text, lits[3 * (s0 + i)], 0), org[0]);
-            const Fix<9> Y = fx::sub<9, true>(fx::parse<9>(text, lits[3 * (s0 + i) + 1], 0), org[1]);
-            const Fix<9> ux = fx::sub<9, true>(hc, hs), uy = fx::add<9, true>(hs, hc);
-            Fix<9> zero;
-            fx::set_zero(zero);
-            const Fix<9> vx = fx::sub<9, true>(zero, fx::add<9, true>(hc, hs)), vy = fx::sub<9, true>(hc, hs);
-            const Fix<9> px[4] = {fx::add<9, true>(X, ux), fx::add<9, true>(X, vx), fx::sub<9, true>(X, ux), fx::sub<9, true>(X, vx)};
-            const Fix<9> py[4] = {fx::add<9, true>(Y, uy), fx::add<9, true>(Y, vy), fx::sub<9, true>(Y, uy), fx::sub<9, true>(Y, vy)};
-            for (int c = 0; c < 4; ++c) {
-                if (!have) {
-                    mnx = mxx = px[c];
-                    mny = mxy = py[c];
-                    have = true;
-                    continue;
+            // corners: x + a, x - b, x - a, x + b and y + b, y + a, y - b, y - a
+            const Fix<9> a = fx::sub<9, true>(hc, hs), b = fx::add<9, true>(hs, hc);
+            const int ax = tid & 1;
+            const Fix<9> Z = fx::sub<9, true>(fx::parse<9>(text, lits[3 * (s0 + i) + ax], 0), org[ax]);
+            double cx[4], cy[4];
+            fcorners(sq[i], cx, cy);
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {  // only corners that can be the extreme
+                const double z = ax ? cy[c] : cx[c];
+                const bool lo = z <= gext[2 * ax] + 1e-8, hi = z >= gext[2 * ax + 1] - 1e-8;
+                if (!lo && !hi) continue;
+                Fix<9> off = (c & 1) == ax ? a : b;
+                if (ax ? c >= 2 : (c == 1 || c == 2)) off = fx::neg(off);
+                const Fix<9> v = fx::add<9, true>(Z, off);
+                if (lo && (!have[0] || fx::cmp<9, true>(v, ex[0]) < 0)) {
+                    ex[0] = v;
+                    have[0] = true;
                 }
-                if (fx::cmp<9, true>(px[c], mnx) < 0) mnx = px[c];
-                if (fx::cmp<9, true>(px[c], mxx) > 0) mxx = px[c];
-                if (fx::cmp<9, true>(py[c], mny) < 0) mny = py[c];
-                if (fx::cmp<9, true>(py[c], mxy) > 0) mxy = py[c];
+                if (hi && (!have[1] || fx::cmp<9, true>(v, ex[1]) > 0)) {
+                    ex[1] = v;
+                    have[1] = true;
+                }
             }
         }
         __syncwarp();
     }
-    if (__any_sync(0xffffffffu, have)) {
-        bool h0 = have, h1 = have, h2 = have, h3 = have;
-        fix_shfl_min_max(mnx, h0, true);
-        fix_shfl_min_max(mxx, h1, false);
-        fix_shfl_min_max(mny, h2, true);
-        fix_shfl_min_max(mxy, h3, false);
+    for (int k = 0; k < 4; ++k) {
+        Fix<9> v = ex[k & 1];
+        const bool got = warp_extreme(v, have[k & 1] && (tid & 1) == k / 2, (k & 1) == 0);
         if (lane == 0) {
-            ext[warp][0] = mnx;
-            ext[warp][1] = mxx;
-            ext[warp][2] = mny;
-            ext[warp][3] = mxy;
-            ext_have[warp] = 1;
+            ext_have[warp][k] = got;
+            if (got) ext[warp][k] = v;
         }
-    } else if (lane == 0) {
-        ext_have[warp] = 0;
     }
     __syncthreads();  // the candidates are read
     // 3. sort the AABBs by their padded min x, ties by square id
@@ -615,23 +622,17 @@ __global__ void __launch_bounds__(T, 512 / T) cert_packing_kernel(
         idx[i] = (int16_t)i;
     }
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0) {
         Fix<9> e[4];
-        bool any = false;
-        for (int w = 0; w < W; ++w) {
-            if (!ext_have[w]) continue;
-            if (!any) {
-                for (int k = 0; k < 4; ++k) e[k] = ext[w][k];
-                any = true;
-                continue;
-            }
-            if (fx::cmp(ext[w][0], e[0]) < 0) e[0] = ext[w][0];
-            if (fx::cmp(ext[w][1], e[1]) > 0) e[1] = ext[w][1];
-            if (fx::cmp(ext[w][2], e[2]) < 0) e[2] = ext[w][2];
-            if (fx::cmp(ext[w][3], e[3]) > 0) e[3] = ext[w][3];
+        for (int k = 0; k < 4; ++k) {
+            const bool own = lane < W && ext_have[lane][k];
+            e[k] = ext[own ? lane : 0][k];
+            warp_extreme(e[k], own, (k & 1) == 0);
         }
-        const Fix<9> sx = fx::sub(e[1], e[0]), sy = fx::sub(e[3], e[2]);
-        out[pk].side = fx::cmp(sx, sy) >= 0 ? sx : sy;
+        if (lane == 0) {
+            const Fix<9> sx = fx::sub(e[1], e[0]), sy = fx::sub(e[3], e[2]);
+            out[pk].side = fx::cmp(sx, sy) >= 0 ? sx : sy;
+        }
     }
     int np = 1;
     while (np < n) np <<= 1;
