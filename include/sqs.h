@@ -127,7 +127,7 @@ int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, const int64_
  * allocation once it runs.  No counterpart in the reference, which always
  * certifies on the CPU.  Same arguments, results and errors as
  * sqs_certify_batch, but it calls no cudaMalloc, cudaFree or other allocating
- * routine: all device scratch is one static array of about 7.6 MiB that
+ * routine: all device scratch is one static array of about 7.5 MiB that
  * every device loading the library holds until process exit, and host
  * staging is static too.  Limits per call: 4,096 packings, 16,384 squares,
  * 2 MiB of literal text (and, with SQS_CERT_ROUNDTRIP, literals under 4,096
@@ -210,12 +210,14 @@ typedef struct sqs_job {
 #define SQS_JOB_COLLECTIVE 4
 #define SQS_JOB_KICK 8
 /* Evaluate proposals strictly one at a time.  Without move-set options a
- * replica's warp evaluates two consecutive proposals at once, one per
- * half-warp, against the same state, and evaluates the second again when the
- * first was accepted and moved something the second read (the same square,
- * or a square or cell list inside its 3 x 3 cell block).  Energies are exact
- * integers, so the trajectory is the one-at-a-time trajectory bit for bit;
- * this flag changes only the time taken, and lets a caller check that. */
+ * replica's warp evaluates two or four consecutive proposals at once (grids of
+ * 4 x 4 and 6 x 6 cells on), each by a share of its lanes against the same
+ * state, and settles them up to the first that an accepted one before it
+ * touched (the same square, or a square or cell list inside its 3 x 3 cell
+ * block); replicas of up to 32 squares go one at a time from registers.
+ * Energies are exact integers, so the trajectory is the one-at-a-time
+ * trajectory bit for bit; this flag changes only the time taken, and lets a
+ * caller check that. */
 #define SQS_JOB_SERIAL 16
 /* Quench every replica, not only the coldest, at each exchange round: the
  * counterpart of the reference search's per-epoch gradient polish of every

@@ -1550,10 +1550,11 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
             __syncthreads();
         } else {
             // the replica on the coldest rung, by warps of the CTA that holds it; its scratch in shared memory after the replicas when
-            // the launch left room, else this CTA's block of the job's scratch
+            // the launch left room, else its first replica's block of the job's scratch
+            // (the other CTAs' replicas may be using theirs)
             float4* qs = (int64_t)dyn_bytes >= (int64_t)Rl * rb + (int64_t)sizeof(float4) * kQuenchScr * n
                              ? reinterpret_cast<float4*>(dyn + (int64_t)Rl * rb)
-                             : pos + jd.scr_off + (int64_t)rank * kQuenchScr * n;
+                             : pos + jd.scr_off + (int64_t)rank * Rl * kQuenchScr * n;
             int cold = 0;
             for (int q = 0; q < R; ++q)
                 if (S.jm.perm[q] == 0) cold = q;

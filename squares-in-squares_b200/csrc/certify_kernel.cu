@@ -265,8 +265,9 @@ __device__ __noinline__ int float_sat(const FSq& p, const FSq& q) {
 // certain to decide the same way:
 //   * separated when some axis's overlap lies strictly below zero,
 //     overlapping when every axis's lies strictly above: the exact overlap of
-//     the exact decimal inputs then has that sign and is at least 2^-60 in
-//     magnitude, which the 7-limb stage (widths below 1e-60) resolves alike;
+//     the exact decimal inputs then has that sign and is at least 2^-120 in
+//     magnitude (the spacing of the doubles involved), which the 7-limb stage
+//     (widths below 1e-60) resolves alike;
 //   * two axis-aligned squares (angle literals exactly zero, the reference's
 //     flat path) whose literals on an axis, and square 0's, are dyadic within
 //     25 decimal places are compared exactly on it: touching edges count as
@@ -1421,7 +1422,7 @@ constexpr size_t kSoOut = kSoLits + al256(sizeof(Lit) * 3 * kStaticMaxSquares);
 constexpr size_t kSoPa = kSoOut + al256(sizeof(PkOut) * kStaticMaxPackings);
 constexpr size_t kSoPb = kSoPa + al256(sizeof(Pair) * kStaticPairCap);
 constexpr size_t kSoCnt = kSoPb + al256(sizeof(Pair) * kStaticPairCap);
-constexpr size_t kStaticScratchBytes = kSoCnt + 256;  // about 7.6 MiB
+constexpr size_t kStaticScratchBytes = kSoCnt + 256;  // about 7.5 MiB
 
 // The scratch every call of sqs_certify_batch_static shares.  In host code
 // this name is only a stand-in: the device address comes from

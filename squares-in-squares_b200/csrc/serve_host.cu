@@ -320,6 +320,10 @@ extern "C" int sqs_server_create(sqs_ctx* ctx, size_t hbm_bytes, int max_active,
         e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
         if (e == cudaSuccess) e = cudaStreamDestroy(w.ctx->stream);
         if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&w.ctx->stream, cudaStreamNonBlocking, greatest);
+        for (cudaStream_t& a : w.ctx->aux) {  // the certifier's size classes run on these
+            if (e == cudaSuccess) e = cudaStreamDestroy(a);
+            if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&a, cudaStreamNonBlocking, greatest);
+        }
         if (e == cudaSuccess) e = cudaMalloc(&w.d_list, sizeof(int32_t) * (size_t)max_active);
         // Staging of the certifier, its interval cache and the rescue polish,
         // sized now: growing a buffer later frees the old one, which waits for
