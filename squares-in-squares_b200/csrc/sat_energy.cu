@@ -37,8 +37,8 @@ constexpr int kQueue = 256, kCtaQueue = 128;  // pair queue entries of a warp: w
 
 // Pair energies are summed as 64-bit integers in units of 2^-40: every term
 // is rounded once (error below 5e-13), the sum is exact, and 1024 squares'
-// pairs stay far below 2^23, so below 2^63 units.  The warp form sums its wall
-// terms the same way; the CTA form in double, in thread order.
+// pairs stay far below 2^23, so below 2^63 units.  Wall terms have no bound (a
+// square may lie anywhere), so they are summed in double, in thread order.
 constexpr double kEUnit = 1099511627776.0;  // 2^40
 __device__ __forceinline__ long long e_units(float e) { return __float2ll_rn(e * 1099511627776.0f); }
 
@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
     }
     __syncwarp();
     long long e_loc = 0;  // kEUnit units: exact, so the sum does not depend on the order of the pairs
+    double e_wall = 0.0;
     // Wall gradients wait in registers for the pair sums; with many squares a
     // lane there is no room, and they go straight out and are read back.
     constexpr bool kKeepWalls = NPL <= 2;
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
         if (i < n) {
             sincosf(pa[k], &ps[k], &pc[k]);
             float gx = 0.f, gy = 0.f, ga = 0.f;
-            e_loc += e_units(wall_energy_grad(px[k], py[k], pc[k], ps[k], L, gx, gy, ga));
+            e_wall += (double)wall_energy_grad(px[k], py[k], pc[k], ps[k], L, gx, gy, ga);
             // (kept apart from the pair sums: unbounded for squares far outside the box)
             if (kKeepWalls) {
                 wx[k % (kKeepWalls ? NPL : 1)] = gx;
@@ -533,8 +534,9 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
     // 4. reductions and the gradient store
     e_loc = warp_sum_units(e_loc);
     if (COUNT) cand_loc = __reduce_add_sync(0xffffffffu, cand_loc);
+    for (int o = 16; o > 0; o >>= 1) e_wall += __shfl_xor_sync(0xffffffffu, e_wall, o);
     if (lane == 0) {
-        energy[cfg] = (float)((double)e_loc * (1.0 / kEUnit));
+        energy[cfg] = (float)(e_wall + (double)e_loc * (1.0 / kEUnit));
         if (COUNT) cand[cfg] = cand_loc;
     }
     if (!gdst) return;

@@ -75,3 +75,22 @@ def test_proposal_forms_equal_one_at_a_time(ctx, n):
         for key in ("xya", "energy", "energy_full", "rung"):
             np.testing.assert_array_equal(a["trace"][key], b["trace"][key], err_msg=key)
         np.testing.assert_array_equal(a["trace"]["energy"], a["trace"]["energy_full"])
+
+
+@pytest.mark.parametrize("n", [2, 33, 65, 256, 257, 1000])
+@pytest.mark.parametrize("stray", [1, 2, 5])
+def test_sat_energy_of_squares_far_outside(ctx, oracle, n, stray):
+    """Wall terms have no bound: squares 1e4 outside the box (1e8 of energy
+    each) within the same tolerances as any others."""
+    from sqs import sat
+    from sqs.workloads import sat_microbench
+
+    stray = min(stray, n)
+    x, L = sat_microbench(configs=3, n=n, seed=900 + n)
+    x[:, :stray, :2] += [[9.0e3, -1.1e4]]
+    x32, L32 = x.astype(np.float32), L.astype(np.float32)
+    e, g, _ = sat.energy(x32, L32, ctx=ctx, grad=True)
+    eo, go, _ = oracle.total_batch(x32.astype(np.float64), L32.astype(np.float64))
+    np.testing.assert_allclose(e, eo, rtol=1e-5)
+    off = np.abs(g - go) - 1e-4 * (1 + np.abs(go))
+    assert np.mean(off > 0) <= 2e-3
