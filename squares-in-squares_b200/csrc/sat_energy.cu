@@ -35,20 +35,32 @@ constexpr int kSatMaxN = 1024;
 constexpr float kCellMin = 1.41422f;  // > sqrt(2.000001) = 1.4142139
 constexpr int kQueue = 256, kCtaQueue = 128;  // pair queue entries of a warp: warp form, CTA form
 
-// Pair energies are summed as 64-bit integers in units of 2^-40: every term
-// is rounded once (error below 5e-13), the sum is exact, and 1024 squares'
-// pairs stay far below 2^23, so below 2^63 units.  Wall terms have no bound (a
-// square may lie anywhere), so they are summed in double, in thread order.
-constexpr double kEUnit = 1099511627776.0;  // 2^40
-__device__ __forceinline__ long long e_units(float e) { return __float2ll_rn(e * 1099511627776.0f); }
+// Pair energies are summed as integers in units of 2^-48.  A gap below zero is
+// the difference of two floats of at least 1/2, or lies below -1/2 itself: a
+// multiple of 2^-24 either way, so its square is a whole number of units and
+// nothing is lost down to the smallest overlap (in units of 2^-40 a gap below
+// 7e-7 vanished).  A term is below 1.46 * 2^48, and pairs go to the lanes in turn, at
+// most 16,384 to one (half a million pairs, all taken by one warp), so a lane's
+// sum stays below 2^63.  Wall terms have no bound (a square may lie anywhere), so
+// they are summed in double, in thread order.
+constexpr float kEnergyUnits = 281474976710656.0f;  // 2^48
+__device__ __forceinline__ long long e_units(float e) { return __float2ll_rn(e * kEnergyUnits); }
 
-// Exact 64-bit warp sum: the 26 low bits, the next 26 and the signed rest
-// each sum within 32 bits.
-__device__ __forceinline__ long long warp_sum_units(long long v) {
+// Exact sum past 64 bits: hi * 2^52 + lo with 0 <= lo < 2^52, one form for each
+// value, so converting it does not depend on how the terms were dealt out.
+struct EnergySum {
+    long long hi, lo;
+    __device__ __forceinline__ EnergySum(long long h, long long l) : hi(h + (l >> 52)), lo(l & ((1ll << 52) - 1)) {}
+    __device__ __forceinline__ double value() const { return (double)hi * 0x1p4 + (double)lo * 0x1p-48; }
+};
+
+// Warp sum: the 26 low bits, the next 26 and the signed rest each sum within
+// 32 bits.
+__device__ __forceinline__ EnergySum warp_sum_units(long long v) {
     const unsigned s0 = __reduce_add_sync(0xffffffffu, (unsigned)v & 0x3ffffffu);
     const unsigned s1 = __reduce_add_sync(0xffffffffu, (unsigned)(v >> 26) & 0x3ffffffu);
     const int s2 = __reduce_add_sync(0xffffffffu, (int)(v >> 52));
-    return (long long)(((unsigned long long)(long long)s2 << 52) + ((unsigned long long)s1 << 26) + s0);
+    return EnergySum(s2, (long long)(((unsigned long long)s1 << 26) + s0));
 }
 
 // Nearest integer (ties to even) of |x| < 2^22 on the FMA pipe: x + 1.5 * 2^23
@@ -90,7 +102,7 @@ __host__ __device__ inline size_t sat_smem_bytes(int n, int threads) {
     b += (size_t)(threads / 32) * kCtaQueue * 4;  // warp pair queues
     b += ((size_t)(G * G + 1) * 2 + 3) & ~(size_t)3;  // cell counts / starts
     b += (size_t)n * 4;                       // sorted -> (original index, cell)
-    b += 8 + (size_t)(threads / 32) * 24;     // reduction scratch
+    b += 8 + (size_t)(threads / 32) * 32;     // reduction scratch
     return (b + 15) & ~(size_t)15;
 }
 
@@ -304,24 +316,26 @@ __global__ void __launch_bounds__(T, T == 256 ? 4 : 1) sat_energy_kernel(int n, 
     __syncthreads();
 
     // 4. reductions and stores
-    e_loc = warp_sum_units(e_loc);
+    const EnergySum e_warp = warp_sum_units(e_loc);
     cand_loc = __reduce_add_sync(0xffffffffu, cand_loc);
     for (int o = 16; o > 0; o >>= 1) e_wall += __shfl_xor_sync(0xffffffffu, e_wall, o);
     if (lane == 0) {
-        red[3 * warp] = e_loc;
-        red[3 * warp + 1] = cand_loc;
-        red[3 * warp + 2] = __double_as_longlong(e_wall);
+        red[4 * warp] = e_warp.hi;
+        red[4 * warp + 1] = e_warp.lo;
+        red[4 * warp + 2] = cand_loc;
+        red[4 * warp + 3] = __double_as_longlong(e_wall);
     }
     __syncthreads();
     if (tid == 0) {
-        long long e = 0, cc = 0;
+        long long hi = 0, lo = 0, cc = 0;
         double walls = 0.0;
         for (int w = 0; w < W; ++w) {
-            e += red[3 * w];
-            cc += red[3 * w + 1];
-            walls += __longlong_as_double(red[3 * w + 2]);
+            hi += red[4 * w];
+            lo += red[4 * w + 1];
+            cc += red[4 * w + 2];
+            walls += __longlong_as_double(red[4 * w + 3]);
         }
-        energy[cfg] = (float)(walls + (double)e * (1.0 / kEUnit));
+        energy[cfg] = (float)(walls + EnergySum(hi, lo).value());
         if (cand) cand[cfg] = (uint32_t)cc;
     }
     if (grad) {
@@ -416,7 +430,7 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
         }
     }
     __syncwarp();
-    long long e_loc = 0;  // kEUnit units: exact, so the sum does not depend on the order of the pairs
+    long long e_loc = 0;  // exact, so the sum does not depend on the order of the pairs
     double e_wall = 0.0;
     // Wall gradients wait in registers for the pair sums; with many squares a
     // lane there is no room, and they go straight out and are read back.
@@ -532,11 +546,11 @@ __global__ void __launch_bounds__(W * 32, 28 / W) sat_energy_warp_kernel(int con
     __syncwarp();
 
     // 4. reductions and the gradient store
-    e_loc = warp_sum_units(e_loc);
+    const EnergySum e_sum = warp_sum_units(e_loc);
     if (COUNT) cand_loc = __reduce_add_sync(0xffffffffu, cand_loc);
     for (int o = 16; o > 0; o >>= 1) e_wall += __shfl_xor_sync(0xffffffffu, e_wall, o);
     if (lane == 0) {
-        energy[cfg] = (float)(e_wall + (double)e_loc * (1.0 / kEUnit));
+        energy[cfg] = (float)(e_wall + e_sum.value());
         if (COUNT) cand[cfg] = cand_loc;
     }
     if (!gdst) return;

@@ -94,3 +94,19 @@ def test_sat_energy_of_squares_far_outside(ctx, oracle, n, stray):
     np.testing.assert_allclose(e, eo, rtol=1e-5)
     off = np.abs(g - go) - 1e-4 * (1 + np.abs(go))
     assert np.mean(off > 0) <= 2e-3
+
+
+@pytest.mark.parametrize("n", [2, 33, 256, 257, 512, 1024])
+def test_sat_energy_of_the_smallest_overlaps(ctx, n):
+    """One pair overlapping by 2^-22 .. 2^-18 in an otherwise separated lattice:
+    every value is exact in FP32, so the energy is the overlap's square."""
+    from sqs import sat
+
+    gaps = [2.0 ** -k for k in range(18, 23)]
+    x = np.zeros((len(gaps), n, 3))
+    i = np.arange(n)
+    x[:, :, 0], x[:, :, 1] = 1.0 + 1.25 * (i % 32), 1.0 + 1.25 * (i // 32)
+    for k, gap in enumerate(gaps):
+        x[k, 0, 0] = x[k, 1, 0] - 1.0 + gap
+    e, _, _ = sat.energy(x.astype(np.float32), np.float32(48.0), ctx=ctx)
+    np.testing.assert_array_equal(e, [np.float32(gap * gap) for gap in gaps])
