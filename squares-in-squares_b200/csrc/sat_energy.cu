@@ -168,20 +168,21 @@ __device__ __forceinline__ void broad_phase(const float2* sxy, int p, float px, 
     }
 }
 
-// One CTA per configuration.  n = 999 holds 54 KB of shared memory, so four
-// CTAs of 256 threads share an SM.  The form before kept an original-order copy
-// of the squares and the wall gradients there and summed energies in float,
-// for which every cell was sorted: 76 KB, eight warps an SM, 243 us at
-// 1,500 x 999 against 88.6 (queues of 64 or 256 pairs a warp: 96 us, the one
-// for its rounds, the other for a CTA less an SM; 512 threads: 97 us).
-template <int T>
+// One CTA per configuration, a thread's squares (at most NPT) in registers from
+// the load to the scatter.  n = 999 holds 52 KB of shared memory, so four CTAs
+// of 256 threads share an SM.  The form before kept an original-order copy of
+// the squares and the wall gradients there and summed energies in float, for
+// which every cell was sorted: 76 KB, eight warps an SM, 243 us at 1,500 x 999
+// against 88.6 (queues of 64 or 256 pairs a warp: 96 us, the one for its
+// rounds, the other for a CTA less an SM; 512 threads: 97 us).
+template <int T, int NPT>
 __global__ void __launch_bounds__(T, T == 256 ? 4 : 1) sat_energy_kernel(int n, const float* __restrict__ xya,
                                                         const float* __restrict__ side,
                                                         float* __restrict__ energy,
                                                         float* __restrict__ grad,
                                                         uint32_t* __restrict__ cand) {
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int W = T / 32, NPT = kSatMaxN / T;
+    constexpr int W = T / 32;
     const int cfg = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int Gcap = sat_grid_cap(n);
@@ -611,18 +612,25 @@ static int launch_warp(sqs_ctx* ctx, cudaStream_t st, int configs, int n, const 
     }
 }
 
-template <int T>
+// The CTA form at T threads, in the instance with the squares a thread has,
+// rounded up to a power of two.  One instance for 1024 / T squares a thread at
+// every n cost registers and unrolled rounds that small configurations have no
+// use for (255 at 32 threads): 8,192 x 17 at 32 threads took 61.8 us against
+// 14.7 now, 4,096 x 200 at 64 threads 90.6 against 53.3.
+template <int T, int NPT = 1>
 static int launch(sqs_ctx* ctx, cudaStream_t st, int configs, int n, const float* xya, const float* side,
                   float* energy, float* grad, uint32_t* cand) {
+    if constexpr (T * NPT < kSatMaxN)
+        if (n > T * NPT) return launch<T, 2 * NPT>(ctx, st, configs, n, xya, side, energy, grad, cand);
     const size_t smem = sat_smem_bytes(n, T);
     static bool attr_set[64] = {false};
     const int dev = ctx->device & 63;
     if (!attr_set[dev]) {
-        SQS_CUDA(cudaFuncSetAttribute(sat_energy_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        SQS_CUDA(cudaFuncSetAttribute(sat_energy_kernel<T, NPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       96 * 1024));
         attr_set[dev] = true;
     }
-    sat_energy_kernel<T><<<configs, T, smem, st>>>(n, xya, side, energy, grad, cand);
+    sat_energy_kernel<T, NPT><<<configs, T, smem, st>>>(n, xya, side, energy, grad, cand);
     SQS_CUDA(cudaGetLastError());
     ctx->launches += 1;
     return SQS_OK;

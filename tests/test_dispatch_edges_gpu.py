@@ -110,3 +110,62 @@ def test_sat_energy_of_the_smallest_overlaps(ctx, n):
         x[k, 0, 0] = x[k, 1, 0] - 1.0 + gap
     e, _, _ = sat.energy(x.astype(np.float32), np.float32(48.0), ctx=ctx)
     np.testing.assert_array_equal(e, [np.float32(gap * gap) for gap in gaps])
+
+
+def _device_batch(ctx, x32, L32):
+    from sqs import sat
+
+    configs, n, _ = x32.shape
+    bufs = [ctx.alloc(x32.shape, np.float32).upload(x32), ctx.alloc((configs,), np.float32).upload(L32),
+            ctx.alloc((configs,), np.float32), ctx.alloc(x32.shape, np.float32), ctx.alloc((configs,), np.uint32)]
+    return bufs, lambda threads: sat.energy_device(ctx, configs, n, *bufs, threads=threads)
+
+
+@pytest.mark.parametrize("threads", [32, 64, 128, 256])
+def test_cta_form_at_squares_a_thread(ctx, oracle, threads):
+    """Every CTA width at the sizes where the squares a thread holds change
+    their bound, 1 to 1024 squares."""
+    from sqs.workloads import sat_microbench
+
+    edges = {1, 2, 1023, 1024}
+    npt = 1
+    while threads * npt < 1024:
+        edges |= {threads * npt - 1, threads * npt, threads * npt + 1}
+        npt *= 2
+    for n in sorted(edges):
+        x, L = sat_microbench(configs=2, n=n, seed=n)
+        x32, L32 = x.astype(np.float32), L.astype(np.float32)
+        bufs, run = _device_batch(ctx, x32, L32)
+        run(threads)
+        e, g, c = (b.download() for b in bufs[2:])
+        for b in bufs:
+            b.free()
+        eo, go, co = oracle.total_batch(x32.astype(np.float64), L32.astype(np.float64))
+        np.testing.assert_allclose(e, eo, rtol=1e-5, atol=1e-6)
+        assert np.all(np.abs(c.astype(np.int64) - co) <= np.maximum(1, 1e-5 * co))
+        off = np.abs(g - go) - 1e-4 * (1 + np.abs(go))
+        assert np.mean(off > 0) <= 2e-3
+
+
+def test_narrow_ctas_pay_off_for_small_configurations(ctx):
+    """8,192 configurations of 17 squares leave all but one warp of a wide CTA
+    without work, so CTAs of 32 threads take well under the time of 256."""
+    import time
+
+    from sqs.workloads import sat_microbench
+
+    x, L = sat_microbench(configs=8192, n=17, seed=1)
+    bufs, run = _device_batch(ctx, x.astype(np.float32), L.astype(np.float32))
+    took = {32: [], 256: []}
+    for _ in range(7):
+        for threads, ts in took.items():
+            run(threads)
+            ctx.sync()
+            t0 = time.perf_counter()
+            for _ in range(50):
+                run(threads)
+            ctx.sync()
+            ts.append(time.perf_counter() - t0)
+    for b in bufs:
+        b.free()
+    assert min(took[32]) < 0.7 * min(took[256]), took
