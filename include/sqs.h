@@ -114,7 +114,10 @@ typedef struct sqs_verdict {
  * Every verdict, reason, score and 50-decimal side equals the reference
  * certifier's evaluate_single_puzzle (certifier.cpp:738-912) on the same
  * strings; SQS_CERT_ROUNDTRIP applies its --roundtrip literal transform
- * (certifier.cpp:914-929, main :1002-1006) first.  Replaces the `certifier`
+ * (certifier.cpp:914-929, main :1002-1006) first.  A call holds up to 2^30
+ * squares, whose literals start within the first 4 GiB (less 1 MiB) of the
+ * text, as given or round-tripped; larger calls fail with SQS_EINVAL and are
+ * split by the caller.  Replaces the `certifier`
  * process (certifier.cpp:933-1077) and the Python gate core.certify /
  * core.evaluate (core.py:52-62) for whole batches. */
 int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, const int64_t* row_start,

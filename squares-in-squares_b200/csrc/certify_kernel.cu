@@ -69,6 +69,9 @@ struct SqText {
     uint32_t off, len[3];
 };
 constexpr uint32_t kLenMax = 1u << 20;  // a longer literal is read as far as this
+// The offsets have 32 bits, so the last literal a square's record names must
+// start here at the latest; calls with more text are refused.
+constexpr int64_t kOffMax = (1ll << 32) - kLenMax;
 
 struct Consts {
     Fix<9> half_pi9, two_pi9, half9;
@@ -1202,7 +1205,7 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
         for (++t; t <= nt; ++t) p_lo[(size_t)t] = count;
     }
     std::vector<std::string> rt((size_t)nt);  // round-tripped text of each thread's packings
-    std::vector<int64_t> bad_row((size_t)nt, -1);
+    std::vector<int64_t> bad_row((size_t)nt, -1), far_row((size_t)nt, -1);
     // A large literal text is staged in pinned memory too, each thread copying
     // the span of its own packings (the first from offset 0), so that it
     // uploads at the full host-link rate.
@@ -1240,9 +1243,10 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
                 const int64_t r = row_of[(size_t)i];
                 SqText& q = raw[pk_sq0[(size_t)p] + i];
                 q.off = (uint32_t)(do_rt ? (int64_t)rt[(size_t)t].size() : lit_off[3 * r]);
+                if (!do_rt && lit_off[3 * r + 2] > kOffMax) far_row[(size_t)t] = r;
                 for (int k = 0; k < 3; ++k) {
                     const int64_t a = lit_off[3 * r + k], b = lit_off[3 * r + k + 1];
-                    if (b < a) {
+                    if (a < 0 || b < a || (size_t)b > text_bytes) {
                         bad_row[(size_t)t] = r;
                         return;
                     }
@@ -1251,7 +1255,7 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
                         q.len[k] = (uint32_t)s2.size();
                         rt[(size_t)t] += s2;
                     } else {
-                        q.len[k] = (uint32_t)(b - a);
+                        q.len[k] = (uint32_t)std::min<int64_t>(b - a, UINT32_MAX);
                     }
                 }
             }
@@ -1265,10 +1269,16 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
         for (auto& th : pool) th.join();
     }
     for (int t = 0; t < nt; ++t)
-        SQS_REQUIRE(bad_row[(size_t)t] < 0, "literal offsets not monotone at row %lld", (long long)bad_row[(size_t)t]);
+        SQS_REQUIRE(bad_row[(size_t)t] < 0, "literal offsets not monotone, or outside the text, at row %lld",
+                    (long long)bad_row[(size_t)t]);
+    for (int t = 0; t < nt; ++t)
+        SQS_REQUIRE(far_row[(size_t)t] < 0, "literals of row %lld lie past 4 GiB of text (split the call)",
+                    (long long)far_row[(size_t)t]);
     std::string rt_text;  // round-tripped literals, when requested
     if (do_rt) {
-        size_t base = 0;
+        size_t base = 0, rt_bytes = 0;
+        for (const std::string& part : rt) rt_bytes += part.size();
+        SQS_REQUIRE((int64_t)rt_bytes <= kOffMax, "round-tripped literals past 4 GiB of text (split the call)");
         for (int t = 0; t < nt; ++t) {
             if (base)
                 for (int p = p_lo[(size_t)t]; p < p_lo[(size_t)t + 1]; ++p) {
@@ -1521,6 +1531,9 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
     const int dev = ctx->device & 63;
     const bool do_rt = (flags & SQS_CERT_ROUNDTRIP) != 0;
     // envelope checks and literal slices, as sqs_certify_batch does them
+    const int64_t text_end = lit_off[3 * row_start[count]];
+    SQS_REQUIRE(do_rt || text_end <= (int64_t)kStaticMaxText, "literals exceed %zu bytes (static certifier limit)",
+                kStaticMaxText);
     int64_t S = 0;
     size_t rt_used = 0;
     for (int p = 0; p < count; ++p) {
@@ -1559,7 +1572,8 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
             q.off = (uint32_t)(do_rt ? (int64_t)rt_used : lit_off[3 * r]);
             for (int k = 0; k < 3; ++k) {
                 const int64_t a = lit_off[3 * r + k], b = lit_off[3 * r + k + 1];
-                SQS_REQUIRE(b >= a, "literal offsets not monotone at row %lld", (long long)r);
+                SQS_REQUIRE(a >= 0 && b >= a && b <= text_end, "literal offsets not monotone, or outside the text, at row %lld",
+                            (long long)r);
                 if (do_rt) {
                     SQS_REQUIRE((size_t)(b - a) < sizeof(s_lit_tmp), "literal longer than %zu bytes",
                                 sizeof(s_lit_tmp) - 1);
@@ -1578,8 +1592,7 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
         }
         S += n;
     }
-    const size_t text_bytes = do_rt ? rt_used : (size_t)lit_off[3 * row_start[count]];
-    SQS_REQUIRE(text_bytes <= kStaticMaxText, "literals exceed %zu bytes (static certifier limit)", kStaticMaxText);
+    const size_t text_bytes = do_rt ? rt_used : (size_t)text_end;
     int nb[3] = {0, 0, 0};
     for (int p = 0; p < count; ++p)
         if (s_live[p]) ++nb[s_pk_n[p] <= 64 ? 0 : (s_pk_n[p] <= 256 ? 1 : 2)];

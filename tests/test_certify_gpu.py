@@ -211,3 +211,42 @@ def test_pair_decision_matches_oracle(ctx, oracle, kind):
     for p in range(len(items)):
         assert (int(out[p].ok), float(out[p].score), out[p].L.decode(), out[p].reason.decode()) == \
             (int(ok[p]), float(score[p]), sides[p], reasons[p])
+
+
+@pytest.mark.parametrize("entry", ["sqs_certify_batch", "sqs_certify_batch_static"])
+def test_literals_past_4_gib_are_refused(ctx, entry):
+    """Literal offsets are kept in 32 bits: a packing whose literals lie past
+    that is refused, never measured by the digits at the wrapped offset.  The
+    text is sparse: separated squares at offset 0, in a packing refused for its
+    row count, whose last literal reaches to 2^32, where overlapping ones follow."""
+    import ctypes as C
+
+    import numpy as np
+
+    from sqs import SQSError
+    from sqs import _native as N
+
+    far = 2 ** 32
+    decoy, real = b"0.5" b"0.5" b"0" b"2.5" b"0.5" b"0", b"0.5" b"0.5" b"0" b"0.6" b"0.5" b"0"
+    text = np.zeros(far + 4096, np.uint8)
+    text[:len(decoy)] = np.frombuffer(decoy, np.uint8)
+    text[far:far + len(real)] = np.frombuffer(real, np.uint8)
+    n_of, row_start = np.array([2, 2], np.int32), np.array([0, 1, 3], np.int64)
+    lit_off = np.array([0, 3, 6, far, far + 3, far + 6, far + 7, far + 10, far + 13, far + 14], np.int64)
+    out = (N.Verdict * 2)()
+    with pytest.raises(SQSError):
+        N.check(getattr(N.lib(), entry)(ctx.handle, 2, n_of.ctypes.data, row_start.ctypes.data, None,
+                                        C.cast(text.ctypes.data, C.c_char_p), lit_off.ctypes.data, 0, out))
+
+
+def test_literal_offsets_outside_the_text_are_refused(ctx):
+    """A row whose literals end past the text the call names, or start before
+    it, is refused before anything reads them."""
+    import numpy as np
+
+    from sqs import SQSError, core
+
+    text = b"0.50.50" + b" " * 64
+    for off in ([0, 3, 6, 90, 7, 7, 7], [-9, 3, 6, 7, 7, 7, 7]):
+        with pytest.raises(SQSError):
+            core.certify_arrays(np.array([1, 2], np.int32), np.array([0, 1, 2]), None, text, np.array(off), ctx=ctx)
