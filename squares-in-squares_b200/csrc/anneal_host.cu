@@ -76,7 +76,7 @@ void put(char* dst, size_t cap, const std::string& s) {
 int prepare_job(const sqs_job& J, int j, JobDev& d, JobMut& m, Plan& p, const Shape* shape) {
     SQS_REQUIRE(J.n >= 1 && J.n <= kMaxN, "job %d: n=%d out of 1..%d", j, J.n, kMaxN);
     SQS_REQUIRE(J.replicas >= 1 && J.replicas <= kMaxR, "job %d: replicas=%d out of 1..%d", j, J.replicas, kMaxR);
-    SQS_REQUIRE(J.sweeps >= -2000000000 && J.sweeps <= 100000000, "job %d: sweeps=%d out of range", j, J.sweeps);
+    SQS_REQUIRE(J.sweeps >= -2000000000 && J.sweeps <= kMaxSweeps, "job %d: sweeps=%d out of range", j, J.sweeps);
     SQS_REQUIRE(J.exchange_every != 0 && J.exchange_every >= -1000000000,
                 "job %d: exchange_every must be nonzero (sweeps, or -proposals)", j);
     const int ladders = std::max(1, (J.flags >> 20) & 0xf);

@@ -1508,6 +1508,10 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                         ++q;
                     }
                 }
+                if (accs >= kCountFlush) {
+                    atomicAdd(reinterpret_cast<unsigned long long*>(&jmut[job].accepted), (unsigned long long)accs);
+                    accs = 0;
+                }
             }
             if (small) build_cells(rep, n, g, lane);  // every cell within its capacity
             if (!MOVES) {
@@ -1742,7 +1746,7 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
 
     // ---- write the slice back
     if (active) {
-        const long long accs_all = warp_sum_ll(accs);
+        const long long accs_all = warp_sum_ll((long long)accs);
         const int ovf_all = __reduce_add_sync(0xffffffffu, ovf);
         float4* dst = pos + jd.pos_off + (int64_t)r * n;
         for (int i = lane; i < n; i += 32) dst[i] = make_float4(rep.sq[i].x, rep.sq[i].y, rep.ang[i], 0.f);

@@ -145,3 +145,19 @@ def test_paired_proposals_equal_one_at_a_time(ctx):
     other = anneal_batch([plain_job(seed=52, polish_iters=20, cluster=4, **cases[2])], ctx=ctx)[0]
     for key in KEYS:
         assert other[key] == alone_serial[2][key], key
+
+
+@pytest.mark.parametrize("n,serial", [(10, False), (60, False), (60, True), (150, False)])
+def test_accepted_count_does_not_depend_on_slices(ctx, n, serial):
+    """A lane hands its count of acceptances over as it grows (thousands of
+    times below 2^32): the total of one long launch equals that of launches
+    too short to hand anything over."""
+    from sqs.anneal import AnnealJob, anneal_batch, jittered_grid
+
+    xya, side = jittered_grid(n, seed=n)
+    job = AnnealJob(xya, L0=side, replicas=4, sweeps=60000 // n, exchange_every=10, tmin=1.0, tmax=10.0, seed=n,
+                    serial=serial, polish_iters=0)
+    whole = anneal_batch([job], ctx=ctx)[0]
+    sliced = anneal_batch([job], ctx=ctx, slice_sweeps=2000 // n)[0]
+    assert whole["proposals"] == 4 * n * (60000 // n)
+    assert whole["accepted"] == sliced["accepted"] > 4 * 20000
