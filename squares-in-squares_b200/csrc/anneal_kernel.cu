@@ -50,6 +50,12 @@ constexpr float kHalfPiF = 1.57079632679489662f;
 // the angle itself.
 __device__ __forceinline__ void state_trig(float a, float* s, float* c) { sincosf(a, s, c); }
 
+// An angle into [0, pi/2), in one rounding wherever it is compiled in.
+__device__ __forceinline__ float wrap_quarter_f(float a) {
+    a = __fmaf_rn(-kHalfPiF, floorf(__fmul_rn(a, 1.0f / kHalfPiF)), a);
+    return (a >= 0.f && a < kHalfPiF) ? a : 0.f;
+}
+
 struct Rep {  // one replica's shared-memory view
     float4* sq;        // (x, y, cos a, sin a)
     float* ang;        // a in [0, pi/2)
@@ -695,9 +701,7 @@ __device__ long long quench_grp(const Grp& gp, const Rep& R, int n, const Grid& 
                 const float4 o = saved[i];
                 const float sx = fminf(0.1f, fmaxf(-0.1f, alpha * d.x));
                 const float sy = fminf(0.1f, fmaxf(-0.1f, alpha * d.y));
-                float a = o.z + fminf(0.1f, fmaxf(-0.1f, alpha * d.z));
-                a = a - kHalfPiF * floorf(a * (1.0f / kHalfPiF));
-                if (!(a >= 0.f && a < kHalfPiF)) a = 0.f;
+                const float a = wrap_quarter_f(o.z + fminf(0.1f, fmaxf(-0.1f, alpha * d.z)));
                 float sn, cs;
                 state_trig(a, &sn, &cs);
                 const float nx = o.x + sx, ny = o.y + sy;
@@ -759,11 +763,6 @@ __device__ __forceinline__ long long quench_group(int id, int gw, int t0, long l
     if (t >= 32 * nw) return E;
     if (nw == 1) return quench_grp(WarpGrp{t}, R, n, g, L, iters, stall_limit, scr, E);
     return quench_grp(BarGrp{id, nw, t0, red}, R, n, g, L, iters, stall_limit, scr, E);
-}
-
-__device__ __forceinline__ float wrap_quarter_f(float a) {
-    a = a - kHalfPiF * floorf(a * (1.0f / kHalfPiF));
-    return (a >= 0.f && a < kHalfPiF) ? a : 0.f;
 }
 
 // Pair list of a warp's replica for collective moves: every pair closer than
@@ -1279,9 +1278,7 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
                     // further than the clamped step (it may start outside)
                     tx = fminf(fmaxf(P.x, Lr - 0.5f), fmaxf(fminf(P.x, 0.5f), P.x + dx));
                     ty = fminf(fmaxf(P.y, Lr - 0.5f), fmaxf(fminf(P.y, 0.5f), P.y + dy));
-                    ta = rep.ang[i] + da;
-                    ta = ta - kHalfPiF * floorf(ta * (1.0f / kHalfPiF));
-                    if (!(ta >= 0.f && ta < kHalfPiF)) ta = 0.f;
+                    ta = wrap_quarter_f(__fadd_rn(rep.ang[i], da));
                     state_trig(ta, &ts, &tc);
                     tw = qe(wall_e(tx, ty, tc, ts, Lr)) - qe(wall_e(P.x, P.y, P.z, P.w, Lr));
                     tcells = pack_cells(g.cx(P.x), g.cx(P.y), g.cx(tx), g.cx(ty));

@@ -136,6 +136,9 @@ __device__ __forceinline__ float sat_pair_energy(float dx, float dy, float cp, f
 // Wall penalty of one square in [0, L]^2 (reference seeded.cu:96-113 with the
 // dr_smooth angle derivative, seeded.cu:36-38): sum over the four sides of
 // max(0, violation)^2 where the square's half-extent is r = (|c| + |s|) / 2.
+// Every rounding is spelled out, as for the pairs: the energy and the gradient
+// are compiled into several kernels and group widths whose sums must agree bit
+// for bit.  (Halving, doubling and products with 0 and +-1 are exact.)
 __device__ __forceinline__ float wall_energy_grad(float x, float y, float c, float s, float L,
                                                   float& gx, float& gy, float& ga) {
     const float r = 0.5f * (fabsf(c) + fabsf(s));
@@ -144,10 +147,10 @@ __device__ __forceinline__ float wall_energy_grad(float x, float y, float c, flo
     const float dr = 0.5f * (-sc * s + ss * c);
     float e = 0.f;
     const float v0 = r - x, v1 = x + r - L, v2 = r - y, v3 = y + r - L;
-    if (v0 > 0.f) { e += v0 * v0; gx -= 2.f * v0; ga += 2.f * v0 * dr; }
-    if (v1 > 0.f) { e += v1 * v1; gx += 2.f * v1; ga += 2.f * v1 * dr; }
-    if (v2 > 0.f) { e += v2 * v2; gy -= 2.f * v2; ga += 2.f * v2 * dr; }
-    if (v3 > 0.f) { e += v3 * v3; gy += 2.f * v3; ga += 2.f * v3 * dr; }
+    if (v0 > 0.f) { e = __fmaf_rn(v0, v0, e); gx -= 2.f * v0; ga = __fmaf_rn(2.f * v0, dr, ga); }
+    if (v1 > 0.f) { e = __fmaf_rn(v1, v1, e); gx += 2.f * v1; ga = __fmaf_rn(2.f * v1, dr, ga); }
+    if (v2 > 0.f) { e = __fmaf_rn(v2, v2, e); gy -= 2.f * v2; ga = __fmaf_rn(2.f * v2, dr, ga); }
+    if (v3 > 0.f) { e = __fmaf_rn(v3, v3, e); gy += 2.f * v3; ga = __fmaf_rn(2.f * v3, dr, ga); }
     return e;
 }
 
@@ -155,7 +158,7 @@ __device__ __forceinline__ float wall_energy(float x, float y, float c, float s,
     const float r = 0.5f * (fabsf(c) + fabsf(s));
     const float v0 = fmaxf(0.f, r - x), v1 = fmaxf(0.f, x + r - L);
     const float v2 = fmaxf(0.f, r - y), v3 = fmaxf(0.f, y + r - L);
-    return v0 * v0 + v1 * v1 + v2 * v2 + v3 * v3;
+    return __fmaf_rn(v3, v3, __fmaf_rn(v2, v2, __fmaf_rn(v0, v0, __fmul_rn(v1, v1))));
 }
 
 }  // namespace sqs

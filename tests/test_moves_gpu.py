@@ -10,6 +10,7 @@ from __future__ import annotations
 import math
 from dataclasses import replace
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -202,3 +203,27 @@ def test_group_quench_is_width_independent(ctx):
     for r in (crowd[0], crowd[57], crowd[-1]):
         for k in KEYS:
             assert r[k] == alone[k], k
+
+
+@pytest.mark.parametrize("n", [5, 24, 60])
+@pytest.mark.parametrize("moves", [False, True])
+def test_quench_width_and_corners(ctx, n, moves):
+    """Squares that violate two walls at once (a quarter of them pushed out of
+    each corner) through checkpoint quenches of one warp up to sixteen: every
+    launch shape leaves every replica in the same state with the same energy,
+    which is the energy of that state from scratch."""
+    from sqs.anneal import anneal_batch, jittered_grid
+
+    xya, L0 = jittered_grid(n, seed=n)
+    mid = L0 / 2
+    xya[:, :2] = mid + (xya[:, :2] - mid) * 1.15 + 0.25 * np.sign(xya[:, :2] - mid)
+    opts = dict(adapt=True, kick=True, quench_all=True, quench_steps=2, cert_all=True) if moves else {}
+    base = _job(n=n, replicas=16, sweeps=40, exchange_every=4, tmin=1e-6, tmax=1e-4, **opts)
+    base = replace(base, xya=xya, L0=L0)
+    got = [anneal_batch([replace(base, cluster=c)], ctx=ctx, trace=True)[0] for c in (1, 2, 4, 8, 16)]
+    for r in got:
+        np.testing.assert_array_equal(r["trace"]["energy"], r["trace"]["energy_full"])
+        for k in KEYS:
+            assert r[k] == got[0][k], k
+        for k in ("xya", "energy", "rung"):
+            np.testing.assert_array_equal(r["trace"][k], got[0]["trace"][k], err_msg=k)
