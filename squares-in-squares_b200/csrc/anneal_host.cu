@@ -137,6 +137,9 @@ bool replan(const sqs_job& J, int rl, JobDev& d, Plan& p) {
     const int want = std::min(16, (J.replicas + rl - 1) / rl);
     if (!plan_job(J.n, J.replicas, J.L0, p.cell, want, q) && !plan_job(J.n, J.replicas, J.L0, p.cell, 1, q)) return false;
     if (q.cs == p.cs) return false;
+    int resident = 0;  // a wider cluster needs that many free SMs in one GPC
+    if (anneal_max_clusters(q.cs, q.Rl, (size_t)(q.rb * q.Rl), uses_moves(d.flags), &resident) != SQS_OK || resident < 1)
+        return false;
     p = q;
     d.cs = q.cs;
     d.Rl = q.Rl;

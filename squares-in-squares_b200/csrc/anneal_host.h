@@ -61,7 +61,8 @@ void put(char* dst, size_t cap, const std::string& s);
 // default (smallest cluster that fits, cells of side kCellSide).
 int prepare_job(const sqs_job& J, int j, JobDev& d, JobMut& m, Plan& p, const Shape* shape = nullptr);
 // Another launch shape for a prepared job: about `rl` replicas a CTA (at most
-// the default plan's; the cell side stays).  True when the plan changed.
+// the default plan's; the cell side stays).  True when the plan changed; a
+// shape of which the device cannot hold one cluster is not taken.
 bool replan(const sqs_job& J, int rl, JobDev& d, Plan& p);
 // Resolve SQS_JOB_AUTOTUNE: the tuned shape of the job's class (tuning it on
 // first sight) and, when the job leaves exchange_every at 0, the tuned

@@ -149,3 +149,41 @@ def test_destroy_with_work_in_flight(ctx):
         while again.step():
             pass
         assert again.poll(jid)["status"] == 0
+
+
+def test_launch_shape_follows_the_load_without_changing_results(ctx):
+    """Jobs that run while the server's replicas cross both lines at which it
+    changes the launch shape (2 and 6 replicas an SM), up and down again, end
+    exactly as they do alone."""
+    from sqs.anneal import anneal_batch
+    from sqs.serve import Server
+
+    sms = ctx.info()[1]
+    first = [_job(70, 60, 900, replicas=64), _job(45, 61, 900, replicas=48, adapt=True, collective=True, quench_all=True)]
+    second = [_job(40 + 3 * k, 70 + k, 250, replicas=64) for k in range(2 * sms // 64 + 1)]
+    third = [_job(12 + k, 90 + k, 60, replicas=64 - 16 * (k % 2)) for k in range(5 * sms // 56 + 2)]
+    jobs = first + second + third
+    alone = anneal_batch(jobs, ctx=ctx)
+    got, ids, peaks = {}, {}, set()
+    with Server(ctx, hbm_bytes=1 << 30, max_active=64, slice_proposals=300) as srv:
+        waves = [first, second, third]
+        k = steps = 0
+        while len(got) < len(jobs):
+            if waves and steps % 12 == 0:
+                for j in waves.pop(0):
+                    ids[srv.submit(j)] = k
+                    k += 1
+            srv.step()
+            steps += 1
+            for jid, i in ids.items():
+                if i not in got:
+                    r = srv.poll(jid)
+                    if r is not None:
+                        got[i] = r
+            now = sum(jobs[i].replicas for i in ids.values() if i not in got)
+            peaks.add(0 if now <= 2 * sms else (1 if now <= 6 * sms else 2))
+            assert steps < 200000
+    assert peaks == {0, 1, 2}
+    for i in range(len(jobs)):
+        for key in KEYS:
+            assert got[i][key] == alone[i][key], (i, key)
