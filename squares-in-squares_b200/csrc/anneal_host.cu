@@ -600,7 +600,7 @@ static int anneal_run(sqs_ctx* ctx, const sqs_job* jobs, int njobs, int slice_sw
     auto seg = [&](size_t b) { size_t o = tot; tot += (b + 255) & ~(size_t)255; return o; };
     const size_t o_jd = seg(sizeof(JobDev) * njobs), o_jm = seg(sizeof(JobMut) * njobs);
     const size_t o_pos = seg(sizeof(float4) * (size_t)pos_total), o_best = seg(sizeof(double) * (size_t)best_total);
-    const size_t o_list = seg(sizeof(int32_t) * njobs);
+    const size_t o_list = seg(sizeof(int32_t) * njobs), o_plist = seg(sizeof(int32_t) * njobs);
     const size_t o_init = seg(sizeof(InitRec) * njobs), o_start = seg(sizeof(double) * (size_t)start_total);
     // trace: one (job, replica) item and one record per replica
     int64_t ntrace = 0;
@@ -713,10 +713,20 @@ static int anneal_run(sqs_ctx* ctx, const sqs_job* jobs, int njobs, int slice_sw
     }
     ctx->launches += (int64_t)rounds * (int64_t)keys.size();
     // FP64 gradient polish of every job's best state (jobs with polish_iters > 0)
-    size_t psmem = 0;
-    for (int j = 0; j < njobs; ++j) psmem = std::max(psmem, polish_smem_bytes(jobs[j].n));
-    if (int r = launch_polish(ctx->stream, njobs, d_list, d_jd, d_jm, d_best, psmem)) return r;
-    ctx->launches += 1;
+    std::vector<int32_t> plist, pn;
+    for (int j = 0; j < njobs; ++j)
+        if (jobs[j].polish_iters > 0) {
+            plist.push_back(j);
+            pn.push_back(jobs[j].n);
+        }
+    if (!plist.empty()) {
+        std::vector<int32_t> porder = width_order(ctx, pn);
+        for (int32_t& k : porder) k = plist[(size_t)k];
+        if (porder.empty()) porder = plist;
+        SQS_CUDA(cudaMemcpyAsync(D + o_plist, porder.data(), sizeof(int32_t) * porder.size(), cudaMemcpyHostToDevice,
+                                 ctx->stream));
+        if (int r = launch_polish(ctx, pn, (const int32_t*)(D + o_plist), d_jd, d_jm, d_best)) return r;
+    }
     SQS_CUDA(cudaEventRecord(e1, ctx->stream));
     std::vector<TraceRec> trec((size_t)ntrace);
     std::vector<float4> tpos;
@@ -825,11 +835,9 @@ extern "C" int sqs_polish_batch(sqs_ctx* ctx, int count, const int32_t* n_of, co
     SQS_REQUIRE(n_of && xya && xya_out && out, "null host pointer");
     SQS_REQUIRE(iters >= 0 && iters <= 1000000, "iters %d out of 0..1000000", iters);
     std::vector<int64_t> row0((size_t)count + 1, 0);
-    int nmax = 1;
     for (int k = 0; k < count; ++k) {
         SQS_REQUIRE(n_of[k] >= 1 && n_of[k] <= kMaxN, "packing %d: n=%d out of 1..%d", k, n_of[k], kMaxN);
         row0[(size_t)k + 1] = row0[(size_t)k] + n_of[k];
-        nmax = std::max(nmax, n_of[k]);
     }
     const int64_t rows = row0[(size_t)count];
     for (int64_t i = 0; i < 3 * rows; ++i) SQS_REQUIRE(std::isfinite(xya[i]), "non-finite coordinate at %lld", (long long)i);
@@ -837,15 +845,20 @@ extern "C" int sqs_polish_batch(sqs_ctx* ctx, int count, const int32_t* n_of, co
     auto seg = [&](size_t b) { size_t o = tot; tot += (b + 255) & ~(size_t)255; return o; };
     const size_t o_n = seg(sizeof(int32_t) * count), o_r = seg(sizeof(int64_t) * count);
     const size_t o_x = seg(sizeof(double) * 3 * (size_t)rows), o_res = seg(sizeof(double) * 3 * count);
+    std::vector<int32_t> sizes(n_of, n_of + count);
+    const std::vector<int32_t> order = width_order(ctx, sizes);
+    const size_t o_ord = seg(sizeof(int32_t) * count);
     if (int r = ctx->d_polish.reserve(tot)) return r;
     char* D = (char*)ctx->d_polish.p;
     SQS_CUDA(cudaMemcpyAsync(D + o_n, n_of, sizeof(int32_t) * count, cudaMemcpyHostToDevice, ctx->stream));
     SQS_CUDA(cudaMemcpyAsync(D + o_r, row0.data(), sizeof(int64_t) * count, cudaMemcpyHostToDevice, ctx->stream));
     SQS_CUDA(cudaMemcpyAsync(D + o_x, xya, sizeof(double) * 3 * (size_t)rows, cudaMemcpyHostToDevice, ctx->stream));
-    if (int r = launch_polish_states(ctx->stream, count, (const int32_t*)(D + o_n), (const int64_t*)(D + o_r), iters,
-                                     (double*)(D + o_x), (double*)(D + o_res), polish_smem_bytes(nmax)))
+    if (!order.empty())
+        SQS_CUDA(cudaMemcpyAsync(D + o_ord, order.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice, ctx->stream));
+    if (int r = launch_polish_states(ctx, sizes, order.empty() ? nullptr : (const int32_t*)(D + o_ord),
+                                     (const int32_t*)(D + o_n), (const int64_t*)(D + o_r), iters, (double*)(D + o_x),
+                                     (double*)(D + o_res)))
         return r;
-    ctx->launches += 1;
     std::vector<double> res(3 * (size_t)count);
     SQS_CUDA(cudaMemcpyAsync(xya_out, D + o_x, sizeof(double) * 3 * (size_t)rows, cudaMemcpyDeviceToHost, ctx->stream));
     SQS_CUDA(cudaMemcpyAsync(res.data(), D + o_res, sizeof(double) * res.size(), cudaMemcpyDeviceToHost, ctx->stream));
@@ -866,12 +879,10 @@ extern "C" int sqs_energy_fp64(sqs_ctx* ctx, int count, const int32_t* n_of, con
     if (count == 0) return SQS_OK;
     SQS_REQUIRE(n_of && xya && side && energy, "null host pointer");
     std::vector<int64_t> row0((size_t)count + 1, 0);
-    int nmax = 1;
     for (int k = 0; k < count; ++k) {
         SQS_REQUIRE(n_of[k] >= 1 && n_of[k] <= kMaxN, "packing %d: n=%d out of 1..%d", k, n_of[k], kMaxN);
         SQS_REQUIRE(std::isfinite(side[k]) && side[k] > 0, "packing %d: side must be finite and positive", k);
         row0[(size_t)k + 1] = row0[(size_t)k] + n_of[k];
-        nmax = std::max(nmax, n_of[k]);
     }
     const int64_t rows = row0[(size_t)count];
     for (int64_t i = 0; i < 3 * rows; ++i) SQS_REQUIRE(std::isfinite(xya[i]), "non-finite coordinate at %lld", (long long)i);
@@ -880,17 +891,21 @@ extern "C" int sqs_energy_fp64(sqs_ctx* ctx, int count, const int32_t* n_of, con
     const size_t o_n = seg(sizeof(int32_t) * count), o_r = seg(sizeof(int64_t) * count);
     const size_t o_s = seg(sizeof(double) * count), o_x = seg(sizeof(double) * 3 * (size_t)rows);
     const size_t o_e = seg(sizeof(double) * count), o_g = seg(grad ? sizeof(double) * 3 * (size_t)rows : 0);
+    std::vector<int32_t> sizes(n_of, n_of + count);
+    const std::vector<int32_t> order = width_order(ctx, sizes);
+    const size_t o_ord = seg(sizeof(int32_t) * count);
     if (int r = ctx->d_polish.reserve(tot)) return r;
     char* D = (char*)ctx->d_polish.p;
     SQS_CUDA(cudaMemcpyAsync(D + o_n, n_of, sizeof(int32_t) * count, cudaMemcpyHostToDevice, ctx->stream));
     SQS_CUDA(cudaMemcpyAsync(D + o_r, row0.data(), sizeof(int64_t) * count, cudaMemcpyHostToDevice, ctx->stream));
     SQS_CUDA(cudaMemcpyAsync(D + o_s, side, sizeof(double) * count, cudaMemcpyHostToDevice, ctx->stream));
     SQS_CUDA(cudaMemcpyAsync(D + o_x, xya, sizeof(double) * 3 * (size_t)rows, cudaMemcpyHostToDevice, ctx->stream));
-    if (int r = launch_energy_states(ctx->stream, count, (const int32_t*)(D + o_n), (const int64_t*)(D + o_r),
-                                     (const double*)(D + o_s), (const double*)(D + o_x), (double*)(D + o_e),
-                                     grad ? (double*)(D + o_g) : nullptr, energy_smem_bytes(nmax)))
+    if (!order.empty())
+        SQS_CUDA(cudaMemcpyAsync(D + o_ord, order.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice, ctx->stream));
+    if (int r = launch_energy_states(ctx, sizes, order.empty() ? nullptr : (const int32_t*)(D + o_ord),
+                                     (const int32_t*)(D + o_n), (const int64_t*)(D + o_r), (const double*)(D + o_s),
+                                     (const double*)(D + o_x), (double*)(D + o_e), grad ? (double*)(D + o_g) : nullptr))
         return r;
-    ctx->launches += 1;
     SQS_CUDA(cudaMemcpyAsync(energy, D + o_e, sizeof(double) * count, cudaMemcpyDeviceToHost, ctx->stream));
     if (grad)
         SQS_CUDA(cudaMemcpyAsync(grad, D + o_g, sizeof(double) * 3 * (size_t)rows, cudaMemcpyDeviceToHost, ctx->stream));

@@ -26,9 +26,13 @@ int prime_anneal();
 int launch_init(cudaStream_t stream, int njobs, const InitRec* rec, const double* start, float4* pos);
 int launch_trace(cudaStream_t stream, int items, const int2* list, const JobDev* jdev, const JobMut* jmut,
                  float4* pos, TraceRec* out, size_t smem);
-size_t energy_smem_bytes(int n);
-int launch_energy_states(cudaStream_t stream, int count, const int32_t* n_of, const int64_t* row0, const double* side,
-                         const double* xya, double* energy_out, double* grad, size_t smem);
+// FP64 kernels, one CTA a packing, its width by its size.  `n` holds the sizes in
+// launch order: as they come up to one packing an SM, else descending, as
+// width_order sorts them (it returns the permutation, empty in the first
+// case), and `order` is that permutation on the device (null in the first case).
+std::vector<int32_t> width_order(sqs_ctx* ctx, std::vector<int32_t>& n);
+int launch_energy_states(sqs_ctx* ctx, const std::vector<int32_t>& n, const int32_t* order, const int32_t* n_of,
+                         const int64_t* row0, const double* side, const double* xya, double* energy_out, double* grad);
 
 // One launch of the anneal kernel: the jobs job_list[0 .. njobs) sharing a
 // cluster shape, with the shared memory of the largest.
@@ -49,11 +53,11 @@ int anneal_max_clusters(int cs, int Rl, size_t smem, bool moves, int* out);
 size_t anneal_smem(int cs, int Rl, int64_t rb, int n_max, bool moves, int need = 1 << 30);
 int launch_anneal(cudaStream_t stream, int njobs, int cs, int Rl, size_t smem, bool moves, const int32_t* job_list,
                   const JobDev* jdev, JobMut* jmut, float4* pos, double* best, int slice);
-int launch_polish(cudaStream_t stream, int njobs, const int32_t* job_list, const JobDev* jdev, JobMut* jmut,
-                  double* best, size_t smem);
-size_t polish_smem_bytes(int n);
-int launch_polish_states(cudaStream_t stream, int count, const int32_t* n_of, const int64_t* row0, int iters,
-                         double* xya, double* res, size_t smem);
+// job_list: the jobs in the order of `n`
+int launch_polish(sqs_ctx* ctx, const std::vector<int32_t>& n, const int32_t* job_list, const JobDev* jdev, JobMut* jmut,
+                  double* best);
+int launch_polish_states(sqs_ctx* ctx, const std::vector<int32_t>& n, const int32_t* order, const int32_t* n_of,
+                         const int64_t* row0, int iters, double* xya, double* res);
 
 void put(char* dst, size_t cap, const std::string& s);
 // Validate one job and fill its device records (offsets left to the caller).

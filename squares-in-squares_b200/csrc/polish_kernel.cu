@@ -22,8 +22,11 @@
 // them overlapped, 200 steps: 7.8 -> 3.2 ms a call (one B200).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <type_traits>
+#include <vector>
 
 #include "anneal.cuh"
 #include "common.cuh"
@@ -31,7 +34,15 @@
 namespace sqs {
 namespace ann {
 
-constexpr int kPT = 512;  // threads per polish CTA
+// Threads of a CTA by its size class (see launch_widths): a narrow CTA takes
+// packings of up to kWidthN squares and shares its SM with others.
+constexpr int kSmallT = 128, kMidT = 256, kWideT = 512;
+template <int PT>
+constexpr int kWidthN = PT == kSmallT ? 64 : (PT == kMidT ? 256 : kMaxN);
+template <int PT>
+constexpr int kResident = PT == kSmallT ? 4 : (PT == kMidT ? 2 : 1);  // CTAs an SM the registers allow
+template <int PT>
+constexpr int kPer = (kWidthN<PT> + PT - 1) / PT;  // squares a thread
 constexpr int kPS = 256;  // an energy's partial sums (see energy())
 
 // Neighbour lists of the polish: every partner within sqrt(2.000001) + 0.25
@@ -108,13 +119,14 @@ __device__ __forceinline__ double wall_smooth(double x, double y, double c, doub
     return e;
 }
 
+template <int PT>
 __device__ double block_max(double v, Sh<double> red) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
     double t = red[0];
-    for (int w = 1; w < kPT / 32; ++w) t = fmax(t, red[w]);
+    for (int w = 1; w < PT / 32; ++w) t = fmax(t, red[w]);
     return t;
 }
 
@@ -138,6 +150,7 @@ struct Cells {
 };
 
 // Sort the squares of q into cells.  Starts and ends with a barrier.
+template <int PT>
 __device__ void build_cells(int n, Cells& c, Sh<double3> q, double x0, double y0, double side) {
     c.x0 = x0;
     c.y0 = y0;
@@ -146,12 +159,12 @@ __device__ void build_cells(int n, Cells& c, Sh<double3> q, double x0, double y0
     if (!(c.inv > 0.0 && c.inv * kCellMinW <= 1.0)) c.inv = 0.0, c.G = 1;  // a side below one cell, or not finite
     const int ncell = c.G * c.G, t = threadIdx.x;
     __syncthreads();
-    for (int k = t; k <= ncell; k += kPT) c.start[k] = 0;
+    for (int k = t; k <= ncell; k += PT) c.start[k] = 0;
     __syncthreads();
-    int rank[kMaxN / kPT + 1], cell[kMaxN / kPT + 1];
+    int rank[kPer<PT>], cell[kPer<PT>];
 #pragma unroll
-    for (int m = 0; m < kMaxN / kPT + 1; ++m) {
-        const int i = t + m * kPT;
+    for (int m = 0; m < kPer<PT>; ++m) {
+        const int i = t + m * PT;
         if (i < n) {
             cell[m] = c.cy(q[i]) * c.G + c.cx(q[i]);
             rank[m] = atomicAdd(&c.start[cell[m]], 1);
@@ -177,8 +190,8 @@ __device__ void build_cells(int n, Cells& c, Sh<double3> q, double x0, double y0
     }
     __syncthreads();
 #pragma unroll
-    for (int m = 0; m < kMaxN / kPT + 1; ++m) {
-        const int i = t + m * kPT;
+    for (int m = 0; m < kPer<PT>; ++m) {
+        const int i = t + m * PT;
         if (i < n) c.order[c.start[cell[m]] + rank[m]] = (uint16_t)i;
     }
     __syncthreads();
@@ -186,9 +199,10 @@ __device__ void build_cells(int n, Cells& c, Sh<double3> q, double x0, double y0
 
 // Build the list for state q from its cells; false when a square has more
 // than kNbK partners (the callers then use all pairs).
+template <int PT>
 __device__ bool build_nbr(int n, const NbrList& nb, const Cells& c, Sh<double3> q) {
     bool over = false;
-    for (int i = threadIdx.x; i < n; i += kPT) {
+    for (int i = threadIdx.x; i < n; i += PT) {
         const double3 p = q[i];
         const Sh<uint16_t> L = nb.idx + i * kNbK;
         const int cx = c.cx(p), cy = c.cy(p);
@@ -228,7 +242,7 @@ __device__ bool build_nbr(int n, const NbrList& nb, const Cells& c, Sh<double3> 
 // also ends the reads of the call before.
 struct Red {
     Sh<double> e;       // [kPS / 32]
-    Sh<double> m;       // [kPT / 32]
+    Sh<double> m;       // [kWideT / 32]
     Sh<double> es;      // [kPS]: squares' sums of the lane-parallel form
     Sh<double> terms;   // [n][kTerms]
     Sh<uint8_t> nterm;  // [n]: terms there, kTerms + 1: more than fit
@@ -252,13 +266,14 @@ __device__ __noinline__ double add_square(double e, int i, int n, Sh<double3> q,
     return e;
 }
 
+template <int PT>
 __device__ double energy(int n, Sh<double3> q, Sh<double2> cs, double L, Sh<double3> g, double& gmax2, const Red& red,
                          const NbrList& nb, bool listed) {
     double e = 0.0, gm = 0.0;
     const int t = threadIdx.x;
-    const int w = !listed || 2 * n > min(kPT, 2 * kPS) ? 1 : (4 * n > kPT ? 2 : (8 * n > kPT ? 4 : 8));
+    const int w = !listed || 2 * n > min(PT, 2 * kPS) ? 1 : (4 * n > PT ? 2 : (8 * n > PT ? 4 : 8));
     if (w == 1) {
-        for (int i = t; i < n; i += kPT) {
+        for (int i = t; i < n; i += PT) {
             const double3 p = q[i];
             const double2 pc = cs[i];
             double gx = 0, gy = 0, ga = 0;
@@ -354,17 +369,18 @@ __device__ double energy(int n, Sh<double3> q, Sh<double2> cs, double L, Sh<doub
     }
     __syncthreads();
     double s = 0.0, mx = 0.0;
-    for (int k = 0; k < kPS / 32; ++k) s += red.e[k];
-    for (int k = 0; k < kPT / 32; ++k) mx = fmax(mx, red.m[k]);
+    for (int k = 0; k < min(kPS, PT) / 32; ++k) s += red.e[k];  // (a narrow CTA's squares are all in these)
+    for (int k = 0; k < PT / 32; ++k) mx = fmax(mx, red.m[k]);
     gmax2 = mx;
     return s;
 }
 
 // Certified side of q (dilation lambda, bounding box of the dilated state).
+template <int PT>
 __device__ double cert_side_all(int n, Sh<double3> q, Sh<double2> cs, const Cells& c, Sh<double> red,
                                 double& lam_out, double& x0, double& y0) {
     double lam = 1.0;
-    for (int i = threadIdx.x; i < n; i += kPT) {
+    for (int i = threadIdx.x; i < n; i += PT) {
         const double3 p = q[i];
         const double ci = cs[i].x, si = cs[i].y;
         const int cx = c.cx(p), cy = c.cy(p);
@@ -384,11 +400,11 @@ __device__ double cert_side_all(int n, Sh<double3> q, Sh<double2> cs, const Cell
             }
         }
     }
-    lam = block_max(lam, red);
+    lam = block_max<PT>(lam, red);
     lam_out = lam;
     if (lam > 1.008) return 1e30;
     double a0 = 1e300, a1 = -1e300, b0 = 1e300, b1 = -1e300;
-    for (int i = threadIdx.x; i < n; i += kPT) {
+    for (int i = threadIdx.x; i < n; i += PT) {
         const double r = 0.5 * (fabs(cs[i].x) + fabs(cs[i].y));
         const double x = q[i].x * lam, y = q[i].y * lam;
         a0 = fmin(a0, x - r);
@@ -396,10 +412,10 @@ __device__ double cert_side_all(int n, Sh<double3> q, Sh<double2> cs, const Cell
         b0 = fmin(b0, y - r);
         b1 = fmax(b1, y + r);
     }
-    x0 = -block_max(-a0, red);
-    const double xm = block_max(a1, red);
-    y0 = -block_max(-b0, red);
-    const double ym = block_max(b1, red);
+    x0 = -block_max<PT>(-a0, red);
+    const double xm = block_max<PT>(a1, red);
+    y0 = -block_max<PT>(-b0, red);
+    const double ym = block_max<PT>(b1, red);
     return fmax(xm - x0, ym - y0);
 }
 
@@ -408,8 +424,9 @@ __device__ __forceinline__ double wrap_q(double a) {
     return a < 0.0 ? a + 1.57079632679489661923 : a;
 }
 
+template <int PT>
 __device__ void trig_of(int n, Sh<double3> q, Sh<double2> cs) {
-    for (int i = threadIdx.x; i < n; i += kPT) {
+    for (int i = threadIdx.x; i < n; i += PT) {
         double s, c;
         sincos(q[i].z, &s, &c);
         cs[i] = make_double2(c, s);
@@ -425,18 +442,18 @@ struct PolishBufs {
     Sh<double3> tg;  // gradient at q
     Sh<double3> sv;  // best so far (translated, dilated)
     Sh<double2> cs;  // cos/sin of the state being evaluated
-    Sh<double> max;  // [kPT / 32] partials of block_max
+    Sh<double> max;  // [kWideT / 32] partials of block_max
     NbrList nb;   // neighbour list of the descent
     Cells cells;
     Red red;
 };
 
 // The evaluation's share of the layout (from `off` on), then the polish's.
-constexpr int kRedDoubles = kPS / 32 + 2 * (kPT / 32) + kPS;
+constexpr int kRedDoubles = kPS / 32 + 2 * (kWideT / 32) + kPS;
 __device__ __forceinline__ int eval_bufs(int off, int n, Red& red, NbrList& nb, Cells& cells) {
     red.e = Sh<double>{off};
     red.m = red.e + kPS / 32;
-    red.es = red.m + 2 * (kPT / 32);  // (block_max's partials lie between)
+    red.es = red.m + 2 * (kWideT / 32);  // (block_max's partials lie between)
     red.terms = red.es + kPS;
     cells.start = Sh<int>{red.terms.off + 8 * kTerms * n};
     nb.idx = Sh<uint16_t>{cells.start.off + 4 * (kCG * kCG + 1)};
@@ -458,7 +475,7 @@ __device__ __forceinline__ PolishBufs polish_bufs(int n) {
     b.tg = b.g + n;
     b.sv = b.tg + n;
     eval_bufs(b.sv.off + 24 * n, n, b.red, b.nb, b.cells);
-    b.max = b.red.m + kPT / 32;
+    b.max = b.red.m + kWideT / 32;
     return b;
 }
 
@@ -468,12 +485,13 @@ size_t polish_smem_bytes(int n) { return (size_t)n * (5 * 24 + 16) + eval_bytes(
 // Descend the energy of state q0 (inside [0, Lt] up to its overhang) at side
 // Lt until it vanishes (at most *budget gradient steps, each with up to 8
 // backtracking trials).  Ends with the cells and trig of q0.
+template <int PT>
 __device__ void descend(int n, PolishBufs& B, double Lt, int* budget) {
-    trig_of(n, B.q0, B.cs);
-    build_cells(n, B.cells, B.q0, 0.0, 0.0, Lt);
-    bool listed = build_nbr(n, B.nb, B.cells, B.q0);
+    trig_of<PT>(n, B.q0, B.cs);
+    build_cells<PT>(n, B.cells, B.q0, 0.0, 0.0, Lt);
+    bool listed = build_nbr<PT>(n, B.nb, B.cells, B.q0);
     double gm2;
-    double E = energy(n, B.q0, B.cs, Lt, B.g, gm2, B.red, B.nb, listed);
+    double E = energy<PT>(n, B.q0, B.cs, Lt, B.g, gm2, B.red, B.nb, listed);
     double gmax = sqrt(gm2);
     double moved_by = 0.0;  // bound on any centre's distance from where the list was built
     double alpha = 0.05;
@@ -481,7 +499,7 @@ __device__ void descend(int n, PolishBufs& B, double Lt, int* budget) {
         --*budget;
         bool moved = false;
         for (int ls = 0; ls < 8 && !moved; ++ls) {
-            for (int i = threadIdx.x; i < n; i += kPT) {
+            for (int i = threadIdx.x; i < n; i += PT) {
                 const double3 p = B.q0[i], d = B.g[i];
                 const double3 v = make_double3(p.x - alpha * d.x, p.y - alpha * d.y, wrap_q(p.z - alpha * d.z));
                 double s, c;
@@ -493,11 +511,11 @@ __device__ void descend(int n, PolishBufs& B, double Lt, int* budget) {
             const double step = alpha * gmax;
             bool rebuilt = false;
             if (!(moved_by + step <= kNbMove)) {  // past the list's reach: a list of the trial itself
-                build_cells(n, B.cells, B.q, 0.0, 0.0, Lt);
-                listed = build_nbr(n, B.nb, B.cells, B.q);
+                build_cells<PT>(n, B.cells, B.q, 0.0, 0.0, Lt);
+                listed = build_nbr<PT>(n, B.nb, B.cells, B.q);
                 rebuilt = true;
             }
-            const double En = energy(n, B.q, B.cs, Lt, B.tg, gm2, B.red, B.nb, listed);
+            const double En = energy<PT>(n, B.q, B.cs, Lt, B.tg, gm2, B.red, B.nb, listed);
             if (En < E) {
                 E = En;
                 moved = true;
@@ -518,25 +536,26 @@ __device__ void descend(int n, PolishBufs& B, double Lt, int* budget) {
         if (!moved) break;
     }
     __syncthreads();
-    trig_of(n, B.q0, B.cs);
-    build_cells(n, B.cells, B.q0, 0.0, 0.0, Lt);
+    trig_of<PT>(n, B.q0, B.cs);
+    build_cells<PT>(n, B.cells, B.q0, 0.0, 0.0, Lt);
 }
 
 // Compress-and-descend attempts on the certified state sv of side *Lb
 // (delta shrinking by 0.3 after every attempt that does not certify a
 // smaller side); sv and *Lb are updated in place.
+template <int PT>
 __device__ void polish_loop(int n, PolishBufs& B, double* Lb, int* budget, Sh<double> red) {
     double delta = 1e-4;
     for (int attempt = 0; attempt < 12 && *budget > 0 && delta > 1e-9; ++attempt) {
         const double f = 1.0 - delta, Lt = *Lb * f;
-        for (int i = threadIdx.x; i < n; i += kPT) B.q0[i] = make_double3(B.sv[i].x * f, B.sv[i].y * f, B.sv[i].z);
+        for (int i = threadIdx.x; i < n; i += PT) B.q0[i] = make_double3(B.sv[i].x * f, B.sv[i].y * f, B.sv[i].z);
         __syncthreads();
-        descend(n, B, Lt, budget);
+        descend<PT>(n, B, Lt, budget);
         double lam = 0, x0 = 0, y0 = 0;
-        const double Lc = cert_side_all(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
+        const double Lc = cert_side_all<PT>(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
         if (Lc < *Lb) {
             *Lb = Lc;
-            for (int i = threadIdx.x; i < n; i += kPT)
+            for (int i = threadIdx.x; i < n; i += PT)
                 B.sv[i] = make_double3(B.q0[i].x * lam - x0, B.q0[i].y * lam - y0, B.q0[i].z);
             __syncthreads();
         } else {
@@ -545,7 +564,8 @@ __device__ void polish_loop(int n, PolishBufs& B, double* Lb, int* budget, Sh<do
     }
 }
 
-__global__ void __launch_bounds__(kPT) polish_kernel(const int32_t* __restrict__ job_list,
+template <int PT>
+__global__ void __launch_bounds__(PT, kResident<PT>) polish_kernel(const int32_t* __restrict__ job_list,
                                                      const JobDev* __restrict__ jdev, JobMut* __restrict__ jmut,
                                                      double* __restrict__ best) {
     const int job = job_list[blockIdx.x];
@@ -556,11 +576,11 @@ __global__ void __launch_bounds__(kPT) polish_kernel(const int32_t* __restrict__
     PolishBufs B = polish_bufs(n);
     const Sh<double> red = B.max;
     double* b = best + jd.best_off;
-    for (int i = threadIdx.x; i < n; i += kPT) B.sv[i] = make_double3(b[3 * i], b[3 * i + 1], b[3 * i + 2]);
+    for (int i = threadIdx.x; i < n; i += PT) B.sv[i] = make_double3(b[3 * i], b[3 * i + 1], b[3 * i + 2]);
     __syncthreads();
     int budget = jd.polish_iters;
-    polish_loop(n, B, &Lb, &budget, red);
-    for (int i = threadIdx.x; i < n; i += kPT) {
+    polish_loop<PT>(n, B, &Lb, &budget, red);
+    for (int i = threadIdx.x; i < n; i += PT) {
         b[3 * i] = B.sv[i].x;
         b[3 * i + 1] = B.sv[i].y;
         b[3 * i + 2] = B.sv[i].z;
@@ -574,40 +594,42 @@ __global__ void __launch_bounds__(kPT) polish_kernel(const int32_t* __restrict__
 // 1.008) first descends its energy inside its own bounding box and, if
 // overlaps remain, has its centres spread by that dilation (at most 1.5x)
 // and descends in a box scaled alike.
-// res[k] = {L_in, L_out, iterations used}.
-__global__ void __launch_bounds__(kPT) polish_states_kernel(const int32_t* __restrict__ n_of,
+// res[k] = {L_in, L_out, iterations used}.  CTA b takes state order[b] (b when order is null).
+template <int PT>
+__global__ void __launch_bounds__(PT, kResident<PT>) polish_states_kernel(const int32_t* __restrict__ order,
+                                                            const int32_t* __restrict__ n_of,
                                                             const int64_t* __restrict__ row0, int iters,
                                                             double* __restrict__ xya, double* __restrict__ res) {
-    const int k = blockIdx.x;
+    const int k = order ? order[blockIdx.x] : (int)blockIdx.x;
     const int n = n_of[k];
     double* st = xya + 3 * row0[k];
     PolishBufs B = polish_bufs(n);
     const Sh<double> red = B.max;
-    for (int i = threadIdx.x; i < n; i += kPT) B.q0[i] = make_double3(st[3 * i], st[3 * i + 1], wrap_q(st[3 * i + 2]));
+    for (int i = threadIdx.x; i < n; i += PT) B.q0[i] = make_double3(st[3 * i], st[3 * i + 1], wrap_q(st[3 * i + 2]));
     __syncthreads();
-    trig_of(n, B.q0, B.cs);
+    trig_of<PT>(n, B.q0, B.cs);
     int budget = iters;
     double lam = 0, x0 = 0, y0 = 0;
     // bounding box of the input
     double a0 = 1e300, a1 = -1e300, b0 = 1e300, b1 = -1e300;
-    for (int i = threadIdx.x; i < n; i += kPT) {
+    for (int i = threadIdx.x; i < n; i += PT) {
         const double r = 0.5 * (fabs(B.cs[i].x) + fabs(B.cs[i].y));
         a0 = fmin(a0, B.q0[i].x - r);
         a1 = fmax(a1, B.q0[i].x + r);
         b0 = fmin(b0, B.q0[i].y - r);
         b1 = fmax(b1, B.q0[i].y + r);
     }
-    a0 = -block_max(-a0, red);
-    a1 = block_max(a1, red);
-    b0 = -block_max(-b0, red);
-    b1 = block_max(b1, red);
+    a0 = -block_max<PT>(-a0, red);
+    a1 = block_max<PT>(a1, red);
+    b0 = -block_max<PT>(-b0, red);
+    b1 = block_max<PT>(b1, red);
     const double side = fmax(a1 - a0, b1 - b0);
-    build_cells(n, B.cells, B.q0, a0, b0, side);
-    double Lb = cert_side_all(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
+    build_cells<PT>(n, B.cells, B.q0, a0, b0, side);
+    double Lb = cert_side_all<PT>(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
     const double L_in = Lb, lam_in = lam;
     if (Lb >= 1e29) {
         // translated to the origin, with the bounding box as the side
-        for (int i = threadIdx.x; i < n; i += kPT) {
+        for (int i = threadIdx.x; i < n; i += PT) {
             B.sv[i] = make_double3(B.q0[i].x - a0, B.q0[i].y - b0, B.q0[i].z);  // the input, at the origin
             B.q0[i] = B.sv[i];
         }
@@ -618,24 +640,24 @@ __global__ void __launch_bounds__(kPT) polish_states_kernel(const int32_t* __res
         // most 1.5x) and descend in a box scaled alike
         int half = budget / 2;
         budget -= half;
-        descend(n, B, side, &half);
+        descend<PT>(n, B, side, &half);
         budget += half;
-        Lb = cert_side_all(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
+        Lb = cert_side_all<PT>(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
         if (Lb >= 1e29) {
             const double f = fmin(fmax(lam_in, 1.0), 1.5);
-            for (int i = threadIdx.x; i < n; i += kPT)
+            for (int i = threadIdx.x; i < n; i += PT)
                 B.q0[i] = make_double3(B.sv[i].x * f, B.sv[i].y * f, B.sv[i].z);
             __syncthreads();
-            descend(n, B, side * f, &budget);
-            Lb = cert_side_all(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
+            descend<PT>(n, B, side * f, &budget);
+            Lb = cert_side_all<PT>(n, B.q0, B.cs, B.cells, red, lam, x0, y0);
         }
     }
     if (Lb < 1e29) {
-        for (int i = threadIdx.x; i < n; i += kPT)
+        for (int i = threadIdx.x; i < n; i += PT)
             B.sv[i] = make_double3(B.q0[i].x * lam - x0, B.q0[i].y * lam - y0, B.q0[i].z);
         __syncthreads();
-        polish_loop(n, B, &Lb, &budget, red);
-        for (int i = threadIdx.x; i < n; i += kPT) {
+        polish_loop<PT>(n, B, &Lb, &budget, red);
+        for (int i = threadIdx.x; i < n; i += PT) {
             st[3 * i] = B.sv[i].x;
             st[3 * i + 1] = B.sv[i].y;
             st[3 * i + 2] = B.sv[i].z;
@@ -652,14 +674,16 @@ __global__ void __launch_bounds__(kPT) polish_states_kernel(const int32_t* __res
 // polish's own energy function over a neighbour list (all pairs, bit for
 // bit), with cos and sin taken of the angles as given.  State k has n_of[k]
 // rows at xya + 3 * row0[k] and side side[k]; energy[k], and the gradient rows
-// at the same offsets of grad when grad is not null.
-__global__ void __launch_bounds__(kPT) energy_states_kernel(const int32_t* __restrict__ n_of,
+// at the same offsets of grad when grad is not null; order as above.
+template <int PT>
+__global__ void __launch_bounds__(PT, kResident<PT>) energy_states_kernel(const int32_t* __restrict__ order,
+                                                            const int32_t* __restrict__ n_of,
                                                             const int64_t* __restrict__ row0,
                                                             const double* __restrict__ side,
                                                             const double* __restrict__ xya,
                                                             double* __restrict__ energy_out,
                                                             double* __restrict__ grad) {
-    const int k = blockIdx.x;
+    const int k = order ? order[blockIdx.x] : (int)blockIdx.x;
     const int n = n_of[k];
     const Sh<double2> cs{0};
     const Sh<double3> q{16 * n}, g = q + n;
@@ -668,17 +692,17 @@ __global__ void __launch_bounds__(kPT) energy_states_kernel(const int32_t* __res
     Cells cells;
     eval_bufs(g.off + 24 * n, n, red, nb, cells);
     const double* st = xya + 3 * row0[k];
-    for (int i = threadIdx.x; i < n; i += kPT) q[i] = make_double3(st[3 * i], st[3 * i + 1], st[3 * i + 2]);
+    for (int i = threadIdx.x; i < n; i += PT) q[i] = make_double3(st[3 * i], st[3 * i + 1], st[3 * i + 2]);
     __syncthreads();
-    trig_of(n, q, cs);
-    build_cells(n, cells, q, 0.0, 0.0, side[k]);
-    const bool listed = build_nbr(n, nb, cells, q);
+    trig_of<PT>(n, q, cs);
+    build_cells<PT>(n, cells, q, 0.0, 0.0, side[k]);
+    const bool listed = build_nbr<PT>(n, nb, cells, q);
     double gm2;
-    const double e = energy(n, q, cs, side[k], g, gm2, red, nb, listed);
+    const double e = energy<PT>(n, q, cs, side[k], g, gm2, red, nb, listed);
     if (threadIdx.x == 0) energy_out[k] = e;
     if (grad) {
         double* go = grad + 3 * row0[k];
-        for (int i = threadIdx.x; i < n; i += kPT) {
+        for (int i = threadIdx.x; i < n; i += PT) {
             go[3 * i] = g[i].x;
             go[3 * i + 1] = g[i].y;
             go[3 * i + 2] = g[i].z;
@@ -688,49 +712,116 @@ __global__ void __launch_bounds__(kPT) energy_states_kernel(const int32_t* __res
 
 size_t energy_smem_bytes(int n) { return (size_t)n * (2 * sizeof(double3) + sizeof(double2)) + eval_bytes(n) + 16; }
 
-int launch_energy_states(cudaStream_t stream, int count, const int32_t* n_of, const int64_t* row0, const double* side,
-                         const double* xya, double* energy_out, double* grad, size_t smem) {
-    static std::atomic<bool> attr_done[64];  // set-up once per device (idempotent if repeated)
-    int dev = 0;
-    SQS_CUDA(cudaGetDevice(&dev));
-    if (!attr_done[dev & 63]) {
-        SQS_CUDA(cudaFuncSetAttribute(energy_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
-        attr_done[dev & 63] = true;
+// Launches of a batch whose sizes n[0 .. count) descend, or of any order up to
+// one CTA an SM: launch(width tag, stream, first, count, largest n).
+// Up to one packing an SM each has an SM to itself and takes the widest CTA
+// (64 of n 5..1000 x 200 steps: 7.8 ms with 256 threads and all-pairs lists,
+// 3.2 now).  Beyond that a wide CTA leaves most of its threads and registers
+// idle on a small packing while others wait, so the width goes by size, each
+// class with the shared memory of its own largest, side by side and the
+// longest first: 1,000 of n <= 30 x 100 steps took 4.9 ms a call with 512
+// threads for all and 3.3 now, 444 of n = 250 4.2 and 3.8, 300 of n 5..1000
+// 3.4 and 3.0.
+template <class Launch>
+static int launch_widths(sqs_ctx* ctx, const std::vector<int32_t>& n, Launch&& launch) {
+    const int count = (int)n.size();
+    if (count == 0) return SQS_OK;
+    if (count <= ctx->sm_count)
+        return launch(std::integral_constant<int, kWideT>{}, ctx->stream, 0, count, *std::max_element(n.begin(), n.end()));
+    auto below = [&](int limit) {
+        return (int)(std::partition_point(n.begin(), n.end(), [&](int32_t v) { return v > limit; }) - n.begin());
+    };
+    const int mid = below(kWidthN<kMidT>), small = below(kWidthN<kSmallT>);
+    const bool fork = (mid > 0) + (small > mid) + (count > small) > 1;
+    cudaStream_t s_mid = ctx->stream, s_small = ctx->stream;
+    if (fork) {
+        SQS_CUDA(cudaEventRecord(ctx->fork, ctx->stream));
+        s_mid = ctx->aux[0];
+        s_small = ctx->aux[1];
+        for (int a = 0; a < 2; ++a) SQS_CUDA(cudaStreamWaitEvent(ctx->aux[a], ctx->fork, 0));
     }
-    if (count <= 0) return SQS_OK;
-    energy_states_kernel<<<count, kPT, smem, stream>>>(n_of, row0, side, xya, energy_out, grad);
-    SQS_CUDA(cudaGetLastError());
+    int rc = SQS_OK;
+    if (mid > 0) rc = launch(std::integral_constant<int, kWideT>{}, ctx->stream, 0, mid, n[0]);
+    if (!rc && small > mid)
+        rc = launch(std::integral_constant<int, kMidT>{}, s_mid, mid, small - mid, n[(size_t)mid]);
+    if (!rc && count > small)
+        rc = launch(std::integral_constant<int, kSmallT>{}, s_small, small, count - small, n[(size_t)small]);
+    if (fork) {  // join the side streams, also after a failed launch
+        for (int a = 0; a < 2; ++a) {
+            SQS_CUDA(cudaEventRecord(ctx->join[a], ctx->aux[a]));
+            SQS_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->join[a], 0));
+        }
+    }
+    return rc;
+}
+
+std::vector<int32_t> width_order(sqs_ctx* ctx, std::vector<int32_t>& n) {
+    std::vector<int32_t> order;
+    if ((int)n.size() <= ctx->sm_count) return order;
+    int32_t start[kMaxN + 2] = {0};  // counting sort, the largest first
+    for (int32_t v : n) ++start[kMaxN - v + 1];
+    for (int k = 1; k <= kMaxN + 1; ++k) start[k] += start[k - 1];
+    order.resize(n.size());
+    std::vector<int32_t> sorted(n.size());
+    for (size_t k = 0; k < n.size(); ++k) {
+        const int32_t at = start[kMaxN - n[k]]++;
+        order[(size_t)at] = (int32_t)k;
+        sorted[(size_t)at] = n[k];
+    }
+    n.swap(sorted);
+    return order;
+}
+
+// Room for the largest dynamic shared memory, set once per device and kernel
+// (idempotent if repeated).
+template <class Kernel>
+static int polish_attr(sqs_ctx* ctx, Kernel kernel, std::atomic<bool>* done) {
+    if (!done[ctx->device & 63]) {
+        SQS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
+        done[ctx->device & 63] = true;
+    }
     return SQS_OK;
 }
 
-int launch_polish_states(cudaStream_t stream, int count, const int32_t* n_of, const int64_t* row0, int iters,
-                         double* xya, double* res, size_t smem) {
-    static std::atomic<bool> attr_done[64];  // set-up once per device (idempotent if repeated)
-    int dev = 0;
-    SQS_CUDA(cudaGetDevice(&dev));
-    if (!attr_done[dev & 63]) {
-        SQS_CUDA(cudaFuncSetAttribute(polish_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
-        attr_done[dev & 63] = true;
-    }
-    if (count <= 0) return SQS_OK;
-    polish_states_kernel<<<count, kPT, smem, stream>>>(n_of, row0, iters, xya, res);
-    SQS_CUDA(cudaGetLastError());
-    return SQS_OK;
+int launch_energy_states(sqs_ctx* ctx, const std::vector<int32_t>& n, const int32_t* order, const int32_t* n_of,
+                         const int64_t* row0, const double* side, const double* xya, double* energy_out, double* grad) {
+    return launch_widths(ctx, n, [&](auto width, cudaStream_t st, int first, int count, int nmax) -> int {
+        constexpr int PT = decltype(width)::value;
+        static std::atomic<bool> done[64];
+        if (int r = polish_attr(ctx, energy_states_kernel<PT>, done)) return r;
+        energy_states_kernel<PT><<<count, PT, energy_smem_bytes(nmax), st>>>(order ? order + first : nullptr, n_of, row0,
+                                                                             side, xya, energy_out, grad);
+        SQS_CUDA(cudaGetLastError());
+        ctx->launches += 1;
+        return SQS_OK;
+    });
 }
 
-int launch_polish(cudaStream_t stream, int njobs, const int32_t* job_list, const JobDev* jdev, JobMut* jmut,
-                  double* best, size_t smem) {
-    static std::atomic<bool> attr_done[64];  // set-up once per device (idempotent if repeated)
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!attr_done[dev & 63]) {
-        SQS_CUDA(cudaFuncSetAttribute(polish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024));
-        attr_done[dev & 63] = true;
-    }
-    if (njobs <= 0) return SQS_OK;
-    polish_kernel<<<njobs, kPT, smem, stream>>>(job_list, jdev, jmut, best);
-    SQS_CUDA(cudaGetLastError());
-    return SQS_OK;
+int launch_polish_states(sqs_ctx* ctx, const std::vector<int32_t>& n, const int32_t* order, const int32_t* n_of,
+                         const int64_t* row0, int iters, double* xya, double* res) {
+    return launch_widths(ctx, n, [&](auto width, cudaStream_t st, int first, int count, int nmax) -> int {
+        constexpr int PT = decltype(width)::value;
+        static std::atomic<bool> done[64];
+        if (int r = polish_attr(ctx, polish_states_kernel<PT>, done)) return r;
+        polish_states_kernel<PT><<<count, PT, polish_smem_bytes(nmax), st>>>(order ? order + first : nullptr, n_of, row0,
+                                                                             iters, xya, res);
+        SQS_CUDA(cudaGetLastError());
+        ctx->launches += 1;
+        return SQS_OK;
+    });
+}
+
+int launch_polish(sqs_ctx* ctx, const std::vector<int32_t>& n, const int32_t* job_list, const JobDev* jdev, JobMut* jmut,
+                  double* best) {
+    return launch_widths(ctx, n, [&](auto width, cudaStream_t st, int first, int count, int nmax) -> int {
+        constexpr int PT = decltype(width)::value;
+        static std::atomic<bool> done[64];
+        if (int r = polish_attr(ctx, polish_kernel<PT>, done)) return r;
+        polish_kernel<PT><<<count, PT, polish_smem_bytes(nmax), st>>>(job_list + first, jdev, jmut, best);
+        SQS_CUDA(cudaGetLastError());
+        ctx->launches += 1;
+        return SQS_OK;
+    });
 }
 
 }  // namespace ann

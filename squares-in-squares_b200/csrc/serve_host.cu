@@ -545,13 +545,14 @@ int retire(sqs_server* s, Retirer* me, const std::vector<int32_t>& fin) {
     }
     const int64_t l0 = me->ctx->launches;
     const auto t0 = std::chrono::steady_clock::now();
-    size_t psmem = 0;
-    for (const SJob* j : jobs) psmem = std::max(psmem, polish_smem_bytes(j->job.n));
-    SQS_CUDA(cudaMemcpyAsync(me->d_list, fin.data(), sizeof(int32_t) * fin.size(), cudaMemcpyHostToDevice,
+    std::vector<int32_t> pn;
+    for (const SJob* j : jobs) pn.push_back(j->job.n);
+    std::vector<int32_t> plist = width_order(me->ctx, pn);
+    for (int32_t& q : plist) q = fin[(size_t)q];
+    if (plist.empty()) plist = fin;
+    SQS_CUDA(cudaMemcpyAsync(me->d_list, plist.data(), sizeof(int32_t) * plist.size(), cudaMemcpyHostToDevice,
                              me->ctx->stream));
-    if (int r = launch_polish(me->ctx->stream, (int)fin.size(), me->d_list, s->d_jd, s->d_jm, (double*)s->arena, psmem))
-        return r;
-    me->ctx->launches += 1;
+    if (int r = launch_polish(me->ctx, pn, me->d_list, s->d_jd, s->d_jm, (double*)s->arena)) return r;
     std::vector<std::vector<double>> best(fin.size()), out(fin.size());
     std::vector<JobMut> jm(fin.size());
     for (size_t q = 0; q < fin.size(); ++q) {

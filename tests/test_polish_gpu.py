@@ -94,3 +94,57 @@ def test_polish_errors(ctx):
     with pytest.raises(SQSError):
         polish_batch([np.array([[0.5, 0.5, 0.0]])], -1, ctx=ctx)
     assert polish_batch([], ctx=ctx) == []
+
+
+def test_cta_width_by_size_changes_no_bit(ctx):
+    """A batch past one packing an SM runs on CTAs of 128, 256 or 512 threads
+    by size; each packing alone runs on 512.  Polished states, sides, step
+    counts, energies and gradients are the same, at the sizes where the width
+    changes, for certified and overlapped states."""
+    import numpy as np
+
+    from sqs.polish import polish_batch
+    from sqs.sat import energy_fp64
+    from sqs.workloads import grid_state
+
+    sizes = [1, 2, 7, 16, 17, 32, 33, 63, 64, 65, 128, 129, 255, 256, 257, 400]
+    sizes = sizes * (ctx.info()[1] // len(sizes) + 2)
+    states, sides = [], []
+    for k, n in enumerate(sizes):
+        pitch, jitter = (1.004, 1e-3) if k % 3 else (0.97, 0.06)
+        states.append(grid_state(n, pitch=pitch, jitter=jitter, angle_hi=0.05 if k % 3 == 0 else 0.002, seed=k))
+        sides.append(max(1.05, pitch * np.ceil(np.sqrt(n))))
+    sides = np.array(sides)
+    got = polish_batch(states, 40, ctx=ctx)
+    e, g = energy_fp64(states, sides, ctx=ctx)
+    for k in list(range(16)) + [len(sizes) - 2, len(sizes) - 1]:
+        (q, r), = polish_batch([states[k]], 40, ctx=ctx)
+        e1, g1 = energy_fp64([states[k]], sides[k], ctx=ctx)
+        np.testing.assert_array_equal(got[k][0], q)
+        assert got[k][1] == r
+        assert e[k] == e1[0]
+        np.testing.assert_array_equal(g[k], g1[0])
+
+
+def test_many_small_packings_take_narrow_ctas(ctx):
+    """1,200 packings of 64 squares fit several to an SM: their polish takes
+    well under the 1,200 / 148 turns that one packing an SM at a time would."""
+    import time
+
+    from sqs.polish import polish_batch
+    from sqs.workloads import grid_state
+
+    q = [grid_state(64, pitch=0.97, jitter=0.06, angle_hi=0.05, seed=k) for k in range(1200)]
+    one_wave = q[:ctx.info()[1]]
+
+    def took(states, iters):
+        polish_batch(states, iters, ctx=ctx)
+        best = 1e9
+        for _ in range(5):
+            t0 = time.perf_counter()
+            polish_batch(states, iters, ctx=ctx)
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    per_step = [(took(s, 400) - took(s, 100)) / 300 for s in (one_wave, q)]
+    assert per_step[1] < 0.75 * len(q) / len(one_wave) * per_step[0], per_step
