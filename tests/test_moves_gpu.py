@@ -227,3 +227,24 @@ def test_quench_width_and_corners(ctx, n, moves):
             assert r[k] == got[0][k], k
         for k in ("xya", "energy", "rung"):
             np.testing.assert_array_equal(r["trace"][k], got[0]["trace"][k], err_msg=k)
+
+
+@pytest.mark.parametrize("n,replicas,clusters", [(700, 20, (2, 4, 10)), (1000, 28, (4, 7, 14))])
+@pytest.mark.parametrize("moves", [False, True])
+def test_quench_scratch_in_hbm_equals_shared(ctx, n, replicas, clusters, moves):
+    """At the smallest of these clusters a CTA's replicas leave no room for the
+    quench scratch in shared memory and it lies in HBM; at the larger ones
+    there is room.  Every replica ends in the same state with the same energy,
+    and the CTAs of a cluster do not disturb one another's scratch."""
+    from sqs.anneal import anneal_batch
+
+    opts = dict(adapt=True, collective=True, kick=True, quench_all=True, quench_steps=1, cert_all=True) if moves else {}
+    job = _job(n=n, replicas=replicas, sweeps=-60, exchange_every=-12, tmin=1e-5, tmax=1e-3, polish_iters=0, **opts)
+    got = [anneal_batch([replace(job, cluster=c)], ctx=ctx, trace=True)[0] for c in clusters]
+    for r in got:
+        assert r["status"] == 0, r["reason"]
+        np.testing.assert_array_equal(r["trace"]["energy"], r["trace"]["energy_full"])
+        for k in KEYS:
+            assert r[k] == got[0][k], k
+        for k in ("xya", "energy", "rung"):
+            np.testing.assert_array_equal(r["trace"][k], got[0]["trace"][k], err_msg=k)
