@@ -269,7 +269,8 @@ typedef struct sqs_job_result {
     int32_t status;          /* 0 ok; < 0 job error (see reason)                  */
     int32_t certified;       /* the interval certifier accepted the packing      */
     int32_t shrinks, improvements, sweeps_done, replicas;
-    int32_t cluster_ctas;    /* CTAs per job the job ran on                       */
+    int32_t cluster_ctas;    /* CTAs per job the job ran on (served: its last slice,
+                                whose shape depends on the server's load)          */
     int32_t replicas_per_cta;/* replicas (warps) per CTA                          */
     int32_t exchange_every;  /* sweeps between exchange rounds it ran with        */
     int32_t overflows;       /* moves rejected because the target cell was full  */

@@ -1074,7 +1074,6 @@ struct CtaShared {
     int bad;                   // any overflow in the cluster
     int reset0;                // SQS_JOB_TARGETS: the gain resets every rung of ladder 0, not only heads
     float newL;
-    unsigned long long props[kMaxRl], accs[kMaxRl];
     long long red[kGrpSlots * kMaxRl];  // group sums: kGrpSlots values a warp
     long long qE;              // energy of the replica quenched by this CTA
     long long qEv[kMaxRl];     // each replica's energy before a group quench
@@ -1550,9 +1549,10 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
             }
             __syncthreads();
         } else {
-            // the replica on the coldest rung, by warps of the CTA that holds it; its scratch in shared memory after the replicas when
-            // the launch left room, else its first replica's block of the job's scratch
-            // (the other CTAs' replicas may be using theirs)
+            // the replica on the coldest rung, by warps of the CTA that holds it;
+            // its scratch in shared memory after the replicas when the launch left
+            // room, else its first replica's block of the job's scratch (the other
+            // CTAs' replicas may be using theirs)
             float4* qs = (int64_t)dyn_bytes >= (int64_t)Rl * rb + (int64_t)sizeof(float4) * kQuenchScr * n
                              ? reinterpret_cast<float4*>(dyn + (int64_t)Rl * rb)
                              : pos + jd.scr_off + (int64_t)rank * Rl * kQuenchScr * n;
@@ -1577,7 +1577,7 @@ __global__ void __launch_bounds__(32 * kMaxRl) anneal_kernel(const int32_t* __re
             // so the energy gate skips states that cannot pass); under
             // SQS_JOB_CERT_ALL every replica is measured, as the reference
             // search measures every chain after its polish (seeded.cu:716)
-            if (E < qe(1e-4f) || (jd.flags & kCertAll)) 
+            if (E < qe(1e-4f) || (jd.flags & kCertAll))
                 Lc = cert_side(rep, n, g, lane, reinterpret_cast<double2*>(scr_own), lam, x0, y0);
             if (lane == 0) {
                 S.wE[w] = E;
