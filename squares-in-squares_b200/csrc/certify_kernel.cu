@@ -1209,6 +1209,7 @@ extern "C" int sqs_certify_batch(sqs_ctx* ctx, int count, const int32_t* n_of, c
     // A large literal text is staged in pinned memory too, each thread copying
     // the span of its own packings (the first from offset 0), so that it
     // uploads at the full host-link rate.
+    SQS_REQUIRE(lit_off[3 * row_start[count]] >= 0, "literal offsets end below 0");
     const size_t text_bytes = (size_t)lit_off[3 * row_start[count]];
     char* h_text = nullptr;
     if (!do_rt && text_bytes >= kPinnedTextMin && text_bytes <= kPinnedTextMax) {
@@ -1532,6 +1533,7 @@ extern "C" int sqs_certify_batch_static(sqs_ctx* ctx, int count, const int32_t* 
     const bool do_rt = (flags & SQS_CERT_ROUNDTRIP) != 0;
     // envelope checks and literal slices, as sqs_certify_batch does them
     const int64_t text_end = lit_off[3 * row_start[count]];
+    SQS_REQUIRE(text_end >= 0, "literal offsets end below 0");
     SQS_REQUIRE(do_rt || text_end <= (int64_t)kStaticMaxText, "literals exceed %zu bytes (static certifier limit)",
                 kStaticMaxText);
     int64_t S = 0;

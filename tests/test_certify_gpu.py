@@ -250,3 +250,18 @@ def test_literal_offsets_outside_the_text_are_refused(ctx):
     for off in ([0, 3, 6, 90, 7, 7, 7], [-9, 3, 6, 7, 7, 7, 7]):
         with pytest.raises(SQSError):
             core.certify_arrays(np.array([1, 2], np.int32), np.array([0, 1, 2]), None, text, np.array(off), ctx=ctx)
+
+
+@pytest.mark.parametrize("entry", ["sqs_certify_batch", "sqs_certify_batch_static"])
+def test_negative_text_length_is_refused(ctx, entry):
+    """Offsets that end below zero are an argument error, also when no packing
+    of the call is looked at."""
+    import numpy as np
+
+    from sqs import _native as N
+
+    n_of, row_start, off = np.array([2], np.int32), np.array([0, 1], np.int64), np.array([0, 0, 0, -5], np.int64)
+    out = (N.Verdict * 1)()
+    rc = getattr(N.lib(), entry)(ctx.handle, 1, n_of.ctypes.data, row_start.ctypes.data, None, b"0.50.50",
+                                 off.ctypes.data, 0, out)
+    assert rc == -1  # SQS_EINVAL
